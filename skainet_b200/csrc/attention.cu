@@ -13,14 +13,13 @@
 #include "common.cuh"
 #include "actquant.cuh"
 #include "tma.cuh"
+#include "attn_frag.cuh"
 
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
 
 namespace sk {
-
-constexpr float MASKED = -1.0e30f;
 
 // =================================================================================================
 // Decode attention, split-K: merge of the partial records.
@@ -99,22 +98,7 @@ __global__ void __launch_bounds__(D * MG) attn_merge_kernel(const float* __restr
 // one prmt each. Each warp walks its own keys with an online softmax; warps, then key splits, are merged
 // in a fixed order.
 // =================================================================================================
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// (x, y) -> f16 high parts packed, f16 low parts (x - hi(x)) packed
-__device__ __forceinline__ void split_pack(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __half hx = __float2half_rn(x), hy = __float2half_rn(y);
-    const __half lx = __float2half_rn(x - __half2float(hx)), ly = __float2half_rn(y - __half2float(hy));
-    hi = (uint32_t) __half_as_ushort(hx) | ((uint32_t) __half_as_ushort(hy) << 16);
-    lo = (uint32_t) __half_as_ushort(lx) | ((uint32_t) __half_as_ushort(ly) << 16);
-}
-
 constexpr int AM_WARPS = 8;
-constexpr float LOG2E = 1.4426950408889634f;
-// exp(x) for x <= 0 through the ex2 unit (relative error ~1e-7 after the fp32 pre-scale)
-__device__ __forceinline__ float fast_exp(float x) { return exp2f(x * LOG2E); }
 
 // What the decode step folds into the attention kernel (FUSE): the rotary embedding of q and of the token's new key,
 // and the append of that key and value to the f16 cache. q, k, v of the token arrive unrotated in one merged row
@@ -399,7 +383,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
 
 // Fewest keys a split is given: one 16-key tile per warp of the split-K kernel.
 static int attn_min_keys() { return 128; }
-static int decode_splits(int batch, int kv_heads, int max_kv_len) {
+int decode_splits(int batch, int kv_heads, int max_kv_len) {
     // One wave: the split-K kernel holds one CTA of eight warps per SM (register-bound), and a second wave
     // would double its time. Each split gets at least min_keys keys (one 16-key tile per warp at 128).
     const int ctas = batch * kv_heads;
@@ -453,6 +437,12 @@ attn_merge_quant_kernel(const float* __restrict__ part, float* __restrict__ out,
         if (lane == 0) oq.bsums[((int64_t) b * n + e) >> 5] = (int16_t) sum;
         if (threadIdx.x == 0) oq.d[((int64_t) b * n + e) >> 8] = amax > 0.0f ? amax / 127.0f : 0.0f;
     }
+}
+
+int32_t launch_attn_merge(const float* part, float* out, int rows, int d, int splits, cudaStream_t s) {
+    if (d == 128) SK_CUDA(launch_pdl(attn_merge_kernel<128>, dim3(rows), dim3(128 * MG), 0, s, part, out, splits));
+    else SK_CUDA(launch_pdl(attn_merge_kernel<64>, dim3(rows), dim3(64 * MG), 0, s, part, out, splits));
+    return SKAINET_CUDA_OK;
 }
 
 template <int D, int G>

@@ -12,7 +12,8 @@
 // (skainet-lang/skainet-lang-core/src/commonMain/kotlin/sk/ainet/lang/memory/WindowedAttention.kt:32-80).
 //
 // A second kind of store keeps TurboQuant blocks instead of binary16 rows (TurboQuantKvCacheStore.kt:62-199; codec in
-// turboquant.cu): dense only, one block per (layer, position, head); reads and attention decode the window first.
+// turboquant.cu): dense only, one block per (layer, position, head); reads decode the window, attention decodes the blocks as it goes
+// (tq_attn.cu) or, with a residual stage and for other head and group sizes, the window first.
 #include "common.cuh"
 #include "turboquant.cuh"
 
@@ -311,6 +312,12 @@ int32_t skainet_cuda_kv_attn_decode_dev(skainet_kv_t h, int32_t layer, const flo
         SK_REQUIRE(to_pos <= s->cur, "kv_attn_decode: a TurboQuant store attends appended positions only (window end %d, currentSeqLen %d)", to_pos, s->cur);
         const size_t plane = (size_t) s->heads * len * s->head_dim;
         void* win = nullptr;
+        if (s->kq.rbits == 0 && s->vq.rbits == 0) {        // no residual stage: the attention kernel decodes the blocks itself
+            void* scratch = nullptr;
+            SK_TRY(scratch_get(st, SCRATCH_ATTN, attn_scratch_bytes(1, q_heads, s->head_dim, len), &scratch));
+            const int32_t r = launch_tq_attn_decode(q_dev, s->kq, s->vq, layer, from_pos, len, s->heads, q_heads, s->head_dim, s->max_seq, sc0, out_dev, scratch, st);
+            if (r != 1) return r;
+        }
         if ((G == 1 || G == 2 || G == 4 || G == 8) && (s->head_dim == 64 || s->head_dim == 128)) {
             // the window's blocks decoded to binary16 rows [heads][len][head_dim], then the split-K decode attention over them
             // (the rounding the binary16 store applies to every row it holds)

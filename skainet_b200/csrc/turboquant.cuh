@@ -38,4 +38,10 @@ int32_t launch_tq_decode(const TqPlane& pl, int layer, int start_pos, int n, int
 // the same rows rounded to binary16 (the layout the decode-attention kernel reads: [heads][n][head_dim])
 int32_t launch_tq_decode_f16(const TqPlane& pl, int layer, int start_pos, int n, int heads, int head_dim, int max_seq, int32_t seed_xor, __half* out, cudaStream_t s);
 
+// tq_attn.cu: decode attention of q [q_heads][head_dim] over positions [start_pos, start_pos + len) straight from the blocks; out
+// [q_heads][head_dim], scratch attn_scratch_bytes. 1 = not taken (residual stages, head sizes other than 64 and 128, groups other
+// than 1, 2, 4 and 8)
+int32_t launch_tq_attn_decode(const float* q, const TqPlane& kp, const TqPlane& vp, int layer, int start_pos, int len, int kv_heads, int q_heads, int head_dim,
+                              int max_seq, float scale, float* out, void* scratch, cudaStream_t s);
+
 }  // namespace sk
