@@ -327,7 +327,6 @@ static int32_t check_tokens(const Decoder& m, const int32_t* tokens, int n, cons
 template <typename F>
 static int32_t run_prompt(Decoder* m, int seq, const int32_t* tokens_host, int n, F&& after_pass) {
     cudaStream_t s = m->stream;
-    SK_TRY(m->begin_prompt(seq, s));
     for (int done = 0; done < n;) {
         const int rows = std::min(n - done, m->max_rows);
         SK_CUDA(cudaMemcpyAsync(m->cur_token, tokens_host + done, sizeof(int32_t) * rows, cudaMemcpyHostToDevice, s));

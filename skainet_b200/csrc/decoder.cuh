@@ -45,7 +45,6 @@ struct Decoder {
     // Row b = next token (cur_token[b]) of sequence b at pos[b]; leaves logits[b]. kv_bound bounds every sequence's length after the step.
     virtual int32_t enqueue_decode(int batch, int kv_bound, cudaStream_t s) = 0;
     // Rows = consecutive tokens (cur_token[0..rows)) of sequence seq from pos[seq].
-    virtual int32_t begin_prompt(int seq, cudaStream_t s) { (void) seq; (void) s; return SKAINET_CUDA_OK; }
     virtual int32_t enqueue_prompt(int rows, int seq, int kv_bound, cudaStream_t s) = 0;
     // Logits of n <= logits_rows rows of the prompt pass just enqueued, in the order of `rows` (host), into logits[0..n).
     virtual int32_t enqueue_head(const int32_t* rows, int n, cudaStream_t s) = 0;

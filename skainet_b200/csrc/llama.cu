@@ -39,13 +39,11 @@ constexpr int SWIGLU_PROLOGUE_MAX_COLS = SK_SWIGLU_PROLOGUE_MAX_COLS;
 // each sequence's position. grid (rows, heads + 2*kv_heads), head_dim/2 threads. The rotation factors
 // come from a table built on the host in double precision.
 __global__ void rope_append_kernel(float* __restrict__ qkv, int heads, int kv_heads, int d, const float* __restrict__ cos_t,
-                                   const float* __restrict__ sin_t, const int32_t* __restrict__ pos, const int32_t* __restrict__ seq_of_row,
-                                   int pos_step, __half* __restrict__ kc, __half* __restrict__ vc, int64_t cache_stride, int mode) {
+                                   const float* __restrict__ sin_t, const int32_t* __restrict__ pos, __half* __restrict__ kc, __half* __restrict__ vc, int64_t cache_stride, int mode) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
-    const int row = blockIdx.x, hh = blockIdx.y, i = threadIdx.x, half = d >> 1;
-    const int seq = seq_of_row ? seq_of_row[row] : row;
-    const int p = pos[seq] + (pos_step ? row : 0);       // prefill: consecutive rows of one sequence
+    const int row = blockIdx.x, seq = row, hh = blockIdx.y, i = threadIdx.x, half = d >> 1;
+    const int p = pos[seq];
     float* base = qkv + (size_t) row * (heads + 2 * kv_heads) * d + (size_t) hh * d;
     if (hh < heads + kv_heads) {
         const float c = cos_t[(size_t) p * half + i], s = sin_t[(size_t) p * half + i];
@@ -60,6 +58,43 @@ __global__ void rope_append_kernel(float* __restrict__ qkv, int heads, int kv_he
     } else {
         __half* dst = vc + (((size_t) seq * kv_heads + (hh - heads - kv_heads)) * cache_stride + p) * d;
         dst[2 * i] = __float2half_rn(base[2 * i]); dst[2 * i + 1] = __float2half_rn(base[2 * i + 1]);
+    }
+}
+
+// The same for the rows of a prompt pass (consecutive positions of one sequence from pos[0]), with q going rotated into a dense
+// [rows][heads * d] buffer, the attention's input. A thread takes four rotation pairs, 32 bytes in and out, so a row of the 7B
+// shape is 1536 threads; with one pair per thread and a CTA per head the 512 rows of a pass took 53 us, and 10 more for the
+// copy of q (a 512-token prompt through the 7B shape: 23.0 against 21.5 ms). grid (ceil((heads + 2 kv_heads) * d / 8 / 256), rows).
+__global__ void __launch_bounds__(256)
+rope_prompt_kernel(const float* __restrict__ qkv, float* __restrict__ q, int heads, int kv_heads, int d, const float* __restrict__ cos_t,
+                   const float* __restrict__ sin_t, const int32_t* __restrict__ pos, __half* __restrict__ kc, __half* __restrict__ vc,
+                   int64_t cache_stride, int mode) {
+    skd::pdl_launch_dependents();
+    skd::pdl_wait();
+    const int per_head = d >> 3, item = blockIdx.x * 256 + threadIdx.x, hh = item / per_head, j = item % per_head, row = blockIdx.y, half = d >> 1;
+    if (hh >= heads + 2 * kv_heads) return;
+    const int p = pos[0] + row;
+    // elements: two runs of four, the pairs' halves (mode 1) or adjacent (mode 0, values)
+    const bool rotate = hh < heads + kv_heads;
+    const int e0 = mode == 0 || !rotate ? 8 * j : 4 * j, e1 = mode == 0 || !rotate ? e0 + 4 : e0 + half;
+    const float* src = qkv + ((size_t) row * (heads + 2 * kv_heads) + hh) * d;
+    float4 a = __ldg(reinterpret_cast<const float4*>(src + e0)), b = __ldg(reinterpret_cast<const float4*>(src + e1));
+    if (rotate) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(cos_t + (size_t) p * half) + j), s = __ldg(reinterpret_cast<const float4*>(sin_t + (size_t) p * half) + j);
+        auto turn = [](float& x, float& y, float cc, float ss) {
+            const float rx = __fsub_rn(__fmul_rn(x, cc), __fmul_rn(y, ss)), ry = __fadd_rn(__fmul_rn(x, ss), __fmul_rn(y, cc));
+            x = rx; y = ry;
+        };
+        if (mode == 0) { turn(a.x, a.y, c.x, s.x); turn(a.z, a.w, c.y, s.y); turn(b.x, b.y, c.z, s.z); turn(b.z, b.w, c.w, s.w); }
+        else { turn(a.x, b.x, c.x, s.x); turn(a.y, b.y, c.y, s.y); turn(a.z, b.z, c.z, s.z); turn(a.w, b.w, c.w, s.w); }
+    }
+    if (hh < heads) {
+        float* dst = q + ((size_t) row * heads + hh) * d;
+        *reinterpret_cast<float4*>(dst + e0) = a; *reinterpret_cast<float4*>(dst + e1) = b;
+    } else {
+        __half* dst = rotate ? kc + ((size_t) (hh - heads) * cache_stride + p) * d : vc + ((size_t) (hh - heads - kv_heads) * cache_stride + p) * d;
+        const __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y), __floats2half2_rn(b.z, b.w)};
+        *reinterpret_cast<uint2*>(dst + e0) = *reinterpret_cast<const uint2*>(h); *reinterpret_cast<uint2*>(dst + e1) = *reinterpret_cast<const uint2*>(h + 2);
     }
 }
 
@@ -103,12 +138,10 @@ struct Llama : Decoder {
     float *x = nullptr, *qkv = nullptr, *q = nullptr, *attn = nullptr, *gu = nullptr, *tmp = nullptr;
     void *act = nullptr; size_t act_bytes = 0;
     void *attn_scratch = nullptr; size_t attn_scratch_bytes = 0;
-    int32_t* row_seq = nullptr;
 
     ~Llama() override;
     int32_t finalize() override;
     int32_t enqueue_decode(int batch, int kv_bound, cudaStream_t s) override;
-    int32_t begin_prompt(int seq, cudaStream_t s) override;
     int32_t enqueue_prompt(int rows, int seq, int kv_bound, cudaStream_t s) override;
     int32_t enqueue_head(const int32_t* rows, int n, cudaStream_t s) override;
     int32_t fill_context(int seq, int n, uint64_t seed) override;
@@ -250,15 +283,16 @@ static int32_t body(Llama& m, int rows, bool prefill, int seq, int kv_bound, cud
                 continue;
             }
         }
-        SK_CUDA(launch_pdl(rope_append_kernel, dim3(rows, H + 2 * HK), dim3(D / 2), 0, s, m.qkv, H, HK, D, (const float*) m.cos_t,
-                           (const float*) m.sin_t, (const int32_t*) m.pos, (const int32_t*) (prefill ? m.row_seq : nullptr), prefill ? 1 : 0,
-                           L.kc, L.vc, (int64_t) c.max_seq, c.rope_mode));
+        const size_t seq_at = prefill ? (size_t) seq * HK * c.max_seq * D : 0;
+        if (prefill) SK_CUDA(launch_pdl(rope_prompt_kernel, dim3(((H + 2 * HK) * D / 8 + 255) / 256, rows), dim3(256), 0, s, (const float*) m.qkv, m.q, H, HK, D,
+                                        (const float*) m.cos_t, (const float*) m.sin_t, (const int32_t*) (m.pos + seq), L.kc + seq_at, L.vc + seq_at,
+                                        (int64_t) c.max_seq, c.rope_mode));
+        else SK_CUDA(launch_pdl(rope_append_kernel, dim3(rows, H + 2 * HK), dim3(D / 2), 0, s, m.qkv, H, HK, D, (const float*) m.cos_t,
+                                (const float*) m.sin_t, (const int32_t*) m.pos, L.kc, L.vc, (int64_t) c.max_seq, c.rope_mode));
         const bool fused_attn = !prefill && (H * D) % 256 == 0;
-        if (!fused_attn) SK_CUDA(launch_pdl(gather_q_kernel, dim3(rows), dim3(256), 0, s, (const float*) m.qkv, m.q, H * D, qkv_dim));
+        if (!prefill && !fused_attn) SK_CUDA(launch_pdl(gather_q_kernel, dim3(rows), dim3(256), 0, s, (const float*) m.qkv, m.q, H * D, qkv_dim));
         if (prefill) {
-            const __half* kc = L.kc + (size_t) seq * HK * c.max_seq * D;
-            const __half* vc = L.vc + (size_t) seq * HK * c.max_seq * D;
-            SK_TRY(launch_sdpa_cache(m.q, kc, vc, m.attn, 1, H, HK, rows, kv_bound, c.max_seq, D, scale, 0, m.pos + seq, s));
+            SK_TRY(launch_sdpa_cache(m.q, L.kc + seq_at, L.vc + seq_at, m.attn, 1, H, HK, rows, kv_bound, c.max_seq, D, scale, 0, m.pos + seq, s));
         } else if (fused_attn) {   // q read in place from the merged buffer; merge of the key splits quantizes for o_proj
             ActQ8K oq = {nullptr, nullptr, nullptr}; ActSplit os = {nullptr, nullptr, nullptr};
             if (o_split) os = act_split_layout(m.act, rows, H * D); else oq = act_q8k_layout(m.act, rows, H * D);
@@ -286,12 +320,6 @@ int32_t Llama::enqueue_decode(int batch, int kv_bound, cudaStream_t s) {
     SK_TRY(body(*this, batch, false, 0, kv_bound, s, fold_out_norm ? g_out : nullptr, &head_ready));
     if (head_ready) return linear(*this, *head, batch, logits, nullptr, s);
     return linear_normed(*this, *head, x, g_out, batch, logits, s);
-}
-
-int32_t Llama::begin_prompt(int seq, cudaStream_t s) {
-    const std::vector<int32_t> seqs(max_rows, seq);
-    SK_CUDA(cudaMemcpyAsync(row_seq, seqs.data(), sizeof(int32_t) * max_rows, cudaMemcpyHostToDevice, s));
-    return SKAINET_CUDA_OK;
 }
 
 int32_t Llama::enqueue_prompt(int rows, int seq, int kv_bound, cudaStream_t s) {
@@ -336,7 +364,7 @@ Llama::~Llama() {
     if (embed) weight_release(embed);
     if (head && head != embed) weight_release(head);
     for (void* p : {(void*) g_out, (void*) cos_t, (void*) sin_t, (void*) x, (void*) qkv, (void*) q, (void*) attn, (void*) gu, (void*) tmp, act,
-                    attn_scratch, (void*) row_seq})
+                    attn_scratch})
         if (p) cudaFree(p);
 }
 
@@ -418,7 +446,6 @@ int32_t skainet_cuda_llama_create(const skainet_llama_config* cfg, skainet_model
     if (st == SKAINET_CUDA_OK && cudaMalloc(&m->act, m->act_bytes) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "cudaMalloc(act)", __FILE__, __LINE__);
     m->attn_scratch_bytes = attn_scratch_bytes(c.max_batch, m->heads_l, c.head_dim, c.max_seq);
     if (st == SKAINET_CUDA_OK && cudaMalloc(&m->attn_scratch, m->attn_scratch_bytes) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "cudaMalloc(attn scratch)", __FILE__, __LINE__);
-    A(dalloc(&m->row_seq, R));
     if (st == SKAINET_CUDA_OK) {
         std::vector<float> ones(c.d_model, 1.0f);
         for (auto& L : m->layers) { cudaMemcpy(L.g_attn, ones.data(), 4 * c.d_model, cudaMemcpyHostToDevice); cudaMemcpy(L.g_ffn, ones.data(), 4 * c.d_model, cudaMemcpyHostToDevice); }
