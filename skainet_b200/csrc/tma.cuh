@@ -47,6 +47,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The same by a whole warp, with one verdict for all its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* timeout_flag) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, timeout_flag));
+}
+
+// One lane of a converged warp. Loops that issue tcgen05 or TMA instructions are run by the whole warp, with only the instructions
+// themselves under this predicate: their operands are then known to be the same in all lanes and stay in uniform registers
+// (under `lane == 0` every operand is moved there first, 70 to 80 cycles an instruction).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 
 // d = c + sum_i a.u8[i] * b.s8[i]
