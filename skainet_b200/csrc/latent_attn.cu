@@ -2,6 +2,7 @@
 //
 // A step's chain for few rows (decode):  prep + fold of W_uk | attention over key splits | merge + W_uv + gate
 // and for many rows (prefill):           prep | fold (grouped GEMM) | attention | [merge] | W_uv + gate (grouped GEMM)
+//                                    or  prep | keys and values of all heads (GEMM) | attention and gate
 //
 // latent_attn_mma_kernel (bf16): the MMA rows are (activation row, head) pairs, which all read the same keys; one staged
 // [key][latent | rotated part] tile is the B operand of the scores and, its latent columns transposed on load, of the mix.
@@ -376,6 +377,143 @@ latent_attn_mma_kernel(const LatentArgs a, const SplitArgs sp) {
     }
 }
 
+// ---- expanded form for prompts --------------------------------------------------------------------------------------
+// With many rows the keys and values of each head are worth forming: per (query, key, head) the scores and the mix then take
+// 192 + 128 products instead of 576 + 512, for 2 * 128 * 512 per (key, head) once (one product on tcgen05). kv holds them
+// for the sequence's cache slots, [slot][keys of all heads | values of all heads]; the rotated key part comes from the cache row.
+// CTA = 128 query rows of one head, a warp 16 of them with its query fragments and 16 x 128 output in registers, over tiles of
+// 64 keys through a ring of three. Bound by the mma.sync rate and the fragment loads. A 2048-token prompt of the 2B shape (24 layers,
+// 16 heads, latent 512, window 1024, passes of 1024 rows) takes 12.76 ms so and 20.34 in the folded form, whose attention alone took
+// 211 us of the 430 a layer and pass.
+constexpr int EX_ROWS = 128, EX_BK = 64, EX_DIM = 128, EX_ROT = 64, EX_ST = 3, EX_KLD = EX_DIM + EX_ROT + 8, EX_VLD = EX_DIM + 8;
+constexpr int EX_STAGE = EX_BK * (EX_KLD + EX_VLD), EX_SMEM = (EX_ROWS * EX_KLD + EX_ST * EX_STAGE) * 2;
+
+__global__ void __launch_bounds__(256, 1) latent_attn_expanded_kernel(const LatentArgs a) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const LatentGeom& g = a.g;
+    bf16* sq = (bf16*) smem;                                  // [EX_ROWS][EX_KLD]
+    bf16* ring = sq + EX_ROWS * EX_KLD;                       // [EX_ST][keys EX_BK x EX_KLD | values EX_BK x EX_VLD]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x, r0 = (gridDim.y - 1 - blockIdx.y) * EX_ROWS;     // the rows with the most keys first
+    const int width = g.heads * EX_DIM, kld = g.key_ld(), RP = g.rank_pad();
+    skd::pdl_launch_dependents();
+    skd::pdl_wait();
+    const int r_last = min(r0 + EX_ROWS, a.rows) - 1, pos0 = a.map.pos_of(r0), hi = a.map.pos_of(r_last), lo = max(0, pos0 - a.window + 1), cap = a.cache.cap;
+    const int n_tiles = (hi - lo + EX_BK) / EX_BK;
+    const bf16* cache = (const bf16*) a.cache.rows + (size_t) a.map.seq_of(r0) * cap * kld + RP;
+    const bf16* kv = (const bf16*) a.kv + (size_t) h * EX_DIM;
+
+    auto fetch = [&](int t) {                                 // keys past hi repeat the newest one; their weights are masked
+        if (t < n_tiles) {
+            bf16* kd = ring + (t % EX_ST) * EX_STAGE;
+            bf16* vd = kd + EX_BK * EX_KLD;
+            // four threads per key, ten 16-byte pieces each: four of the key, two rotated, four of the value
+            const int j = threadIdx.x >> 2, c0 = threadIdx.x & 3;
+            const int slot = min(lo + t * EX_BK + j, hi) % cap;
+            const bf16 *ks = kv + (size_t) slot * 2 * width, *rs = cache + (size_t) slot * kld;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                cp16(kd + j * EX_KLD + (c0 + 4 * c) * 8, ks + (c0 + 4 * c) * 8);
+                cp16(vd + j * EX_VLD + (c0 + 4 * c) * 8, ks + width + (c0 + 4 * c) * 8);
+                if (c < 2) cp16(kd + j * EX_KLD + EX_DIM + (c0 + 4 * c) * 8, rs + (c0 + 4 * c) * 8);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int i = threadIdx.x; i < EX_ROWS * 24; i += 256) {   // query rows, the last one repeated where there is none
+        const int m = i / 24, c = i - m * 24;
+        const size_t rh = (size_t) min(r0 + m, r_last) * g.heads + h;
+        cp16(sq + m * EX_KLD + c * 8, c < 16 ? (const bf16*) a.qn + rh * EX_DIM + c * 8 : (const bf16*) a.qf + rh * kld + RP + (c - 16) * 8);
+    }
+    for (int i = 0; i < EX_ST - 1; ++i) fetch(i);
+
+    uint32_t fq[12][4];
+    float o[16][4];
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[n][i] = 0.0f;
+    float m_run[2] = {NEG_BIG, NEG_BIG}, l_run[2] = {0.0f, 0.0f};
+    const int ra = warp * 16 + (lane >> 2), pa = pos0 + ra, pb = pa + 8;         // this lane's rows and their positions
+    const float sc = a.scale * LOG2E;
+    for (int t = 0; t < n_tiles; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(EX_ST - 2) : "memory");
+        __syncthreads();                                      // tile t is staged; every warp is done with tile t - 1
+        if (t == 0) {
+#pragma unroll
+            for (int k = 0; k < 12; ++k) ldsm4(fq[k], sq + (warp * 16 + (lane & 15)) * EX_KLD + (lane >> 4) * 8 + k * 16);
+        }
+        fetch(t + EX_ST - 1);
+        const bf16* kt = ring + (t % EX_ST) * EX_STAGE;
+        const bf16* vt = kt + EX_BK * EX_KLD;
+        const int k0 = lo + t * EX_BK, first = pos0 + warp * 16, last = first + 15;       // positions of the warp's rows
+        if (k0 > last || k0 + EX_BK - 1 <= first - a.window) continue;                    // no key of the tile is seen by a row of the warp
+        float s[8][4];
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[n][i] = 0.0f;
+        const bf16* kb = kt + ((lane & 7) + (lane >> 4) * 8) * EX_KLD + ((lane >> 3) & 1) * 8;
+#pragma unroll
+        for (int k = 0; k < 12; ++k)
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                uint32_t fb[4];
+                ldsm4(fb, kb + n * 8 * EX_KLD + k * 16);
+                skd::mma_bf16(s[n], fq[k][0], fq[k][1], fq[k][2], fq[k][3], fb[0], fb[1]);
+                skd::mma_bf16(s[n + 1], fq[k][0], fq[k][1], fq[k][2], fq[k][3], fb[2], fb[3]);
+            }
+        // scaled scores in powers of two; masked where the tile crosses the newest position or the window's far edge of a row
+        const bool edge = k0 + EX_BK - 1 > first || k0 <= last - a.window;
+        float mx[2] = {m_run[0], m_run[1]};
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int key = k0 + n * 8 + 2 * (lane & 3) + (i & 1), p = i < 2 ? pa : pb;
+                s[n][i] = !edge || (key <= p && p - key < a.window) ? s[n][i] * sc : -INFINITY;
+                mx[i >> 1] = fmaxf(mx[i >> 1], s[n][i]);
+            }
+        float al[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            mx[r] = fmaxf(mx[r], __shfl_xor_sync(~0u, mx[r], 1)); mx[r] = fmaxf(mx[r], __shfl_xor_sync(~0u, mx[r], 2));
+            al[r] = exp2f(m_run[r] - mx[r]);
+            m_run[r] = mx[r]; l_run[r] *= al[r];
+        }
+        uint32_t fp[4][4];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float e0 = exp2f(s[n][0] - mx[0]), e1 = exp2f(s[n][1] - mx[0]), e2 = exp2f(s[n][2] - mx[1]), e3 = exp2f(s[n][3] - mx[1]);
+            l_run[0] += e0 + e1; l_run[1] += e2 + e3;
+            fp[n >> 1][2 * (n & 1)] = skd::pack_bf16(e0, e1); fp[n >> 1][2 * (n & 1) + 1] = skd::pack_bf16(e2, e3);
+        }
+        if (__any_sync(~0u, al[0] != 1.0f || al[1] != 1.0f))             // a running maximum moved
+#pragma unroll
+            for (int n = 0; n < 16; ++n) { o[n][0] *= al[0]; o[n][1] *= al[0]; o[n][2] *= al[1]; o[n][3] *= al[1]; }
+        const bf16* vb = vt + ((lane & 7) + ((lane >> 3) & 1) * 8) * EX_VLD + (lane >> 4) * 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int n = 0; n < 16; n += 2) {
+                uint32_t fb[4];
+                ldsm4_t(fb, vb + k * 16 * EX_VLD + n * 8);
+                skd::mma_bf16(o[n], fp[k][0], fp[k][1], fp[k][2], fp[k][3], fb[0], fb[1]);
+                skd::mma_bf16(o[n + 1], fp[k][0], fp[k][1], fp[k][2], fp[k][3], fb[2], fb[3]);
+            }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        l_run[r] += __shfl_xor_sync(~0u, l_run[r], 1); l_run[r] += __shfl_xor_sync(~0u, l_run[r], 2);
+        const int row = r0 + ra + 8 * r;
+        if (row >= a.rows) continue;
+        const float f = a.gates[(size_t) row * g.heads + h] / l_run[r];
+        bf16* d = (bf16*) a.out + (size_t) row * g.out_ld() + h * EX_DIM + 2 * (lane & 3);
+#pragma unroll
+        for (int n = 0; n < 16; ++n) *(uint32_t*) (d + n * 8) = skd::pack_bf16(o[n][2 * r] * f, o[n][2 * r + 1] * f);
+    }
+}
+
 constexpr int ROWS_BK = 64;
 template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_rows_kernel(const LatentArgs a, int n_splits) {
@@ -548,6 +686,15 @@ int32_t launch_latent_attention(const LatentArgs& args, cudaStream_t s) {
         if (a.f32_act) SK_CUDA(launch_pdl(latent_prep_kernel<float>, dim3(a.rows), dim3(256), 0, s, a));
         else SK_CUDA(launch_pdl(latent_prep_kernel<bf16>, dim3(a.rows), dim3(256), 0, s, a));
         LinearArgs l;
+        if (a.kv && a.map.seq >= 0 && a.rows >= LATENT_EXPAND_ROWS) {
+            // keys and values of the cache slots in use, then attention over them; out is final
+            l.w = a.ukv; l.w_rows = g.heads * 2 * g.dim; l.ldw = g.rank_ld(); l.x = (const bf16*) a.cache.rows + (size_t) a.map.seq * a.cache.cap * g.key_ld(); l.ldx = g.key_ld();
+            l.x_rows_alloc = a.cache.cap; l.rows = std::min(a.cache.cap, a.kv_bound); l.y = a.kv; l.ldy = l.w_rows; l.out = LIN_OUT_ACT;
+            SK_TRY(launch_linear_bf16(l, s));
+            SK_TRY(ensure_dynamic_smem((const void*) latent_attn_expanded_kernel, EX_SMEM));
+            SK_CUDA(launch_pdl(latent_attn_expanded_kernel, dim3(g.heads, (a.rows + EX_ROWS - 1) / EX_ROWS), dim3(256), EX_SMEM, s, a));
+            return SKAINET_CUDA_OK;
+        }
         l.w = a.uk_t; l.w_rows = g.kv_rank; l.ldw = g.dim_ld(); l.groups = g.heads; l.x = a.qn; l.ldx = g.heads * g.dim_ld(); l.x_group_stride = g.dim_ld();
         l.x_rows_alloc = a.rows_alloc; l.rows = a.rows; l.y = a.qf; l.ldy = g.heads * g.key_ld(); l.y_group_stride = g.key_ld(); l.f32_act = a.f32_act; l.out = LIN_OUT_ACT;
         SK_TRY(launch_linear_bf16(l, s));

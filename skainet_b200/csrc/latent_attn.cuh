@@ -4,8 +4,8 @@
 //   score(i, j, h) = ( q_h . (W_uk,h c_j) + qr_h . kr_j ) * scale = ( (W_uk,h^T q_h) . c_j + qr_h . kr_j ) * scale
 //   out(i, h)      = W_uv,h ( sum_j p_ij c_j ) * sigmoid(gate_h)
 //
-// W_uk is folded into the query and W_uv applied to the mixed latent, in prompts and in decoding alike: attention then reads
-// one [latent | rotated part] row per key for all heads, and a cached row is never expanded.
+// W_uk is folded into the query and W_uv applied to the mixed latent: attention then reads one [latent | rotated part] row per key
+// for all heads. Passes of many prompt rows expand the cached rows instead, once per pass, and attend keys and values per head.
 #pragma once
 #include "linear_bf16.cuh"
 #include "rowmap.cuh"
@@ -47,6 +47,8 @@ struct LatentArgs {
     float *gates = nullptr;               // sigmoid gates, [row][heads]
     float *part = nullptr;                // key-split records, [row][head][split][rank_pad + 2]
     const bf16 *uk_t = nullptr, *uv = nullptr;   // [heads][kv_rank][dim_ld], [heads][vdim][rank_ld]
+    const bf16* ukv = nullptr;            // expanded form: W_uk, then W_uv, [2][heads * dim][rank_ld]
+    void* kv = nullptr;                   // and room for the keys and values of a sequence's cache slots, [cap][2][heads * dim]; null: not taken
     int rows = 0, rows_alloc = 0;
     RowMap map = {nullptr, -1};
     int kv_bound = 0;                     // bound on the sequence length after this step
@@ -54,6 +56,10 @@ struct LatentArgs {
 };
 
 constexpr int LATENT_FUSED_ROWS = 4;      // rows up to which the folds of W_uk and W_uv run inside the kernels around attention
+// The expanded form's geometry, and the prompt rows from which forming the keys and values pays.
+constexpr bool latent_expands(const LatentGeom& g) { return g.dim == 128 && g.rot_dim == 64 && g.vdim == 128 && g.kv_rank % 64 == 0; }
+constexpr int LATENT_EXPAND_ROWS = 192;
+constexpr size_t LATENT_EXPAND_MAX_BYTES = (size_t) 256 << 20;
 constexpr int LATENT_PART_RECORDS = 64 * 320;
 
 // proj -> rotation, latent norm, cache append, gates, folded query, attention over the cache, gated heads in a.out.

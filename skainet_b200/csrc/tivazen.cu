@@ -53,6 +53,7 @@ struct TvLayer {
     const float *cos_t = nullptr, *sin_t = nullptr;
     AttnBuffers buf;
     void* hidden = nullptr;
+    Weight* ukv = nullptr;                // W_uk and W_uv stacked, for prompts (laid out by finalize)
 };
 
 const bf16* data(const Weight* w) { return (const bf16*) w->qs; }
@@ -67,12 +68,12 @@ struct Tivazen : Decoder {
     std::set<std::tuple<int, int, int>> missing;       // (layer, matrix | 100 + vector, expert) not set yet
     // per row in flight
     float *x = nullptr, *states = nullptr, *proj = nullptr, *gates = nullptr, *y = nullptr, *part = nullptr, *z = nullptr;
-    void *act = nullptr, *act_sorted = nullptr, *act_final = nullptr;
+    void *act = nullptr, *act_sorted = nullptr, *act_final = nullptr, *kv = nullptr;
     int32_t* want = nullptr;
     RouteBuffers route;
 
     ~Tivazen() override {
-        for (auto& L : layers) for (Weight* w : {L.proj, L.uk, L.uv, L.o, L.router, L.gate, L.up, L.down}) if (w) weight_release(w);
+        for (auto& L : layers) for (Weight* w : {L.proj, L.uk, L.uv, L.o, L.router, L.gate, L.up, L.down, L.ukv}) if (w) weight_release(w);
         if (embed) weight_release(embed);
         if (head) weight_release(head);
     }
@@ -90,6 +91,24 @@ struct Tivazen : Decoder {
                       std::get<0>(k), std::get<2>(k));
             return SKAINET_CUDA_ERR_INVALID;
         }
+        return expand_weights();
+    }
+    // W_uk back in its own orientation, with W_uv below it, for the layers whose prompts take the expanded form of attention; the room
+    // for the widest of their caches is shared, since a layer uses it within its own attention only.
+    int32_t expand_weights() {
+        size_t room = 0;
+        for (auto& L : layers) {
+            const LatentGeom& g = L.geom;
+            const size_t bytes = (size_t) L.cache.cap * g.heads * 2 * g.dim * 2;
+            if (f32 || L.ukv || !latent_expands(g) || max_rows < LATENT_EXPAND_ROWS || bytes > LATENT_EXPAND_MAX_BYTES) continue;
+            SK_TRY(weight_alloc(SKAINET_ENC_BF16, g.heads * 2 * g.dim, g.kv_rank, &L.ukv));
+            bf16* dst = (bf16*) L.ukv->qs;
+            SK_TRY(launch_transpose_heads(data(L.uk), dst, g.heads, g.kv_rank, g.dim, nullptr));
+            SK_CUDA(cudaMemcpy(dst + (size_t) g.heads * g.dim * g.rank_ld(), L.uv->qs, (size_t) g.heads * g.vdim * g.rank_ld() * 2, cudaMemcpyDeviceToDevice));
+            room = std::max(room, bytes);
+        }
+        if (room && !kv) SK_TRY(alloc(&kv, room));
+        SK_CUDA(cudaStreamSynchronize(nullptr));
         return SKAINET_CUDA_OK;
     }
     int32_t enqueue_decode(int batch, int kv_bound, cudaStream_t s) override {
@@ -255,6 +274,7 @@ int32_t Tivazen::body(int rows, RowMap map, int kv_bound, cudaStream_t s) {
         a.owner = L.owner == (int) i; a.norm = L.dkv_norm; a.cos_t = L.cos_t; a.sin_t = L.sin_t; a.cache = L.cache;
         a.qn = L.buf.qn; a.qf = L.buf.qf; a.mix = L.buf.mix; a.out = L.buf.out; a.gates = gates; a.part = part;
         a.uk_t = data(L.uk); a.uv = data(L.uv); a.rows = rows; a.rows_alloc = max_rows; a.map = map; a.kv_bound = kv_bound; a.f32_act = f32;
+        if (L.ukv) { a.ukv = data(L.ukv); a.kv = kv; }
         SK_TRY(launch_latent_attention(a, s));
         l.w = data(L.o); l.w_rows = d_model; l.ldw = l.ldx = L.geom.out_ld(); l.x = L.buf.out; l.y = y; l.ldy = d_model;
         SK_TRY(launch_linear_bf16(l, s));
