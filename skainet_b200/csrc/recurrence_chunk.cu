@@ -9,7 +9,7 @@
 //
 //   recur_conv_kernel      convolution and silu in fp32, rounded to bf16; inverse lengths of q and k, step sizes, log decays.
 //   recur_inverse_kernel   T of every chunk and head: column-wise substitution in fp32.
-//   recur_scan_kernel      one CTA per head and 32 or 64 state columns walks the chunks; the state stays in registers (fp32).
+//   recur_scan_kernel      one CTA per head and 16, 32 or 64 state columns walks the chunks; the state stays in registers (fp32).
 //
 // Exactness: q, k, v behind the convolution are bf16, everything after it is 32-bit. The tensor cores see fp32 factors as sums of
 // three bf16 terms (24 bits); the lengths, decays and step sizes are applied outside the products, so q, k, v enter as one exact
@@ -28,7 +28,13 @@ namespace {
 constexpr int CH = 64;                       // tokens of a chunk
 constexpr int CONV_ROWS = 16;
 
-int state_cols(const RecurGeom& g) { return !g.delta && g.vdim > 32 && g.kdim <= 128 ? 64 : 32; }
+// State columns of a CTA of the scan: the walk over the chunks is serial, so what is left to spread over the SMs is heads and columns.
+// Wide pieces share the products of keys and queries; half as wide where that still leaves every CTA an SM of its own
+// (16 heads x 128 columns on 128 CTAs instead of 64: a 2048-token prompt of the 2B Fomalix shape 14.67 against 15.66 ms).
+int state_cols(const RecurGeom& g) {
+    const int cols = !g.delta && g.vdim > 32 && g.kdim <= 128 ? 64 : 32;
+    return g.vdim >= cols && 2 * g.heads * ((g.vdim + cols - 1) / cols) <= sm_count() ? cols / 2 : cols;
+}
 
 // Work buffers, all padded to whole chunks with zeros.
 struct Work {
@@ -280,7 +286,7 @@ struct ScanShape {
 template <bool DELTA, int VT, int KT>
 __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, const Work w) {
     typedef ScanShape<DELTA, VT, KT> Z;
-    constexpr int NT = VT / 8, LV = Z::LV;
+    constexpr int NT = VT / 8, LV = Z::LV, NF = NT < 4 ? NT : 4;      // NF: 8-column sums in flight
     const RecurGeom& g = a.g;
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ double sG[2][CH];
@@ -395,16 +401,16 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 uint32_t f[4];
                 skd::ldsm4(f, a_at + ks * 32);
 #pragma unroll
-                for (int n = 0; n < NT; n += 4) {                   // four sums in flight
-                    uint32_t bb[3][2][4];
+                for (int n = 0; n < NT; n += NF) {
+                    uint32_t bb[3][NF / 2][4];
 #pragma unroll
                     for (int j = 0; j < 3; ++j)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) skd::ldsm4_t(bb[j][e], s_at + j * s_term + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
+                        for (int e = 0; e < NF / 2; ++e) skd::ldsm4_t(bb[j][e], s_at + j * s_term + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
 #pragma unroll
                     for (int j = 2; j >= 0; --j)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) skd::mma_bf16(acc[n + e], f[0], f[1], f[2], f[3], bb[j][e >> 1][2 * (e & 1)], bb[j][e >> 1][2 * (e & 1) + 1]);
+                        for (int e = 0; e < NF; ++e) skd::mma_bf16(acc[n + e], f[0], f[1], f[2], f[3], bb[j][e >> 1][2 * (e & 1)], bb[j][e >> 1][2 * (e & 1) + 1]);
                 }
             }
         }
@@ -434,16 +440,16 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
 #pragma unroll
                     for (int i = 0; i < 3; ++i) skd::ldsm4(f[i], t_at + ((i * CH + mt * 16 + lr + l8 * 8) * Z::LT + ks * 16 + l16 * 8) * 2);
 #pragma unroll
-                    for (int n = 0; n < NT; n += 4)
+                    for (int n = 0; n < NT; n += NF)
 #pragma unroll
                         for (int j = 2; j >= 0; --j) {
-                            uint32_t bb[2][4];
+                            uint32_t bb[NF / 2][4];
 #pragma unroll
-                            for (int e = 0; e < 2; ++e) skd::ldsm4_t(bb[e], w_at + j * Z::V_TERM + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
+                            for (int e = 0; e < NF / 2; ++e) skd::ldsm4_t(bb[e], w_at + j * Z::V_TERM + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
 #pragma unroll
                             for (int i = 2 - j; i >= 0; --i)
 #pragma unroll
-                                for (int e = 0; e < 4; ++e) skd::mma_bf16(acc[n + e], f[i][0], f[i][1], f[i][2], f[i][3], bb[e >> 1][2 * (e & 1)], bb[e >> 1][2 * (e & 1) + 1]);
+                                for (int e = 0; e < NF; ++e) skd::mma_bf16(acc[n + e], f[i][0], f[i][1], f[i][2], f[i][3], bb[e >> 1][2 * (e & 1)], bb[e >> 1][2 * (e & 1) + 1]);
                         }
                 }
 #pragma unroll
@@ -545,16 +551,16 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 skd::split3(p[2 * ks][0], p[2 * ks][1], f[0]); skd::split3(p[2 * ks][2], p[2 * ks][3], f[1]);
                 skd::split3(p[2 * ks + 1][0], p[2 * ks + 1][1], f[2]); skd::split3(p[2 * ks + 1][2], p[2 * ks + 1][3], f[3]);
 #pragma unroll
-                for (int n = 0; n < NT; n += 4)
+                for (int n = 0; n < NT; n += NF)
 #pragma unroll
                     for (int j = DELTA ? 2 : 0; j >= 0; --j) {
-                        uint32_t bb[2][4];
+                        uint32_t bb[NF / 2][4];
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) skd::ldsm4_t(bb[e], (DELTA ? u_at + j * Z::V_TERM : v) + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
+                        for (int e = 0; e < NF / 2; ++e) skd::ldsm4_t(bb[e], (DELTA ? u_at + j * Z::V_TERM : v) + bt_off + (ks * 16 * LV + (n + 2 * e) * 8) * 2);
 #pragma unroll
                         for (int i = 2 - j; i >= 0; --i)
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) skd::mma_bf16(acc[n + e], f[0][i], f[1][i], f[2][i], f[3][i], bb[e >> 1][2 * (e & 1)], bb[e >> 1][2 * (e & 1) + 1]);
+                            for (int e = 0; e < NF; ++e) skd::mma_bf16(acc[n + e], f[0][i], f[1][i], f[2][i], f[3][i], bb[e >> 1][2 * (e & 1)], bb[e >> 1][2 * (e & 1) + 1]);
                     }
             }
 #pragma unroll
@@ -621,14 +627,15 @@ int32_t launch_recur_chunks(const RecurArgs& a, cudaStream_t s) {
         SK_TRY(ensure_dynamic_smem((const void*) recur_conv_kernel, conv_bytes));
         SK_CUDA(launch_pdl(recur_conv_kernel, dim3(w.rows / CONV_ROWS, 2 * g.groups + g.heads), dim3(256), conv_bytes, s, a, w));
     }
-    if (!g.delta) {
-        if (state_cols(g) == 64) return run_scan<false, 64, 2>(a, w, s);
-        return w.kp <= 128 ? run_scan<false, 32, 2>(a, w, s) : run_scan<false, 32, 4>(a, w, s);
-    }
+    const int cols = state_cols(g);
+    const bool wide_keys = w.kp > 128;
+    if (!g.delta)
+        return cols == 64 ? run_scan<false, 64, 2>(a, w, s) : cols == 32 ? (wide_keys ? run_scan<false, 32, 4>(a, w, s) : run_scan<false, 32, 2>(a, w, s))
+                                                           : (wide_keys ? run_scan<false, 16, 4>(a, w, s) : run_scan<false, 16, 2>(a, w, s));
     const int inv_bytes = CH * (w.kp + 8) * 2 + CH * INV_LD * 4;
     SK_TRY(ensure_dynamic_smem((const void*) recur_inverse_kernel, inv_bytes));
     SK_CUDA(launch_pdl(recur_inverse_kernel, dim3(w.rows / CH, g.heads), dim3(128), inv_bytes, s, a, w));
-    return w.kp <= 128 ? run_scan<true, 32, 2>(a, w, s) : run_scan<true, 32, 4>(a, w, s);
+    return cols == 32 ? (wide_keys ? run_scan<true, 32, 4>(a, w, s) : run_scan<true, 32, 2>(a, w, s)) : (wide_keys ? run_scan<true, 16, 4>(a, w, s) : run_scan<true, 16, 2>(a, w, s));
 }
 
 }  // namespace sk
