@@ -26,7 +26,9 @@ namespace sk {
 
 namespace {
 
-constexpr int PREFILL_ROWS = 1024;       // rows of one prompt pass unless the configuration says otherwise
+// Rows of one prompt pass unless the configuration says otherwise. 2048 tokens in one pass instead of two take 11.44 ms instead of
+// 14.5 (2B shape): the 128-row tiles of the linears fill 4.8 rounds of SMs instead of 2.4, and half as many kernels are started.
+constexpr int PREFILL_ROWS = 2048;
 
 // Where a matrix or vector of the checkpoint goes.
 struct MatrixSlot { Weight* w = nullptr; int row0 = 0, rows = 0, cols = 0; };

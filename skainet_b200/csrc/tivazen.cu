@@ -24,7 +24,9 @@ namespace sk {
 
 namespace {
 
-constexpr int PREFILL_ROWS = 1024;       // rows of one prompt pass unless the configuration says otherwise
+// Rows of one prompt pass unless the configuration says otherwise. 2048 tokens in one pass instead of two take 9.77 ms instead of
+// 12.76 (2B shape): the 128-row tiles of the linears fill 4.8 rounds of SMs instead of 2.4, and half as many kernels are started.
+constexpr int PREFILL_ROWS = 2048;
 
 // Seeded noise in a sequence's cache rows; the zero tails stay zero.
 template <typename T>
