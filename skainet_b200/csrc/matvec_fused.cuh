@@ -38,13 +38,15 @@ int32_t launch_matvec_ring(const Weight& w, const MatvecIn& in, int prep, float*
 // gemm_mma.cu: y[m][w.rows] (= resid +) for m >= 2 quantized activation rows on the tensor cores; 1 = not taken
 int32_t launch_gemm_mma(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 int32_t launch_gemm_mma_q8(const Weight& w, ActSplit a, int m, float* y, const float* resid, cudaStream_t s);
-// Fewest activation rows sent to the tcgen05 kernel. Its call has a floor (activation tile preparation + one wave of
-// 128 x 128 tiles): measured per call on the 25 MB shapes, tcgen05 / mma.sync: 128 rows 86 / 64 us, 256 rows 108 / 95,
-// 384 rows 111 / 131, 512 rows 132 / 176.
-constexpr int TC_MIN_ROWS = 288;
+// Rows from which the tcgen05 kernel is considered (fewer: the matvec and ring kernels), and from which it is taken whatever the shape;
+// between them it is where its call is expected to cost less than the mma.sync tile kernel's. Measured per call, tcgen05 / mma.sync, us:
+// 4096 x 11008 at 64 rows 26.8 / 65.6, at 128 32.0 / 70.5; 4096 x 4096 at 64 rows 16.9 / 22.1; 11008 x 4096 at 32 rows 26.0 / 28.0, at 128
+// 37.3 / 53.9; the other way 22016 x 4096 at 32 rows 47.0 / 30.0, 4096 x 1024 at 64 rows 12.2 / 8.9.
+constexpr int TC_MIN_ROWS = 9, TC_ALWAYS_ROWS = 288;
 // gemm_ring.cu: 2..8 activation rows over a Q4_K weight through the persistent ring; 1 = not taken
 int32_t launch_rows_ring(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
-// gemm_tc.cu: the same for m >= 128 on tcgen05 with TMEM accumulators; 1 = not taken
+// gemm_tc.cu: the same for m >= TC_MIN_ROWS on tcgen05 with TMEM accumulators; 1 = not taken
+size_t gemm_tc_scratch_bytes(int m, int cols);
 int32_t launch_gemm_tc(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 
 }  // namespace sk

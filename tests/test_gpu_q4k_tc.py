@@ -1,0 +1,42 @@
+"""The tcgen05 kernel of Q4_K rows (csrc/gemm_tc.cu) at the edges of its tiles (32, 64 and 128 activation rows and one more, 128 weight
+rows), with one super-block, with fewer super-blocks than a cluster has parts, and with odd numbers of them.
+
+Bar: the integer sums of a super-block are exact, what differs from the oracle is the order of the fp32 sums over super-blocks (and
+of the parts of a cluster): 1e-5 of the largest of an element and the outputs' root mean square, as for the other kernels of this format."""
+import numpy as np
+import pytest
+
+from conftest import rel_err_ok
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k", [(1, 256), (127, 768), (129, 1280), (300, 4352)])
+@pytest.mark.parametrize("m", [9, 32, 33, 64, 65, 128, 129, 257])
+def test_tile_edges(gpu, oracle, n, k, m):
+    rng = np.random.default_rng(n + k + m)
+    w_bytes = oracle.quantize_q4k((0.02 * rng.standard_normal((n, k))).astype(np.float32))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[0, :256] = 0.0
+    w = gpu.Weight.upload(w_bytes, "Q4_K", n, k)
+    got = gpu.matmul_host(w, x)
+    rel_err_ok(got, oracle.matmul("Q4_K", x, w_bytes, k, n, "rm", use_ref=oracle.ref() is not None), 1e-5)
+    assert np.array_equal(got, gpu.matmul_host(w, x))
+    w.free()
+
+
+@pytest.mark.parametrize("n,k,m", [(300, 1024, 20), (5000, 512, 64), (20000, 512, 140), (11008, 1024, 512)])
+def test_back_to_back_calls_with_other_inputs(gpu, n, k, m):
+    """Calls that follow each other at once, each with rows of its own, through the same scratch: every call starts before the one before
+    it has left the GPU, and none may see its operands."""
+    rng = np.random.default_rng(n)
+    w = gpu.Weight.synth("Q4_K", n, k, seed=5, std=0.02)
+    xs = [gpu.DeviceBuffer.from_host(((10.0 ** (j % 3)) * rng.standard_normal((m, k))).astype(np.float32)) for j in range(6)]
+    ys = [gpu.DeviceBuffer(4 * m * n) for _ in xs]
+    want = [gpu.matmul_host(w, x.download(np.float32, m * k).reshape(m, k)) for x in xs]
+    for _ in range(5):
+        for x, y in zip(xs, ys):
+            gpu.matmul(w, x.ptr, m, y.ptr)
+    for y, ref in zip(ys, want):
+        assert np.array_equal(y.download(np.float32, m * n).reshape(m, n), ref)
+    w.free()
