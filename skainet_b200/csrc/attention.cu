@@ -145,8 +145,9 @@ __device__ __forceinline__ float4 rope_load4(const float* __restrict__ base, int
     return f;
 }
 
-template <int D, bool FUSE>
-__global__ void __launch_bounds__(AM_WARPS * 32)
+// W warps: eight, one CTA per SM; or four, two CTAs per SM, for grids of more CTAs than SMs over short contexts.
+template <int D, bool FUSE, int W = AM_WARPS>
+__global__ void __launch_bounds__(W * 32)
 attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const __half* __restrict__ kc, const __half* __restrict__ vc,
                        float* __restrict__ part, int heads, int kv_heads, int G, int64_t cache_stride,
                        const int32_t* __restrict__ kv_len, float scale, int window, int chunk, int splits, float* __restrict__ out_direct,
@@ -155,7 +156,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
     constexpr int KS = D / 16;     // k-steps of the score contraction
     constexpr int U = D / 64;      // chunks of a V row per lane
     constexpr int NT = D / 8;      // 8-dim output tiles
-    constexpr int NP = AM_WARPS + (FUSE ? 1 : 0);      // partial records merged per CTA: one per warp (+ the token's own key)
+    constexpr int NP = W + (FUSE ? 1 : 0);      // partial records merged per CTA: one per warp (+ the token's own key)
     __shared__ float sm_m[NP][8], sm_l[NP][8], sm_c[NP][8];
     __shared__ uint32_t sm_q[KS][4][32];
     __shared__ float sm_acc[NP][8][D + 4];
@@ -204,7 +205,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
             for (int u = 0; u < U; ++u) vr[kk][u] = key < stop ? skd::ld_stream(vb + slot_of(key) * D + (g + 8 * u) * 8) : zero4;
         }
     };
-    constexpr int STEP = AM_WARPS * 16;
+    constexpr int STEP = W * 16;
     int k0 = begin + warp * 16;
     if (k0 < stop) load_tile(krA, vrA, k0);          // in flight while q is fetched and split below
     if (k0 + STEP < stop) load_tile(krB, vrB, k0 + STEP);
@@ -212,7 +213,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
     // q of head g as A fragments, per k-step {hi(k 2t..), lo(k 2t..), hi(k 2t+8..), lo(k 2t+8..)}: warp w
     // converts k-step w (k-step 2s+j covers floats 4j..4j+3 of chunk t+4s) and all warps read the result.
     const int pos_new = len - 1;                       // FUSE: the position being decoded
-    for (int ks = warp; ks < KS; ks += AM_WARPS) {
+    for (int ks = warp; ks < KS; ks += W) {
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
         if (g < G) {
             const float* qrow = q + (int64_t) b * q_row_stride + (int64_t) (kvh * G + g) * D;
@@ -226,7 +227,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
     }
     if (FUSE) {
         // the token's own key and value: rotated / rounded to binary16 exactly as the cache will hold them, appended by
-        // the owner CTA, and entered as partial record AM_WARPS (score of head hg against the new key, weight 1, its value)
+        // the owner CTA, and entered as partial record W (score of head hg against the new key, weight 1, its value)
         if (owner) {
             const float* krow = step.qkv + (int64_t) b * q_row_stride + (int64_t) (heads + kvh) * D;
             const float* vrow = step.qkv + (int64_t) b * q_row_stride + (int64_t) (heads + kv_heads + kvh) * D;
@@ -248,16 +249,16 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
                 *reinterpret_cast<__half2*>(vdst + e0) = v01; *reinterpret_cast<__half2*>(vdst + e0 + 2) = v23;
                 const float2 a = __half22float2(v01), c2 = __half22float2(v23);
 #pragma unroll
-                for (int hg = 0; hg < 8; ++hg) { sm_acc[AM_WARPS][hg][e0] = a.x; sm_acc[AM_WARPS][hg][e0 + 1] = a.y; sm_acc[AM_WARPS][hg][e0 + 2] = c2.x; sm_acc[AM_WARPS][hg][e0 + 3] = c2.y; }
+                for (int hg = 0; hg < 8; ++hg) { sm_acc[W][hg][e0] = a.x; sm_acc[W][hg][e0 + 1] = a.y; sm_acc[W][hg][e0 + 2] = c2.x; sm_acc[W][hg][e0 + 3] = c2.y; }
             }
         } else {
-            for (int i = threadIdx.x; i < 8 * (D + 4); i += AM_WARPS * 32) (&sm_acc[AM_WARPS][0][0])[i] = 0.0f;
+            for (int i = threadIdx.x; i < 8 * (D + 4); i += W * 32) (&sm_acc[W][0][0])[i] = 0.0f;
         }
     }
     __syncthreads();
     if (FUSE) {
-        // warp hg: score of head hg against the new key (fp32 rotated q, the cache's binary16 key)
-        const int hg = warp;
+        // score of head hg against the new key (fp32 rotated q, the cache's binary16 key), a warp per head at a time
+        for (int hg = warp; hg < 8; hg += W) {
         float sc_new = MASKED;
         if (owner && hg < G) {
             const float* qrow = q + (int64_t) b * q_row_stride + (int64_t) (kvh * G + hg) * D;
@@ -269,7 +270,8 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
             }
             sc_new = skd::warp_sum(p) * scale;
         }
-        if (lane == 0) { sm_m[AM_WARPS][hg] = sc_new; sm_l[AM_WARPS][hg] = (owner && hg < G) ? 1.0f : 0.0f; }
+        if (lane == 0) { sm_m[W][hg] = sc_new; sm_l[W][hg] = (owner && hg < G) ? 1.0f : 0.0f; }
+        }
     }
     uint32_t qa[KS][4];
 #pragma unroll
@@ -358,7 +360,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
     }
     __syncthreads();
     const bool direct = out_direct != nullptr;
-    for (int idx = threadIdx.x; idx < G * D; idx += AM_WARPS * 32) {
+    for (int idx = threadIdx.x; idx < G * D; idx += W * 32) {
         const int hg = idx / D, dd = idx % D;
         float at = 0.0f;
 #pragma unroll
@@ -381,6 +383,12 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
     }
 }
 
+// More (sequence, cache head) pairs than SMs: with one CTA of eight warps per SM they run in waves, and short contexts spend a wave on a
+// prologue and a tile or two. Four warps a CTA let two CTAs share an SM: 64 x 8 pairs over 96 keys 13.0 -> 9.7 us, over 512 29.0 -> 26.4,
+// over 1024 (64 wide) 32.3 -> 28.2; eight decode steps of the 7B shape side by side gain 2 %. Over long contexts the waves even out and eight
+// warps stream better: 20 x 8 pairs over 2048 keys 34 against 40 us, 64 x 8 over 4096 135 against 143.
+constexpr int NARROW_MAX_KEYS = 1024;
+static bool narrow_ctas(int batch, int kv_heads, int max_kv_len) { return (int64_t) batch * kv_heads > sm_count() && max_kv_len <= NARROW_MAX_KEYS; }
 // Fewest keys a split is given: one 16-key tile per warp of the split-K kernel.
 static int attn_min_keys() { return 128; }
 int decode_splits(int batch, int kv_heads, int max_kv_len) {
@@ -452,7 +460,9 @@ static void launch_decode_dg(const float* q, const __half* k, const __half* v, f
                              int ring_cap, cudaStream_t s) {
     dim3 grid(splits, kv_heads, batch);
     const bool direct = splits == 1 && !always_partials;
-    launch_pdl(attn_decode_mma_kernel<D, false>, grid, dim3(AM_WARPS * 32), 0, s, q, q_row_stride, k, v, part, heads, kv_heads, G, cache_stride, kv_len,
+    if (narrow_ctas(batch, kv_heads, max_len)) launch_pdl(attn_decode_mma_kernel<D, false, 4>, grid, dim3(128), 0, s, q, q_row_stride, k, v, part, heads, kv_heads, G, cache_stride, kv_len,
+               scale, window, chunk, splits, direct ? out : (float*) nullptr, max_len, ring_start, ring_cap, AttnStep());
+    else launch_pdl(attn_decode_mma_kernel<D, false>, grid, dim3(AM_WARPS * 32), 0, s, q, q_row_stride, k, v, part, heads, kv_heads, G, cache_stride, kv_len,
                scale, window, chunk, splits, direct ? out : (float*) nullptr, max_len, ring_start, ring_cap, AttnStep());
     if (!always_partials && !direct) launch_pdl(attn_merge_kernel<D>, dim3(batch * heads), dim3(D * MG), 0, s, (const float*) part, out, splits);
 }
@@ -496,12 +506,12 @@ int32_t launch_attn_step(const float* qkv, __half* k, __half* v, float* out, int
     st.qkv = qkv; st.cos_t = cos_t; st.sin_t = sin_t; st.kc_w = k; st.vc_w = v; st.rope_mode = rope_mode;
     const int64_t stride = (int64_t) (heads + 2 * kv_heads) * d;
     dim3 grid(splits, kv_heads, batch);
-    if (d == 128)
-        SK_CUDA(launch_pdl(attn_decode_mma_kernel<128, true>, grid, dim3(AM_WARPS * 32), 0, s, qkv, stride, (const __half*) k, (const __half*) v, (float*) scratch,
-                           heads, kv_heads, G, cache_stride, kv_len, scale, window, chunk, splits, (float*) nullptr, std::max(1, max_kv_len), 0, 0, st));
-    else
-        SK_CUDA(launch_pdl(attn_decode_mma_kernel<64, true>, grid, dim3(AM_WARPS * 32), 0, s, qkv, stride, (const __half*) k, (const __half*) v, (float*) scratch,
-                           heads, kv_heads, G, cache_stride, kv_len, scale, window, chunk, splits, (float*) nullptr, std::max(1, max_kv_len), 0, 0, st));
+    auto launch = [&](auto kernel, int warps) {
+        return launch_pdl(kernel, grid, dim3(warps * 32), 0, s, qkv, stride, (const __half*) k, (const __half*) v, (float*) scratch, heads, kv_heads, G, cache_stride, kv_len,
+                          scale, window, chunk, splits, (float*) nullptr, std::max(1, max_kv_len), 0, 0, st);
+    };
+    if (narrow_ctas(batch, kv_heads, max_kv_len)) SK_CUDA(d == 128 ? launch(attn_decode_mma_kernel<128, true, 4>, 4) : launch(attn_decode_mma_kernel<64, true, 4>, 4));
+    else SK_CUDA(d == 128 ? launch(attn_decode_mma_kernel<128, true>, AM_WARPS) : launch(attn_decode_mma_kernel<64, true>, AM_WARPS));
     dim3 mgrid(heads * d / 256, batch);
     if (d == 128) {
         if (split) SK_CUDA(launch_pdl(attn_merge_quant_kernel<128, true>, mgrid, dim3(256 * MG), 0, s, (const float*) scratch, out, splits, heads, oq, os));
