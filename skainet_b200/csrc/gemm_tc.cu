@@ -310,8 +310,6 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             for (int e = 0; e < PER; ++e)
 #pragma unroll
                 for (int c = 0; c < 2; ++c) q[e][c] = skd::lds128(wrow + (((2 * (my + 2 * e) + c) ^ (r & 7)) << 4));
-            __syncwarp();
-            if (lane == 0) mbar_arrive1(w_empty + s);
             uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
             skd::k4_unpack(hd.y, hd.z, hd.w, sc_lo, sc_hi, mn_lo, mn_hi);
             bool ok = true;
@@ -358,7 +356,14 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) { mbar_arrive1(a_full + h); if (writes_mins && e == PER - 1) mbar_arrive1(s2_full + (i & 3)); }
+                if (lane == 0) {
+                    mbar_arrive1(a_full + h);
+                    // The weight slot goes back only now that what was read from it lies in TMEM. Given back right behind the reads, the next
+                    // tile could overtake them: at 32 and 64 rows of 11008 x 4096 up to 15 of 100 queued calls had a warp's 32 rows of a
+                    // group from the super-block WS further on.
+                    if (e == PER - 1) mbar_arrive1(w_empty + s);
+                    if (writes_mins && e == PER - 1) mbar_arrive1(s2_full + (i & 3));
+                }
             }
             if (!ok) break;
             if (my == 0) {
