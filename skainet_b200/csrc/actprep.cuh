@@ -45,14 +45,14 @@ __device__ __forceinline__ void q8k_prep_to_smem(const MatvecIn& in, int cols, i
     if (PREP == PREP_QUANTIZED) {
         for (int c = tid; c < (cols >> 4); c += NT) {
             const int blk = c >> 4, ch = c & 15;
-            *reinterpret_cast<uint4*>(s_q8 + (size_t) blk * 256 + (ch ^ (((blk >> 1) & 1) << 1)) * 16) = skd::ld_ro(in.q8.q + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_q8 + (size_t) blk * 256 + (ch ^ (((blk >> 1) & 1) << 1)) * 16) = skd::ld_dep16(in.q8.q + (size_t) c * 16);
         }
         for (int c = tid; c < (cols >> 5); c += NT) {
-            const int sum = (int) __ldg(in.q8.bsums + c), hi = (sum + 64) >> 7, lo = sum - (hi << 7);
+            const int sum = (int) skd::ld_dep(in.q8.bsums + c), hi = (sum + 64) >> 7, lo = sum - (hi << 7);
             int8_t* dst = s_bs + (size_t) (c >> 3) * 16 + ((c >> 2) & 1) * 8 + (c & 3);
             dst[0] = (int8_t) hi; dst[4] = (int8_t) lo;
         }
-        for (int c = tid; c < bpr; c += NT) s_d[c] = __ldg(in.q8.d + c);
+        for (int c = tid; c < bpr; c += NT) s_d[c] = skd::ld_dep(in.q8.d + c);
         return;
     }
     constexpr int B = 4;     // blocks per warp per batch: 8 float4 loads in flight per lane
@@ -65,8 +65,8 @@ __device__ __forceinline__ void q8k_prep_to_smem(const MatvecIn& in, int cols, i
             for (int j = 0; j < B; ++j) {
                 const int blk = b0 + j * NW;
                 if (blk < bpr) {
-                    v[2 * j] = __ldg(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + lane);
-                    v[2 * j + 1] = __ldg(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + 32 + lane);
+                    v[2 * j] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + lane);
+                    v[2 * j + 1] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + 32 + lane);
                 } else { v[2 * j] = make_float4(0, 0, 0, 0); v[2 * j + 1] = v[2 * j]; }
             }
 #pragma unroll
@@ -81,15 +81,15 @@ __device__ __forceinline__ void q8k_prep_to_smem(const MatvecIn& in, int cols, i
         for (int j = 0; j < B; ++j) {
             const int blk = b0 + j * NW;
             if (blk < bpr) {
-                v[2 * j] = __ldg(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + lane);
-                v[2 * j + 1] = __ldg(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + 32 + lane);
+                v[2 * j] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + lane);
+                v[2 * j + 1] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + (size_t) blk * 256) + 32 + lane);
                 if (PREP == PREP_NORM_F32) {
                     g[2 * j] = __ldg(reinterpret_cast<const float4*>(in.gamma + (size_t) blk * 256) + lane);
                     g[2 * j + 1] = __ldg(reinterpret_cast<const float4*>(in.gamma + (size_t) blk * 256) + 32 + lane);
                 }
                 if (PREP == PREP_SWIGLU_F32) {       // the "up" half follows the "gate" half of the row
-                    g[2 * j] = __ldg(reinterpret_cast<const float4*>(in.x + cols + (size_t) blk * 256) + lane);
-                    g[2 * j + 1] = __ldg(reinterpret_cast<const float4*>(in.x + cols + (size_t) blk * 256) + 32 + lane);
+                    g[2 * j] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + cols + (size_t) blk * 256) + lane);
+                    g[2 * j + 1] = skd::ld_dep(reinterpret_cast<const float4*>(in.x + cols + (size_t) blk * 256) + 32 + lane);
                 }
             } else { v[2 * j] = make_float4(0, 0, 0, 0); v[2 * j + 1] = v[2 * j]; g[2 * j] = v[2 * j]; g[2 * j + 1] = v[2 * j]; }
         }
@@ -146,10 +146,10 @@ __device__ __forceinline__ void split_prep_to_smem(const MatvecIn& in, int cols,
     constexpr int NT = NW * 32;
     if (PREP == PREP_QUANTIZED) {
         for (int c = tid; c < (cols >> 4); c += NT) {
-            *reinterpret_cast<uint4*>(s_hi + (size_t) c * 16) = skd::ld_ro(in.split.hi + (size_t) c * 16);
-            *reinterpret_cast<uint4*>(s_lo + (size_t) c * 16) = skd::ld_ro(in.split.lo + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_hi + (size_t) c * 16) = skd::ld_dep16(in.split.hi + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_lo + (size_t) c * 16) = skd::ld_dep16(in.split.lo + (size_t) c * 16);
         }
-        for (int c = tid; c < bpr; c += NT) s_dx[c] = __ldg(in.split.d + c);
+        for (int c = tid; c < bpr; c += NT) s_dx[c] = skd::ld_dep(in.split.d + c);
         return;
     }
     constexpr int B = 8;     // float4 loads in flight per thread
@@ -162,7 +162,7 @@ __device__ __forceinline__ void split_prep_to_smem(const MatvecIn& in, int cols,
 #pragma unroll
             for (int j = 0; j < B; ++j) {
                 const int i = i0 + j * NT;
-                v[j] = i < n4 ? __ldg(reinterpret_cast<const float4*>(in.x) + i) : make_float4(0, 0, 0, 0);
+                v[j] = i < n4 ? skd::ld_dep(reinterpret_cast<const float4*>(in.x) + i) : make_float4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int j = 0; j < B; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
@@ -178,7 +178,7 @@ __device__ __forceinline__ void split_prep_to_smem(const MatvecIn& in, int cols,
         for (int j = 0; j < B; ++j) {
             const int i = i0 + j * NT;
             const bool ok = i < n4;
-            v[j] = ok ? __ldg(reinterpret_cast<const float4*>(in.x) + i) : make_float4(0, 0, 0, 0);
+            v[j] = ok ? skd::ld_dep(reinterpret_cast<const float4*>(in.x) + i) : make_float4(0, 0, 0, 0);
             if (PREP == PREP_NORM_F32) g[j] = ok ? __ldg(reinterpret_cast<const float4*>(in.gamma) + i) : make_float4(0, 0, 0, 0);
         }
 #pragma unroll

@@ -58,8 +58,8 @@ __device__ __forceinline__ void quant_q8k_regs(const float (&v)[8], int8_t* q_ou
     if (lane == 0) *d_out = amax > 0.0f ? amax / 127.0f : 0.0f;
 }
 __device__ __forceinline__ void quant_q8k_block(const float* x, int8_t* q_out, float* d_out, int16_t* bsums_out, int lane) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(x) + lane * 2);
-    const float4 b = __ldg(reinterpret_cast<const float4*>(x) + lane * 2 + 1);
+    const float4 a = skd::ld_dep(reinterpret_cast<const float4*>(x) + lane * 2);
+    const float4 b = skd::ld_dep(reinterpret_cast<const float4*>(x) + lane * 2 + 1);
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     quant_q8k_regs(v, q_out, d_out, bsums_out, lane);
 }
@@ -90,8 +90,8 @@ __device__ __forceinline__ void quant_split_regs(const float (&v)[8], sk::ActSpl
     }
 }
 __device__ __forceinline__ void quant_split_block(const float* x, sk::ActSplit a, int64_t blk, int part, bool live) {
-    const float4 p = __ldg(reinterpret_cast<const float4*>(x + blk * 32 + part * 8));
-    const float4 q = __ldg(reinterpret_cast<const float4*>(x + blk * 32 + part * 8) + 1);
+    const float4 p = skd::ld_dep(reinterpret_cast<const float4*>(x + blk * 32 + part * 8));
+    const float4 q = skd::ld_dep(reinterpret_cast<const float4*>(x + blk * 32 + part * 8) + 1);
     const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
     quant_split_regs(v, a, blk, part, live);
 }

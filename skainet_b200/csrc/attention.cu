@@ -30,7 +30,7 @@ namespace sk {
 // the merged output element to the threads of group 0; the other groups get 0.
 constexpr int MG = 4;          // split groups per CTA
 template <int D, int E>        // E = elements per CTA
-__device__ __forceinline__ float merge_splits(const float* __restrict__ rec, int splits, int dd, int e, int grp, float (*sm)[MG][E]) {
+__device__ __forceinline__ float merge_splits(const float* rec, int splits, int dd, int e, int grp, float (*sm)[MG][E]) {
     float mx = MASKED, lt = 0.0f, at = 0.0f;
     for (int s0 = grp * 8; s0 < splits; s0 += MG * 8) {
         float mm[8], ll[8], aa[8];
@@ -38,9 +38,9 @@ __device__ __forceinline__ float merge_splits(const float* __restrict__ rec, int
         for (int i = 0; i < 8; ++i) {
             const bool live = s0 + i < splits;
             const float* r = rec + (int64_t) (s0 + i) * (D + 2);
-            mm[i] = live ? __ldg(r) : MASKED;
-            ll[i] = live ? __ldg(r + 1) : 0.0f;
-            aa[i] = live ? __ldg(r + 2 + dd) : 0.0f;
+            mm[i] = live ? skd::ld_dep(r) : MASKED;
+            ll[i] = live ? skd::ld_dep(r + 1) : 0.0f;
+            aa[i] = live ? skd::ld_dep(r + 2 + dd) : 0.0f;
         }
         float cm = mx;
 #pragma unroll
@@ -72,7 +72,7 @@ __device__ __forceinline__ float merge_splits(const float* __restrict__ rec, int
 
 // grid batch*heads, D*MG threads
 template <int D>
-__global__ void __launch_bounds__(D * MG) attn_merge_kernel(const float* __restrict__ part, float* __restrict__ out, int splits) {
+__global__ void __launch_bounds__(D * MG) attn_merge_kernel(const float* part, float* __restrict__ out, int splits) {
     __shared__ float sm[3][MG][D];
     skd::pdl_launch_dependents();
     skd::pdl_wait();
@@ -121,9 +121,9 @@ __device__ __forceinline__ void rope_pair(float& x, float& y, float c, float sn)
 }
 // Four consecutive elements [e0, e0+4) of a head row at `base`, rotated for position p.
 template <int D>
-__device__ __forceinline__ float4 rope_load4(const float* __restrict__ base, int e0, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__device__ __forceinline__ float4 rope_load4(const float* base, int e0, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                              int p, int mode) {
-    float4 f = __ldg((const float4*) (base + e0));
+    float4 f = skd::ld_dep((const float4*) (base + e0));
     const float* cr = cos_t + (size_t) p * (D / 2);
     const float* sr = sin_t + (size_t) p * (D / 2);
     if (mode == 0) {
@@ -133,7 +133,7 @@ __device__ __forceinline__ float4 rope_load4(const float* __restrict__ base, int
     } else {
         const bool lower = e0 < D / 2;
         const int i = lower ? e0 : e0 - D / 2;
-        float4 o = __ldg((const float4*) (base + (lower ? e0 + D / 2 : e0 - D / 2)));
+        float4 o = skd::ld_dep((const float4*) (base + (lower ? e0 + D / 2 : e0 - D / 2)));
         float* fa = &f.x; float* oa = &o.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -148,9 +148,9 @@ __device__ __forceinline__ float4 rope_load4(const float* __restrict__ base, int
 // W warps: eight, one CTA per SM; or four, two CTAs per SM, for grids of more CTAs than SMs over short contexts.
 template <int D, bool FUSE, int W = AM_WARPS>
 __global__ void __launch_bounds__(W * 32)
-attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const __half* __restrict__ kc, const __half* __restrict__ vc,
+attn_decode_mma_kernel(const float* q, int64_t q_row_stride, const __half* __restrict__ kc, const __half* __restrict__ vc,
                        float* __restrict__ part, int heads, int kv_heads, int G, int64_t cache_stride,
-                       const int32_t* __restrict__ kv_len, float scale, int window, int chunk, int splits, float* __restrict__ out_direct,
+                       const int32_t* kv_len, float scale, int window, int chunk, int splits, float* __restrict__ out_direct,
                        int max_len, int ring_start, int ring_cap, AttnStep step) {
     constexpr int S4 = D / 32;     // chunks of a K row per lane
     constexpr int KS = D / 16;     // k-steps of the score contraction
@@ -166,7 +166,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
 
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int len = min(__ldg(kv_len + b), max_len);      // never past what the launch was sized (and the cache allocated) for
+    const int len = min(skd::ld_dep(kv_len + b), max_len);      // never past what the launch was sized (and the cache allocated) for
     int first = 0;
     if (window > 0 && len - window > first) first = len - window;
     // FUSE: the newest key (index len - 1) is not in the cache yet; the CTA whose split would hold it appends it and
@@ -218,7 +218,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
         if (g < G) {
             const float* qrow = q + (int64_t) b * q_row_stride + (int64_t) (kvh * G + g) * D;
             const int e0 = (t + 4 * (ks >> 1)) * 8 + 4 * (ks & 1);
-            f = FUSE ? rope_load4<D>(qrow, e0, step.cos_t, step.sin_t, pos_new, step.rope_mode) : __ldg((const float4*) (qrow + e0));
+            f = FUSE ? rope_load4<D>(qrow, e0, step.cos_t, step.sin_t, pos_new, step.rope_mode) : skd::ld_dep((const float4*) (qrow + e0));
         }
         uint32_t h0, l0, h1, l1;
         split_pack(f.x, f.y, h0, l0);
@@ -244,7 +244,7 @@ attn_decode_mma_kernel(const float* __restrict__ q, int64_t q_row_stride, const 
                 sm_knew[e0] = a.x; sm_knew[e0 + 1] = a.y; sm_knew[e0 + 2] = c2.x; sm_knew[e0 + 3] = c2.y;
             } else if (threadIdx.x < D / 2) {
                 const int e0 = (threadIdx.x - D / 4) * 4;
-                const float4 vf = __ldg((const float4*) (vrow + e0));
+                const float4 vf = skd::ld_dep((const float4*) (vrow + e0));
                 const __half2 v01 = __floats2half2_rn(vf.x, vf.y), v23 = __floats2half2_rn(vf.z, vf.w);
                 *reinterpret_cast<__half2*>(vdst + e0) = v01; *reinterpret_cast<__half2*>(vdst + e0 + 2) = v23;
                 const float2 a = __half22float2(v01), c2 = __half22float2(v23);
@@ -413,7 +413,7 @@ size_t attn_scratch_bytes(int batch, int heads, int head_dim, int max_kv_len) {
 // well. grid (heads*D/256, batch), 256*MG threads (MG split groups, see merge_splits).
 template <int D, bool SPLIT>
 __global__ void __launch_bounds__(256 * MG)
-attn_merge_quant_kernel(const float* __restrict__ part, float* __restrict__ out, int splits, int heads, ActQ8K oq, ActSplit os) {
+attn_merge_quant_kernel(const float* part, float* __restrict__ out, int splits, int heads, ActQ8K oq, ActSplit os) {
     __shared__ float red[8];
     __shared__ float sm[3][MG][256];
     skd::pdl_launch_dependents();
@@ -683,8 +683,8 @@ int32_t launch_sdpa_f32(const float* q, const float* k, const float* v, float* o
 // =================================================================================================
 template <int D>
 __global__ void __launch_bounds__(AM_WARPS * 32)
-attn_prefill_mma_kernel(const float* __restrict__ q, const __half* __restrict__ kc, const __half* __restrict__ vc, float* __restrict__ out,
-                        int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* __restrict__ q_abs_base,
+attn_prefill_mma_kernel(const float* q, const __half* kc, const __half* vc, float* __restrict__ out,
+                        int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* q_abs_base,
                         float scale, int window) {
     constexpr int S4 = D / 32, KS = D / 16, U = D / 64, NT = D / 8;
     __shared__ float sm_m[AM_WARPS][8], sm_l[AM_WARPS][8], sm_c[AM_WARPS][8];
@@ -696,7 +696,7 @@ attn_prefill_mma_kernel(const float* __restrict__ q, const __half* __restrict__ 
     const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / (heads / kv_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int base = __ldg(q_abs_base + b);
+    const int base = skd::ld_dep(q_abs_base + b);
     const int nq = min(8, seq_q - qt * 8);                        // live query rows of this tile
     // row g: keys [first_g, end_g); the CTA walks [begin, stop)
     const int qi = qt * 8 + g;
@@ -714,13 +714,13 @@ attn_prefill_mma_kernel(const float* __restrict__ q, const __half* __restrict__ 
         for (int nt = 0; nt < 2; ++nt) {
             const int key = k0 + 8 * nt + g;
 #pragma unroll
-            for (int s = 0; s < S4; ++s) kr[nt][s] = key < stop ? skd::ld_ro(kb + (int64_t) key * D + (t + 4 * s) * 8) : zero4;
+            for (int s = 0; s < S4; ++s) kr[nt][s] = key < stop ? skd::ld_dep16(kb + (int64_t) key * D + (t + 4 * s) * 8) : zero4;
         }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             const int key = k0 + 2 * t + (kk & 1) + 8 * (kk >> 1);
 #pragma unroll
-            for (int u = 0; u < U; ++u) vr[kk][u] = key < stop ? skd::ld_ro(vb + (int64_t) key * D + (g + 8 * u) * 8) : zero4;
+            for (int u = 0; u < U; ++u) vr[kk][u] = key < stop ? skd::ld_dep16(vb + (int64_t) key * D + (g + 8 * u) * 8) : zero4;
         }
     };
     constexpr int STEP = AM_WARPS * 16;
@@ -730,7 +730,7 @@ attn_prefill_mma_kernel(const float* __restrict__ q, const __half* __restrict__ 
 
     for (int ks = warp; ks < KS; ks += AM_WARPS) {
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (g < nq) f = __ldg((const float4*) (q + (((int64_t) b * seq_q + qi) * heads + h) * D + (t + 4 * (ks >> 1)) * 8 + 4 * (ks & 1)));
+        if (g < nq) f = skd::ld_dep((const float4*) (q + (((int64_t) b * seq_q + qi) * heads + h) * D + (t + 4 * (ks >> 1)) * 8 + 4 * (ks & 1)));
         uint32_t h0, l0, h1, l1;
         split_pack(f.x, f.y, h0, l0);
         split_pack(f.z, f.w, h1, l1);
@@ -841,8 +841,8 @@ template <int D> constexpr int ap_smem() { return 2 * 2 * AP_BK * (D + 8) * 2; }
 
 template <int D>
 __global__ void __launch_bounds__(AP_THREADS, 2)
-attn_prompt_kernel(const float* __restrict__ q, const __half* __restrict__ kc, const __half* __restrict__ vc, float* __restrict__ out,
-                   int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* __restrict__ q_abs_base, float scale, int window, int parts) {
+attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __restrict__ out,
+                   int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* q_abs_base, float scale, int window, int parts) {
     constexpr int KS = D / 16, NT = D / 8, LD = D + 8, STAGE = 2 * AP_BK * LD, OLD = D + 4;
     static_assert(AP_ROWS * (OLD + 2) * 4 <= 2 * STAGE * 2, "the records take the place of the ring");
     extern __shared__ __align__(16) uint8_t smem[];
@@ -851,7 +851,7 @@ attn_prompt_kernel(const float* __restrict__ q, const __half* __restrict__ kc, c
     skd::pdl_wait();
     const int h = blockIdx.x / parts, part = blockIdx.x % parts, q0 = (gridDim.y - 1 - blockIdx.y) * AP_ROWS, b = blockIdx.z, kvh = h / (heads / kv_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int base = __ldg(q_abs_base + b), q_last = min(q0 + AP_ROWS, seq_q) - 1;
+    const int base = skd::ld_dep(q_abs_base + b), q_last = min(q0 + AP_ROWS, seq_q) - 1;
     const int hi = base + q_last, lo = window > 0 ? max(0, base + q0 - window + 1) : 0, n_all = (hi - lo) / AP_BK + 1;
     const int t_first = (int) ((int64_t) n_all * part / parts), t_end = (int) ((int64_t) n_all * (part + 1) / parts);      // this part's tiles
     const __half* kb = kc + ((int64_t) b * kv_heads + kvh) * cache_stride * D;
@@ -877,7 +877,7 @@ attn_prompt_kernel(const float* __restrict__ q, const __half* __restrict__ kc, c
         const float* qb = q + (((int64_t) b * seq_q + min(rb, q_last)) * heads + h) * D + 2 * t;
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
-            const float2 f[4] = {__ldg((const float2*) (qa + ks * 16)), __ldg((const float2*) (qb + ks * 16)), __ldg((const float2*) (qa + ks * 16 + 8)), __ldg((const float2*) (qb + ks * 16 + 8))};
+            const float2 f[4] = {skd::ld_dep((const float2*) (qa + ks * 16)), skd::ld_dep((const float2*) (qb + ks * 16)), skd::ld_dep((const float2*) (qa + ks * 16 + 8)), skd::ld_dep((const float2*) (qb + ks * 16 + 8))};
 #pragma unroll
             for (int j = 0; j < 4; ++j) split_pack(f[j].x, f[j].y, qh[ks][j], ql[ks][j]);
         }

@@ -178,6 +178,33 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
     return r;
 }
 __device__ __forceinline__ uint4 ld_ro(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+// A read of what an earlier launch has written, for kernels that start early (launch_pdl), behind their pdl_wait(). Never through the
+// read-only path (__ldg, ld.global.nc, or a plain read of a `const __restrict__` argument, for which the compiler takes that path
+// by itself): it may be used only for what nobody writes while the kernel runs, and such a kernel has begun while its predecessor still
+// writes and the launch before that still reads the buffer's last contents into L1. Ordinary loads are ordered behind the wait; volatile,
+// so that the compiler leaves them there too. (Past L1, ld.global.cg, costs where neighbouring loads share sectors: 0.5 us a quantizer call,
+// 1.3 % of a 512-token prompt of the 7B shape.)
+template <typename T>
+__device__ __forceinline__ T ld_dep(const T* p) {
+    static_assert(sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "one load");
+    union U { T t; uint16_t h; uint32_t w[4]; __device__ U() {} } u;
+    if constexpr (sizeof(T) == 2) asm volatile("ld.global.u16 %0, [%1];" : "=h"(u.h) : "l"(p));
+    else if constexpr (sizeof(T) == 4) asm volatile("ld.global.u32 %0, [%1];" : "=r"(u.w[0]) : "l"(p));
+    else if constexpr (sizeof(T) == 8) asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(u.w[0]), "=r"(u.w[1]) : "l"(p));
+    else asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
+    return u.t;
+}
+__device__ __forceinline__ uint4 ld_dep16(const void* p) { return ld_dep(reinterpret_cast<const uint4*>(p)); }
+// The same for the compiler to place where it likes behind the wait: of a pointer that behind_wait() has made known there.
+template <typename T>
+__device__ __forceinline__ T* behind_wait(T* p) { asm volatile("" : "+l"(p)); return p; }
+__device__ __forceinline__ uint32_t ld_free(const uint32_t* p) { uint32_t v; asm("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ float ld_free(const float* p) { float v; asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint4 ld_free(const uint4* p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 
 // ggml get_scale_min_k4 on the three scale words of a Q4_K/Q5_K header:
 // sc[0..3] | sc[4..7] | mn[0..3] | mn[4..7], one value per byte.

@@ -15,7 +15,7 @@ namespace sk {
 // Arg max per row (lowest index on ties) + bookkeeping of the step: the token becomes the next
 // step's input, is recorded in the output log, and the sequence position advances.
 __global__ void __launch_bounds__(1024)
-argmax_advance_kernel(const float* __restrict__ logits, int cols, int32_t* __restrict__ cur_token, int32_t* __restrict__ pos,
+argmax_advance_kernel(const float* logits, int cols, int32_t* __restrict__ cur_token, int32_t* __restrict__ pos,
                       int32_t* __restrict__ log, int32_t* __restrict__ log_cursor, int batch) {
     __shared__ float sv[32];
     __shared__ int si[32];
@@ -55,7 +55,7 @@ __global__ void bump_cursor_kernel(int32_t* cursor) { skd::pdl_launch_dependents
 
 // Row-wise arg max of a vocabulary shard -> (value, global index) pairs, for the TP merge.
 __global__ void __launch_bounds__(1024)
-argmax_pairs_kernel(const float* __restrict__ logits, int cols, int idx_offset, float* __restrict__ vals, int32_t* __restrict__ idxs) {
+argmax_pairs_kernel(const float* logits, int cols, int idx_offset, float* __restrict__ vals, int32_t* __restrict__ idxs) {
     __shared__ float sv[32];
     __shared__ int si[32];
     skd::pdl_launch_dependents();
@@ -85,7 +85,7 @@ argmax_pairs_kernel(const float* __restrict__ logits, int cols, int idx_offset, 
 // finish_step_kernel picks among them (lowest index on ties, as the reference's arg max does).
 constexpr int ARGMAX_CHUNKS = 32;
 __global__ void __launch_bounds__(256)
-argmax_chunks_kernel(const float* __restrict__ logits, int cols, int chunk_cols, float2* __restrict__ out, int batch) {
+argmax_chunks_kernel(const float* logits, int cols, int chunk_cols, float2* __restrict__ out, int batch) {
     __shared__ float sv[8];
     __shared__ int si[8];
     skd::pdl_launch_dependents();
@@ -112,8 +112,8 @@ argmax_chunks_kernel(const float* __restrict__ logits, int cols, int chunk_cols,
     }
 }
 // pairs[world][batch] as (float, int) interleaved 8-byte records -> token per row, then the step's bookkeeping
-__global__ void finish_step_kernel(const float2* __restrict__ pairs, int world, int batch, int32_t* __restrict__ cur_token,
-                                   int32_t* __restrict__ pos, int32_t* __restrict__ log, const int32_t* __restrict__ log_cursor) {
+__global__ void finish_step_kernel(const float2* pairs, int world, int batch, int32_t* __restrict__ cur_token,
+                                   int32_t* __restrict__ pos, int32_t* __restrict__ log, const int32_t* log_cursor) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;

@@ -224,13 +224,13 @@ static ActF16Split act_f16split_layout(const void* scratch, int m, int cols) {
 
 // One warp per 256 activation elements: lane l holds elements 8 l .. 8 l + 7, four lanes make one 32-element sum.
 __global__ void __launch_bounds__(256)
-act_f16split_kernel(const float* __restrict__ x, int64_t nblocks, __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ sums) {
+act_f16split_kernel(const float* x, int64_t nblocks, __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ sums) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const int64_t blk = (blockIdx.x * (int64_t) blockDim.x + threadIdx.x) >> 5;
     if (blk >= nblocks) return;
     const int lane = threadIdx.x & 31;
-    const float4 v0 = __ldg(reinterpret_cast<const float4*>(x + blk * 256) + 2 * lane), v1 = __ldg(reinterpret_cast<const float4*>(x + blk * 256) + 2 * lane + 1);
+    const float4 v0 = skd::ld_dep(reinterpret_cast<const float4*>(x + blk * 256) + 2 * lane), v1 = skd::ld_dep(reinterpret_cast<const float4*>(x + blk * 256) + 2 * lane + 1);
     const float e[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     uint32_t ph[4], pl[4];
     float sum = 0.0f;

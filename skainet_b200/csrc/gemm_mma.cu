@@ -56,7 +56,7 @@ __device__ __forceinline__ void mma_u8s8(int (&c)[4], const uint32_t (&a)[4], ui
 template <int NW, int NT, int NS, int EPI>
 __global__ void __launch_bounds__(NW * 32)
 q4k_gemm_mma_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr, int rows, int bpr, ActQ8K act, int m,
-                    float* __restrict__ y, const float* __restrict__ resid) {
+                    float* __restrict__ y, const float* resid) {
     constexpr int RT = NW * 16, MT = NT * 8;
     constexpr int W_BYTES = RT * GW_STRIDE, X_BYTES = MT * GX_STRIDE, S_BYTES = W_BYTES + X_BYTES + MT * 4;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -239,7 +239,7 @@ __device__ __forceinline__ void mma_s8s8(int (&c)[4], const uint32_t (&a)[4], ui
 template <int NW, int NT, int NS, int EPI>
 __global__ void __launch_bounds__(NW * 32)
 q8_0_gemm_mma_kernel(const int8_t* __restrict__ codes, const __half* __restrict__ scales, int rows, int cols, ActSplit act, int m,
-                     float* __restrict__ y, const float* __restrict__ resid) {
+                     float* __restrict__ y, const float* resid) {
     constexpr int RT = NW * 16, MT = NT * 8, ST = 272;
     constexpr int W_BYTES = RT * ST, X_BYTES = MT * ST, S_BYTES = W_BYTES + 2 * X_BYTES;
     extern __shared__ __align__(128) uint8_t smem[];

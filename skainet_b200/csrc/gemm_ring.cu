@@ -56,7 +56,7 @@ __device__ __forceinline__ void gr_group_sync(int grp) {
 template <int NG, int EPI, bool XG>
 __global__ void __launch_bounds__(NG * GR_GW * 32)
 q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr, int rows, int bpr, ActQ8K act, int m,
-                     float* __restrict__ y, const float* __restrict__ resid, int nstages, int x_stride, int* __restrict__ timeout_flag) {
+                     float* __restrict__ y, const float* resid, int nstages, int x_stride, int* __restrict__ timeout_flag) {
     extern __shared__ __align__(128) uint8_t smem[];
     // layout: rings [NG][nstages][GR_STAGE] | activation rows [8][x_stride] | block scales [8][bpr] | partial tiles [NG][2][4][128] | barriers
     const int lane = threadIdx.x & 31;
@@ -107,18 +107,21 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
 
     // ---------------- consumers ----------------
     skd::pdl_wait();                                   // the quantized activation rows are the predecessor's output
+    const int8_t* act_q = skd::behind_wait(act.q);
+    const int16_t* act_bsums = skd::behind_wait(act.bsums);
+    const float* act_d = skd::behind_wait(act.d);
     if (!XG) {
         const int ct = (grp * GR_BLKS + warp) * 32 + lane, nct = NG * GR_BLKS * 32;          // this thread among the consumer threads of the CTA
         for (int c = ct; c < GR_MT * (cols >> 4); c += nct) {                 // 16 codes
             const int row = c / (cols >> 4), ch = c % (cols >> 4), blk = ch >> 4, k16 = ch & 15;
-            const uint4 v = row < m ? skd::ld_ro(act.q + (size_t) row * cols + (size_t) ch * 16) : make_uint4(0, 0, 0, 0);
+            const uint4 v = row < m ? skd::ld_free((const uint4*) (act_q + (size_t) min(row, m - 1) * cols + (size_t) ch * 16)) : make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4*>(s_x + (size_t) row * x_stride + blk * 272 + k16 * 16) = v;
         }
         for (int c = ct; c < GR_MT * bpr; c += nct) {                         // a block's eight int16 sums and its scale
             const int row = c / bpr, blk = c % bpr;
-            const uint4 v = row < m ? skd::ld_ro(act.bsums + ((size_t) row * bpr + blk) * 8) : make_uint4(0, 0, 0, 0);
+            const uint4 v = row < m ? skd::ld_free((const uint4*) (act_bsums + ((size_t) min(row, m - 1) * bpr + blk) * 8)) : make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4*>(s_x + (size_t) row * x_stride + blk * 272 + 256) = v;
-            s_d[row * bpr + blk] = row < m ? __ldg(act.d + (size_t) row * bpr + blk) : 0.0f;
+            s_d[row * bpr + blk] = row < m ? skd::ld_free(act_d + (size_t) min(row, m - 1) * bpr + blk) : 0.0f;
         }
     }
     if (!XG) asm volatile("bar.sync 1, %0;" ::"n"(NG * GR_BLKS * 32) : "memory");
@@ -133,15 +136,15 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
     auto fetch_x = [&](int b, uint32_t (&w)[16], uint4 (&bs2)[2], float (&d2)[2]) {
         const int bb = min(b, bpr - 1);
         const bool live = g < m;
-        const int8_t* src = act.q + (size_t) min(g, m - 1) * cols + (size_t) bb * 256 + 4 * t;
+        const int8_t* src = act_q + (size_t) min(g, m - 1) * cols + (size_t) bb * 256 + 4 * t;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) w[i] = live ? __ldg(reinterpret_cast<const uint32_t*>(src + 16 * i)) : 0u;
+        for (int i = 0; i < 16; ++i) w[i] = live ? skd::ld_free(reinterpret_cast<const uint32_t*>(src + 16 * i)) : 0u;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
             const int col = 2 * t + cc;
             const bool cl = col < m;
-            bs2[cc] = cl ? skd::ld_ro(act.bsums + ((size_t) col * bpr + bb) * 8) : make_uint4(0, 0, 0, 0);
-            d2[cc] = cl ? __ldg(act.d + (size_t) col * bpr + bb) : 0.0f;
+            bs2[cc] = cl ? skd::ld_free((const uint4*) (act_bsums + ((size_t) min(col, m - 1) * bpr + bb) * 8)) : make_uint4(0, 0, 0, 0);
+            d2[cc] = cl ? skd::ld_free(act_d + (size_t) min(col, m - 1) * bpr + bb) : 0.0f;
         }
     };
     if (XG && my_rgs > 0) fetch_x(warp, xw_n, xbs_n, xd_n);

@@ -183,7 +183,7 @@ act_f16_tiles_kernel(ActQ8K act, int m, int m_pad, int cols, int nlog, __half* _
 template <int N>
 __global__ void __launch_bounds__(TcShape<N>::THREADS, 1)
 q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __restrict__ hdr, int rows, int bpr, int parts,
-                   const __half* __restrict__ xh, const __half* __restrict__ hs, const float* __restrict__ dxt, int m, int m_pad,
+                   const __half* xh, const __half* hs, const float* dxt, int m, int m_pad,
                    float* y, const float* resid, int* __restrict__ timeout_flag) {
     typedef TcShape<N> S;
     extern __shared__ uint8_t raw[];
@@ -367,8 +367,6 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             }
             if (!ok) break;
             if (my == 0) {
-                // The predecessor's output, past L1: this grid starts before the preceding call of the same kernel has left the SMs, whose reads
-                // of the same scratch may still lie there.
                 if (i == 0) { skd::pdl_wait(); if (r < N) dx = __ldcg(dxt + (size_t) kb0 * m_pad + col0 + r); }
                 if (r < N) *reinterpret_cast<float*>(smem + S::OFF_DX + ((i & 3) * N + r) * 4) = dx;
                 if (r < N && i + 1 < nk) dx = __ldcg(dxt + (size_t) (kb0 + i + 1) * m_pad + col0 + r);

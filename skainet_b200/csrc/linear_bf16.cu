@@ -240,7 +240,7 @@ linear_f32_kernel(const LinearArgs a) {
 }
 
 template <typename T>
-__global__ void gather_rows_kernel(const T* __restrict__ src, const int32_t* __restrict__ index, T* __restrict__ dst, int ld) {
+__global__ void gather_rows_kernel(const T* src, const int32_t* index, T* __restrict__ dst, int ld) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const uint4* s = reinterpret_cast<const uint4*>(src + (size_t) index[blockIdx.x] * ld);
@@ -250,7 +250,7 @@ __global__ void gather_rows_kernel(const T* __restrict__ src, const int32_t* __r
 }
 
 template <typename T>
-__global__ void to_act_kernel(const float* __restrict__ x, int cols, T* __restrict__ out, int ld) {
+__global__ void to_act_kernel(const float* x, int cols, T* __restrict__ out, int ld) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     for (int i = threadIdx.x; i < ld; i += blockDim.x)

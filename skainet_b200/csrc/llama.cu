@@ -39,7 +39,7 @@ constexpr int SWIGLU_PROLOGUE_MAX_COLS = SK_SWIGLU_PROLOGUE_MAX_COLS;
 // each sequence's position. grid (rows, heads + 2*kv_heads), head_dim/2 threads. The rotation factors
 // come from a table built on the host in double precision.
 __global__ void rope_append_kernel(float* __restrict__ qkv, int heads, int kv_heads, int d, const float* __restrict__ cos_t,
-                                   const float* __restrict__ sin_t, const int32_t* __restrict__ pos, __half* __restrict__ kc, __half* __restrict__ vc, int64_t cache_stride, int mode) {
+                                   const float* __restrict__ sin_t, const int32_t* pos, __half* __restrict__ kc, __half* __restrict__ vc, int64_t cache_stride, int mode) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const int row = blockIdx.x, seq = row, hh = blockIdx.y, i = threadIdx.x, half = d >> 1;
@@ -66,8 +66,8 @@ __global__ void rope_append_kernel(float* __restrict__ qkv, int heads, int kv_he
 // shape is 1536 threads; with one pair per thread and a CTA per head the 512 rows of a pass took 53 us, and 10 more for the
 // copy of q (a 512-token prompt through the 7B shape: 23.0 against 21.5 ms). grid (ceil((heads + 2 kv_heads) * d / 8 / 256), rows).
 __global__ void __launch_bounds__(256)
-rope_prompt_kernel(const float* __restrict__ qkv, float* __restrict__ q, int heads, int kv_heads, int d, const float* __restrict__ cos_t,
-                   const float* __restrict__ sin_t, const int32_t* __restrict__ pos, __half* __restrict__ kc, __half* __restrict__ vc,
+rope_prompt_kernel(const float* qkv, float* __restrict__ q, int heads, int kv_heads, int d, const float* __restrict__ cos_t,
+                   const float* __restrict__ sin_t, const int32_t* pos, __half* __restrict__ kc, __half* __restrict__ vc,
                    int64_t cache_stride, int mode) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
@@ -78,7 +78,7 @@ rope_prompt_kernel(const float* __restrict__ qkv, float* __restrict__ q, int hea
     const bool rotate = hh < heads + kv_heads;
     const int e0 = mode == 0 || !rotate ? 8 * j : 4 * j, e1 = mode == 0 || !rotate ? e0 + 4 : e0 + half;
     const float* src = qkv + ((size_t) row * (heads + 2 * kv_heads) + hh) * d;
-    float4 a = __ldg(reinterpret_cast<const float4*>(src + e0)), b = __ldg(reinterpret_cast<const float4*>(src + e1));
+    float4 a = skd::ld_dep(reinterpret_cast<const float4*>(src + e0)), b = skd::ld_dep(reinterpret_cast<const float4*>(src + e1));
     if (rotate) {
         const float4 c = __ldg(reinterpret_cast<const float4*>(cos_t + (size_t) p * half) + j), s = __ldg(reinterpret_cast<const float4*>(sin_t + (size_t) p * half) + j);
         auto turn = [](float& x, float& y, float cc, float ss) {
@@ -99,7 +99,7 @@ rope_prompt_kernel(const float* __restrict__ qkv, float* __restrict__ q, int hea
 }
 
 // q rows out of the merged q|k|v buffer into a dense [rows][heads*d] buffer (attention input).
-__global__ void gather_q_kernel(const float* __restrict__ qkv, float* __restrict__ q, int qdim, int stride) {
+__global__ void gather_q_kernel(const float* qkv, float* __restrict__ q, int qdim, int stride) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     for (int c = threadIdx.x; c < qdim; c += blockDim.x) q[(size_t) blockIdx.x * qdim + c] = qkv[(size_t) blockIdx.x * stride + c];

@@ -42,7 +42,7 @@ constexpr size_t RING_MIN_BYTES = (size_t) 20 << 20, RING_MIN_BYTES_F32_ROW = (s
 template <int RW, int PREP, int EPI>
 __global__ void __launch_bounds__(MF_THREADS)
 q4k_matvec_fused_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr, int rows, int bpr,
-                        MatvecIn in, int cols, float* __restrict__ y, const float* __restrict__ resid,
+                        MatvecIn in, int cols, float* __restrict__ y, const float* resid,
                         int* __restrict__ timeout_flag, PeerOut peer) {
     constexpr int R = MF_WARPS * RW;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -171,7 +171,7 @@ q4k_matvec_fused_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restric
 template <int RW, int PREP, int EPI>
 __global__ void __launch_bounds__(MF_THREADS)
 q8_0_matvec_fused_kernel(const int8_t* __restrict__ codes, const __half* __restrict__ scales, int rows, int cols,
-                         MatvecIn in, float* __restrict__ y, const float* __restrict__ resid, int* __restrict__ timeout_flag) {
+                         MatvecIn in, float* __restrict__ y, const float* resid, int* __restrict__ timeout_flag) {
     constexpr int R = MF_WARPS * RW;
     extern __shared__ __align__(128) uint8_t smem[];
     const int bpr = cols >> 5;

@@ -40,7 +40,7 @@ __device__ __forceinline__ int q6_code(uint32_t ql_a, uint32_t ql_b, uint32_t qh
 // F32 mode of Q6_K: one lane per element of a 32-element run.
 __global__ void __launch_bounds__(KQ_WARPS * 32)
 q6k_matvec_f32_kernel(const uint8_t* __restrict__ ql, const uint8_t* __restrict__ qh, const int8_t* __restrict__ sc, const uint8_t* __restrict__ dd,
-                      int rows, int bpr, const float* __restrict__ x, float* __restrict__ y) {
+                      int rows, int bpr, const float* x, float* __restrict__ y) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const int lane = threadIdx.x & 31, row = blockIdx.x * KQ_WARPS + (threadIdx.x >> 5), mrow = blockIdx.y;
@@ -123,7 +123,7 @@ q6k_rows_kernel(const uint8_t* __restrict__ ql, const uint8_t* __restrict__ qh, 
         for (int i = 0; i < MT; ++i) {
             if (i < mm) {
                 const int8_t* xq = act.q + (size_t) (m0 + i) * cols + (size_t) blk * 256 + e_lo;
-                const uint4 xl = skd::ld_ro(xq), xh = skd::ld_ro(xq + 64);
+                const uint4 xl = *reinterpret_cast<const uint4*>(xq), xh = *reinterpret_cast<const uint4*>(xq + 64);      // through L1, for all warps of the CTA
                 int gl = 0, gh = 0;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -134,7 +134,7 @@ q6k_rows_kernel(const uint8_t* __restrict__ ql, const uint8_t* __restrict__ qh, 
                 isum += __shfl_xor_sync(0xffffffffu, isum, 1);
                 isum += __shfl_xor_sync(0xffffffffu, isum, 2);
                 isum += __shfl_xor_sync(0xffffffffu, isum, 4);
-                const float term = __fmul_rn(__fmul_rn(cur.d, __ldg(act.d + (size_t) (m0 + i) * bpr + blk)), (float) isum);
+                const float term = __fmul_rn(__fmul_rn(cur.d, act.d[(size_t) (m0 + i) * bpr + blk]), (float) isum);
 #pragma unroll
                 for (int jb = 0; jb < 4; ++jb) {                    // the reference adds the blocks of a row in order
                     const float t = __shfl_sync(0xffffffffu, term, 8 * jb);
@@ -169,7 +169,7 @@ __device__ __forceinline__ float byte_to_float(uint32_t w, int t) {
 template <int MT>
 __global__ void __launch_bounds__(KQR_WARPS * 32)
 q5k_rows_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr, const uint8_t* __restrict__ qh,
-                int rows, int bpr, const float* __restrict__ x, int mm, float* __restrict__ y) {
+                int rows, int bpr, const float* x, int mm, float* __restrict__ y) {
     skd::pdl_launch_dependents();
     const int lane = threadIdx.x & 31, row = min((int) (blockIdx.x * KQR_WARPS + (threadIdx.x >> 5)), rows - 1);   // a warp past the end repeats the last row
     const int cols = bpr * 256, g = lane >> 3, p = 4 * (lane & 7);
@@ -219,7 +219,7 @@ q5k_rows_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr,
             for (int i = 0; i < MT; ++i) {
                 if (i < mm) {
                     const float* xb = x + (size_t) i * cols + (size_t) blk * 256 + 64 * g + p;
-                    const float4 va = __ldg(reinterpret_cast<const float4*>(xb)), vb = __ldg(reinterpret_cast<const float4*>(xb + 32));
+                    const float4 va = *reinterpret_cast<const float4*>(xb), vb = *reinterpret_cast<const float4*>(xb + 32);      // through L1, for all warps of the CTA
                     const float cs_a = (va.x * ca0 + va.y * ca1) + (va.z * ca2 + va.w * ca3), is_a = (va.x + va.y) + (va.z + va.w);
                     const float cs_b = (vb.x * cb0 + vb.y * cb1) + (vb.z * cb2 + vb.w * cb3), is_b = (vb.x + vb.y) + (vb.z + vb.w);
                     acc[i] += (cs_a * s_a - is_a * o_a) + (cs_b * s_b - is_b * o_b);

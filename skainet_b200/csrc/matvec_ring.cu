@@ -64,7 +64,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 template <int NC, int NG, int PREP, int EPI>
 __global__ void __launch_bounds__(NG * (NC + 1) * 32)
 q4k_matvec_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ hdr, int rows, int bpr, MatvecIn in,
-                       int cols, float* __restrict__ y, const float* __restrict__ resid, int nstages, int* __restrict__ timeout_flag, PeerOut peer) {
+                       int cols, float* __restrict__ y, const float* resid, int nstages, int* __restrict__ timeout_flag, PeerOut peer) {
     constexpr int S_QS = NC * 16 * 128, S_HDR = NC * 16 * 16, S_BYTES = S_QS + S_HDR;
     extern __shared__ __align__(128) uint8_t smem[];
     // NG independent groups (one producer warp + NC consumer warps, own ring and barriers each) share one copy of
@@ -221,7 +221,7 @@ constexpr int RG8_COLS = 2048;
 template <int NC, int NG, int PREP, int EPI>
 __global__ void __launch_bounds__(NG * (NC + 1) * 32)
 q8_0_matvec_ring_kernel(const int8_t* __restrict__ codes, const __half* __restrict__ scales, int rows, int cols, MatvecIn in,
-                        float* __restrict__ y, const float* __restrict__ resid, int nstages, int* __restrict__ timeout_flag) {
+                        float* __restrict__ y, const float* resid, int nstages, int* __restrict__ timeout_flag) {
     constexpr int S_CODES = NC * RG8_COLS, S_SC = NC * (RG8_COLS / 32) * 2, S_BYTES = S_CODES + S_SC;
     extern __shared__ __align__(128) uint8_t smem[];
     // NG groups (producer warp + NC consumer warps, own ring and barriers) around one staged activation, as in the Q4_K kernel

@@ -59,11 +59,11 @@ q4k_matvec_stream_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restri
         for (int c = threadIdx.x; c < nchunks; c += MS_THREADS) {
             const int blk = c >> 4, ch = c & 15;           // block (of 256 codes) across all m, chunk inside it
             const int sw = ch ^ ((((blk % bpr) >> 1) & 1) << 1);
-            *reinterpret_cast<uint4*>(s_q8 + (size_t) blk * 256 + sw * 16) = skd::ld_ro(act.q + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_q8 + (size_t) blk * 256 + sw * 16) = skd::ld_dep16(act.q + (size_t) c * 16);
         }
         const int nb16 = M * (cols >> 8);                   // 16 bytes of bsums per block
         for (int c = threadIdx.x; c < nb16; c += MS_THREADS)
-            *reinterpret_cast<uint4*>((uint8_t*) s_bs + (size_t) c * 16) = skd::ld_ro((const uint8_t*) act.bsums + (size_t) c * 16);
+            *reinterpret_cast<uint4*>((uint8_t*) s_bs + (size_t) c * 16) = skd::ld_dep16((const uint8_t*) act.bsums + (size_t) c * 16);
     }
     __syncthreads();
     if (!skd::mbar_wait_bounded(bar, 0, timeout_flag)) return;
@@ -92,7 +92,7 @@ q4k_matvec_stream_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restri
                 a_hi[k] = skd::lds128(qa + 64 * g + off_hi);
             }
             const uint2 bs = *reinterpret_cast<const uint2*>(s_bs + ((size_t) m * bpr + b) * 8 + 4 * h);
-            const float di = __ldg(act.d + (size_t) m * bpr + b);
+            const float di = skd::ld_dep(act.d + (size_t) m * bpr + b);
 #pragma unroll
             for (int r = 0; r < RW; ++r) {
                 const int rl = warp + MS_WARPS * r;
@@ -188,10 +188,10 @@ q8_0_matvec_stream_kernel(const int8_t* __restrict__ codes, const __half* __rest
     {
         const int nchunks = M * (cols >> 4);
         for (int c = threadIdx.x; c < nchunks; c += MS_THREADS) {
-            *reinterpret_cast<uint4*>(s_hi + (size_t) c * 16) = skd::ld_ro(act.hi + (size_t) c * 16);
-            *reinterpret_cast<uint4*>(s_lo + (size_t) c * 16) = skd::ld_ro(act.lo + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_hi + (size_t) c * 16) = skd::ld_dep16(act.hi + (size_t) c * 16);
+            *reinterpret_cast<uint4*>(s_lo + (size_t) c * 16) = skd::ld_dep16(act.lo + (size_t) c * 16);
         }
-        for (int c = threadIdx.x; c < M * bpr; c += MS_THREADS) s_dx[c] = __ldg(act.d + c);
+        for (int c = threadIdx.x; c < M * bpr; c += MS_THREADS) s_dx[c] = skd::ld_dep(act.d + c);
     }
     __syncthreads();
     if (!skd::mbar_wait_bounded(bar, 0, timeout_flag)) return;

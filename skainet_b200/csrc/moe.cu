@@ -34,7 +34,7 @@ __device__ __forceinline__ void pick_row(const float* z, int experts, int top, i
 }
 
 __global__ void __launch_bounds__(SMALL_SLOTS)
-route_small_kernel(const float* __restrict__ z, int rows, int experts, int top, int seg_rows, const RouteBuffers b) {
+route_small_kernel(const float* z, int rows, int experts, int top, int seg_rows, const RouteBuffers b) {
     extern __shared__ int hist[];               // [experts] counts, then exclusive offsets; [experts] segment offsets
     __shared__ int se[SMALL_SLOTS];
     __shared__ float sw[SMALL_SLOTS];
@@ -79,7 +79,7 @@ route_small_kernel(const float* __restrict__ z, int rows, int experts, int top, 
     }
 }
 
-__global__ void __launch_bounds__(256) route_pick_kernel(const float* __restrict__ z, int rows, int experts, int top, const RouteBuffers b) {
+__global__ void __launch_bounds__(256) route_pick_kernel(const float* z, int rows, int experts, int top, const RouteBuffers b) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5);

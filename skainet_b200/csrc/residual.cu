@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(RT) gated_norm_kernel(const GatedNormArgs a) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(RT) embed_rows_kernel(const bf16* __restrict__ table, int ld_, const int32_t* __restrict__ ids, int cols, int vocab,
+__global__ void __launch_bounds__(RT) embed_rows_kernel(const bf16* __restrict__ table, int ld_, const int32_t* ids, int cols, int vocab,
                                                         float* __restrict__ x, float* __restrict__ state0, T* __restrict__ act, int act_ld) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(RT) embed_rows_kernel(const bf16* __restrict__
 }
 
 template <typename T>
-__global__ void __launch_bounds__(RT) row_norm_kernel(const float* __restrict__ x, const int32_t* __restrict__ index, int cols, const float* __restrict__ gains, float gain, float eps,
+__global__ void __launch_bounds__(RT) row_norm_kernel(const float* x, const int32_t* index, int cols, const float* __restrict__ gains, float gain, float eps,
                                                          T* __restrict__ act, int act_ld) {
     __shared__ float sh[RT / 32];
     skd::pdl_launch_dependents();

@@ -18,7 +18,7 @@ namespace sk {
 // in: [rows][n] (PK_SWIGLU: [rows][2n] = gate | up).
 template <int MODE, bool SPLIT>
 __global__ void __launch_bounds__(256)
-prep_kernel(const float* __restrict__ in, const float* __restrict__ gamma, float eps, int n, ActQ8K oq, ActSplit os) {
+prep_kernel(const float* in, const float* __restrict__ gamma, float eps, int n, ActQ8K oq, ActSplit os) {
     __shared__ float red[8];
     skd::pdl_launch_dependents();
     skd::pdl_wait();
@@ -32,7 +32,7 @@ prep_kernel(const float* __restrict__ in, const float* __restrict__ gamma, float
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int i = i0 + j * 256;
-                v[j] = i < (n >> 2) ? __ldg(reinterpret_cast<const float4*>(x) + i) : make_float4(0, 0, 0, 0);
+                v[j] = i < (n >> 2) ? reinterpret_cast<const float4*>(x)[i] : make_float4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
@@ -51,7 +51,7 @@ prep_kernel(const float* __restrict__ in, const float* __restrict__ gamma, float
     const int cc = ok ? c : 0;
     float v[8];
     {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * cc), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * cc + 1);
+        const float4 a = reinterpret_cast<const float4*>(x)[2 * cc], b = reinterpret_cast<const float4*>(x)[2 * cc + 1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
     if (MODE == PK_NORM) {
@@ -61,7 +61,7 @@ prep_kernel(const float* __restrict__ in, const float* __restrict__ gamma, float
         for (int i = 0; i < 8; ++i) v[i] = (v[i] * nscale) * g[i];
     }
     if (MODE == PK_SWIGLU) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(x + n) + 2 * cc), b = __ldg(reinterpret_cast<const float4*>(x + n) + 2 * cc + 1);
+        const float4 a = reinterpret_cast<const float4*>(x + n)[2 * cc], b = reinterpret_cast<const float4*>(x + n)[2 * cc + 1];
         const float u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = (v[i] * (1.0f / (1.0f + expf(-v[i])))) * u[i];
@@ -103,7 +103,7 @@ int32_t launch_prep(int mode, const float* in, const float* gamma, float eps, in
     }
 }
 
-__global__ void add_rows_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t n) {
+__global__ void add_rows_kernel(float* __restrict__ x, const float* y, int64_t n) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) x[i] += y[i];
@@ -167,7 +167,7 @@ int32_t weight_concat_rows(const Weight* a, const Weight* b, const Weight* c, We
 }
 
 // rows [r0, r0 + n) of src[m][stride] -> dst[m][n]
-__global__ void slice_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int m, int stride, int r0, int n) {
+__global__ void slice_rows_kernel(const float* src, float* __restrict__ dst, int m, int stride, int r0, int n) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < (int64_t) m * n; i += (int64_t) gridDim.x * blockDim.x)
@@ -175,7 +175,7 @@ __global__ void slice_rows_kernel(const float* __restrict__ src, float* __restri
 }
 
 // src[m][n] -> columns [r0, r0 + n) of dst[m][stride]
-__global__ void scatter_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int m, int stride, int r0, int n) {
+__global__ void scatter_rows_kernel(const float* src, float* __restrict__ dst, int m, int stride, int r0, int n) {
     skd::pdl_launch_dependents();
     skd::pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < (int64_t) m * n; i += (int64_t) gridDim.x * blockDim.x)

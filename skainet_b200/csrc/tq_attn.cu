@@ -8,6 +8,7 @@
 // bounds the kernel is the instructions of the transform (some 900 per lane and tile), not the bytes: 8 heads x 128 over 4096
 // positions (4 bits) read 6 MB. There a call takes 13.2 us, merge included; decoding the window to HBM first and attending the
 // copy, as stores with a residual stage still do, took five launches and 38.9 us.
+#include "common.cuh"
 #include "turboquant.cuh"
 #include "attn_frag.cuh"
 #include "tma.cuh"
@@ -36,17 +37,17 @@ struct Packed {
 
 template <int EL>
 __device__ __forceinline__ void load_packed(Packed<EL>& p, const TqPlane& pl, int64_t half_row, bool live) {
-    const uint8_t* src = pl.codes + half_row * (EL / 8) * pl.bits;
+    const uint8_t* codes = pl.codes + half_row * (EL / 8) * pl.bits;
     if (EL == 64) {                // 16, 24, 32 or 64 bytes on an 8-byte boundary
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             uint2 v = make_uint2(0, 0);
-            if (live && i < pl.bits) v = __ldg(reinterpret_cast<const uint2*>(src) + i);
+            if (live && i < pl.bits) v = __ldg(reinterpret_cast<const uint2*>(codes) + i);
             p.w[2 * i] = v.x; p.w[(2 * i + 1) % (EL / 4)] = v.y;
         }
     } else {                       // 8, 12, 16 or 32 bytes on a 4-byte boundary
 #pragma unroll
-        for (int i = 0; i < 8; ++i) p.w[i] = live && i < pl.bits ? __ldg(reinterpret_cast<const uint32_t*>(src) + i) : 0u;
+        for (int i = 0; i < 8; ++i) p.w[i] = live && i < pl.bits ? __ldg(reinterpret_cast<const uint32_t*>(codes) + i) : 0u;
     }
 #pragma unroll
     for (int g = 0; g < EL / 32; ++g) {
@@ -137,7 +138,7 @@ struct Row {
 // grid (key splits, cache heads)
 template <int D>
 __global__ void __launch_bounds__(TA_WARPS * 32)
-tq_attn_decode_kernel(const float* __restrict__ q, TqPlane kp, TqPlane vp, int64_t row0, int kv_heads, int G, int len, float scale, int chunk, int splits,
+tq_attn_decode_kernel(const float* q, TqPlane kp, TqPlane vp, int64_t row0, int kv_heads, int G, int len, float scale, int chunk, int splits,
                       float* __restrict__ part, float* __restrict__ out_direct) {
     constexpr int EL = D / 2, S4 = D / 32, KS = D / 16, U = D / 64, NT = D / 8;
     __shared__ float sm_m[TA_WARPS][8], sm_l[TA_WARPS][8], sm_c[TA_WARPS][8];
@@ -165,7 +166,7 @@ tq_attn_decode_kernel(const float* __restrict__ q, TqPlane kp, TqPlane vp, int64
     // q of head g as A fragments, per k-step {hi(k 2t..), lo(k 2t..), hi(k 2t+8..), lo(k 2t+8..)} (k-step 2s+j: floats 4j.. of chunk t+4s)
     for (int ks = warp; ks < KS; ks += TA_WARPS) {
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (g < G) f = __ldg((const float4*) (q + (int64_t) (kvh * G + g) * D + (t + 4 * (ks >> 1)) * 8 + 4 * (ks & 1)));
+        if (g < G) f = skd::ld_dep((const float4*) (q + (int64_t) (kvh * G + g) * D + (t + 4 * (ks >> 1)) * 8 + 4 * (ks & 1)));
         uint4 a;
         split_pack(f.x, f.y, a.x, a.y);
         split_pack(f.z, f.w, a.z, a.w);
