@@ -3,10 +3,14 @@
 //
 // The reference's arithmetic for one 256-element super-block (native/src/q4k_matmul.c:143-251) is
 //     y += d_x * ( d_w * S1 - dmin_w * S2 ),   S1 = sum_sb sc[sb] * <codes_sb, xq_sb>,   S2 = sum_sb mn[sb] * sum(xq_sb)
-// with 4-bit codes, 6-bit sc / mn and int8 activation codes xq. Both sums are products of small integers,
-// so they are exact in f16 x f16 -> f32: the A operand carries code*sc (<= 945 < 2048, exact in f16), the
+// with 4-bit codes, 6-bit sc / mn and int8 activation codes xq. Both sums are products of small integers, exact in f16 x f16 -> f32
+// as long as their sums stay below 2^24: the A operand carries code*sc (<= 945 < 2048, exact in f16), the
 // B operand the activation codes, and one super-block is 16 MMAs of K = 16 accumulated in TMEM. S2 is one
-// more K = 16 MMA of (mn[sb] twice) x (sums of 16 codes, <= 2032). The CUDA cores only unpack nibbles into
+// more K = 16 MMA of (mn[sb] twice) x (sums of 16 codes, <= 2032). |S1| can reach 945 * 127 * 256 = 1.83 * 2^24: tiles of 32 and 64 rows
+// accumulate its halves (128 products, below 2^24) apart and add them once, which gives the integer sum rounded to fp32 as the
+// mma.sync kernel has it; tiles of 128 rows have no TMEM left for that and may lose last places of sums beyond 2^24 (all codes and
+// scales near their largest and activations of one sign: error 9.1e-8 of the result instead of 5.9e-8; normal data is not affected).
+// The CUDA cores only unpack nibbles into
 // the A operand (one LOP3 + one HFMA2 per two elements, using the 0x6400|n trick: f16(1024+n)*s - 1024*s
 // is n*s exactly under the fused rounding) and apply the three fp32 block scales once per super-block.
 //
@@ -51,8 +55,10 @@ struct TcShape {
     static constexpr int OFF_B = WS * TC_W_BYTES, OFF_S2A = OFF_B + BS * SLOT, OFF_DX = OFF_S2A + 4 * TC_S2A_BYTES, OFF_DD = OFF_DX + 4 * N * 4;
     static constexpr int OFF_BAR = OFF_DD + 4 * TC_M * 4, BARS = 2 * WS + 2 * BS + 4 + 4 + 4;
     static constexpr int SMEM = OFF_BAR + BARS * 8 + 16 + 1024;             // the dynamic area is aligned to 1024 by hand
-    static constexpr int S2_SETS = N == 128 ? 1 : 2;                        // TMEM columns: two S1 accumulators, one or two S2, four A groups of 32
-    static constexpr int COL_S2 = 2 * N, COL_A = (2 + S2_SETS) * N;
+    // TMEM columns: two sets of S1 accumulators, one for each half of a super-block where there is room, one or two of S2, four A groups of 32
+    static constexpr int S1_ACC = N == 128 ? 1 : 2, S2_SETS = N == 128 ? 1 : 2;
+    static constexpr int COL_S2 = 2 * S1_ACC * N, COL_A = COL_S2 + S2_SETS * N;
+    static_assert(COL_A + 128 <= 512, "TMEM");
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (TC_M >> 4) << 24);   // f16 x f16 -> f32, K-major both
 };
 
@@ -100,21 +106,9 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void mbar_arrive1(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(skd::smem_u32(bar)) : "memory");
 }
-// Two TMEM loads of 16 or 8 columns and the wait for them in ONE asm statement: the destination registers are only defined
+// TMEM loads of eight columns each and the wait for them in ONE asm statement: the destination registers are only defined
 // for the compiler once the wait has been issued, so no use of them can be scheduled ahead of it.
-__device__ __forceinline__ void tmem_ld_x2(uint32_t ta, uint32_t tb, float (&u)[16], float (&v)[16]) {
-    uint32_t r[16], q[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
-        : "r"(ta), "r"(tb)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(q[i]); }
-}
-__device__ __forceinline__ void tmem_ld_x2(uint32_t ta, uint32_t tb, float (&u)[8], float (&v)[8]) {
+__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t tb, float (&u)[8], float (&v)[8]) {
     uint32_t r[8], q[8];
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
@@ -126,10 +120,39 @@ __device__ __forceinline__ void tmem_ld_x2(uint32_t ta, uint32_t tb, float (&u)[
 #pragma unroll
     for (int i = 0; i < 8; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(q[i]); }
 }
+// the same of three places, eight or four columns each
+__device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, float (&u)[8], float (&v)[8], float (&w)[8]) {
+    uint32_t r[24];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%24];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%25];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%26];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
+        : "r"(ta), "r"(tb), "r"(tc)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[8 + i]); w[i] = __uint_as_float(r[16 + i]); }
+}
+__device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, float (&u)[4], float (&v)[4], float (&w)[4]) {
+    uint32_t r[12];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%12];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%13];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%14];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11])
+        : "r"(ta), "r"(tb), "r"(tc)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[4 + i]); w[i] = __uint_as_float(r[8 + i]); }
+}
 // packed fp32 pairs, each half rounded as the scalar operation
 __device__ __forceinline__ uint64_t pk2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ float2 up2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 __device__ __forceinline__ void cluster_sync_all() {
@@ -242,7 +265,8 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
                     const uint64_t db = d_b + (uint64_t) ((s * S::SLOT + h * (S::B_BYTES / 2)) >> 4);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        umma_f16_ta(tmem + set * N, tmem + S::COL_A + h * 64 + j * 8, db + (uint64_t) (((j >> 2) * (S::B_BYTES / 4) + (j & 3) * 32) >> 4), S::IDESC, (h | j) != 0 ? 1u : 0u);
+                        umma_f16_ta(tmem + (set * S::S1_ACC + (S::S1_ACC == 2 ? h : 0)) * N, tmem + S::COL_A + h * 64 + j * 8, db + (uint64_t) (((j >> 2) * (S::B_BYTES / 4) + (j & 3) * 32) >> 4),
+                                    S::IDESC, (S::S1_ACC == 2 ? j : h | j) != 0 ? 1u : 0u);
                     umma_commit(a_empty + h);
                     if (h == 1) {
                         const uint32_t a2 = skd::smem_u32(smem + S::OFF_S2A + (i & 3) * TC_S2A_BYTES), b2 = skd::smem_u32(smem + S::OFF_B + s * S::SLOT + S::B_BYTES);
@@ -377,7 +401,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     } else {
         // ------------------------------- epilogue: fold every super-block out of TMEM -------------------------------
         const int r = tid & 127, ch = (warp - S::PROD_WARPS) >> 2;      // TMEM lane = weight row; which half of the columns
-        constexpr int NC = N / 2, LD = NC == 16 ? 16 : 8;               // columns a load
+        constexpr int NC = N / 2, LD = N == 64 ? 4 : 8;                 // columns a load: as many as the registers take
         uint64_t yacc[NC / 2];
 #pragma unroll
         for (int c = 0; c < NC / 2; ++c) yacc[c] = 0;
@@ -394,20 +418,21 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             const uint32_t t0 = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + ch * NC, t2 = t0 + S::COL_S2 + (S::S2_SETS == 2 ? set * N : 0);
 #pragma unroll
             for (int c = 0; c < NC; c += LD) {
-                float s1[LD], s2[LD];
-                tmem_ld_x2(t0 + set * N + c, t2 + c, s1, s2);
-                if (c + LD == NC) {                    // both accumulators have been read
+                float s1[LD], s2[LD], s1b[LD];
+                if constexpr (S::S1_ACC == 2) tmem_ld3(t0 + 2 * set * N + c, t0 + (2 * set + 1) * N + c, t2 + c, s1, s1b, s2);
+                else tmem_ld8(t0 + set * N + c, t2 + c, s1, s2);
+                if (c + LD == NC) {                    // all accumulators have been read
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive1(acc_empty + set);
                 }
 #pragma unroll
-                for (int j = 0; j < LD; j += 4) {
-                    const float4 x4 = *reinterpret_cast<const float4*>(dx + c + j);
-                    uint64_t& ya = yacc[(c + j) / 2];
-                    uint64_t& yb = yacc[(c + j) / 2 + 1];
-                    ya = fma2(pk2(x4.x, x4.y), fma2(nd2, pk2(s2[j], s2[j + 1]), mul2(dw2, pk2(s1[j], s1[j + 1]))), ya);
-                    yb = fma2(pk2(x4.z, x4.w), fma2(nd2, pk2(s2[j + 2], s2[j + 3]), mul2(dw2, pk2(s1[j + 2], s1[j + 3]))), yb);
+                for (int j = 0; j < LD; j += 2) {
+                    const float2 x2 = *reinterpret_cast<const float2*>(dx + c + j);
+                    uint64_t sum = pk2(s1[j], s1[j + 1]);
+                    if (S::S1_ACC == 2) sum = add2(sum, pk2(s1b[j], s1b[j + 1]));
+                    uint64_t& y2 = yacc[(c + j) / 2];
+                    y2 = fma2(pk2(x2.x, x2.y), fma2(dw2, sum, mul2(nd2, pk2(s2[j], s2[j + 1]))), y2);
                 }
             }
         }

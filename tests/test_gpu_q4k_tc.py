@@ -62,3 +62,28 @@ def test_many_queued_calls(gpu, n, k, m):
                 rel_err_ok(got, want[j & 1], 1e-5)
             assert np.array_equal(got, first[j & 1])
     w.free()
+
+
+@pytest.mark.parametrize("m", [20, 64, 128])
+def test_largest_sums(gpu, m):
+    """One super-block of codes 14 and 15, scales 62 and 63 and activation codes 126 and 127 (the others meet zeros): its integer sum is
+    1.7 times 2^24 and all other factors are powers of two, so the result is that sum rounded once.
+
+    Bar: equal for the tiles of 32 and 64 rows, which hold its two halves exactly. Tiles of 128 rows sum it in one accumulator, whose
+    sixteen additions may each lose the last place of numbers below 2^25: 16 * 2."""
+    n, nb, rng = 300, 17, np.random.default_rng(m)
+    codes, sc = rng.integers(14, 16, (n, nb, 8, 32)), rng.integers(62, 64, (n, nb, 8))
+    raw = np.zeros((n, nb, 144), np.uint8)
+    raw[..., 0:2] = np.full((n, nb, 1), 2.0 ** -10, np.float16).view(np.uint8)
+    raw[..., 4:8], raw[..., 12:16] = sc[..., :4] | (sc[..., 4:] >> 4 << 6), sc[..., 4:] & 15
+    raw[..., 16:] = (codes[:, :, 0::2] | codes[:, :, 1::2] << 4).reshape(n, nb, 128)
+    q, at = rng.integers(126, 128, (m, 256)), rng.integers(0, nb, m)
+    q[:, 0] = 127                                      # the scale of a row's block is then exactly 2^-7
+    x = np.zeros((m, nb, 256), np.float32)
+    x[np.arange(m), at] = q * 2.0 ** -7
+    sums = np.einsum("mje,nmje->mn", q.reshape(m, 8, 32), (codes * sc[..., None])[:, at])
+    assert sums.min() > 1.5 * 2 ** 24
+    w = gpu.Weight.upload(raw.reshape(-1), "Q4_K", n, 256 * nb)
+    got = gpu.matmul_host(w, x.reshape(m, -1)).astype(np.float64) * 2.0 ** 17
+    assert np.abs(got - sums.astype(np.float32)).max() <= (32 if m == 128 else 0)
+    w.free()
