@@ -37,7 +37,7 @@
 
 #include <cuda_fp16.h>
 #include <algorithm>
-#include <mutex>
+#include <atomic>
 
 namespace sk {
 
@@ -221,6 +221,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     uint64_t* acc_full = s2_full + 4;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = (uint32_t*) (acc_empty + 2);
+    uint32_t* gave_up = tmem_slot + 1;                       // a wait of the fold ran out: this part's sums are not whole
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int MMA_WARP = S::PROD_WARPS + TC_EPI_WARPS;
@@ -235,6 +236,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             for (int i = 0; i < 2; ++i) { skd::mbar_init(a_full + i, 8); skd::mbar_init(a_empty + i, 1); skd::mbar_init(acc_full + i, 1); skd::mbar_init(acc_empty + i, TC_EPI_WARPS); }
             for (int i = 0; i < 4; ++i) skd::mbar_init(s2_full + i, 8);
             skd::mbar_fence_init();
+            *gave_up = 0;
         }
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(skd::smem_u32(tmem_slot)), "r"(512) : "memory");
@@ -438,6 +440,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
         }
         if (parts > 1) {
             // this part's sums into shared memory, [column][row], where the activation tiles were (all MMAs have read them)
+            if (!ok) *gave_up = 1;
             float* mine = (float*) (smem + S::OFF_B) + (ch * NC) * TC_M + r;
 #pragma unroll
             for (int c = 0; c < NC / 2; ++c) {
@@ -469,10 +472,12 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
         cluster_sync_all();                            // every part's sums are in place
         skd::pdl_wait();
         const uint32_t base = skd::smem_u32(smem + S::OFF_B);
+        bool whole = true;
+        for (int p = 0; p < parts; ++p) whole = whole && ld_cluster(skd::smem_u32(gave_up), p) == 0.0f;
         const int per = (N * TC_M / 4 + parts - 1) / parts * 4, e0 = part * per, e1 = min(N * TC_M, e0 + per);
         for (int e = e0 + tid; e < e1; e += S::THREADS) {
             const int row = row0 + (e & (TC_M - 1)), col = col0 + e / TC_M;
-            if (row >= rows || col >= m) continue;
+            if (!whole || row >= rows || col >= m) continue;
             float v = 0.0f;
             for (int p = 0; p < parts; ++p) v += ld_cluster(base + e * 4, p);
             const size_t o = (size_t) col * rows + row;
@@ -483,27 +488,27 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     }
 }
 
-// Clusters of `parts` CTAs the current device holds at once (they lie within a GPC, so 148 SMs hold 33 of four), found once per device.
+// Clusters of `parts` CTAs the current device holds at once (they lie within a GPC, so 148 SMs hold 33 of four), found once per device; two
+// threads that both find it missing find the same.
 template <int N>
 int tc_clusters(int parts) {
-    static std::mutex mu;
-    static int known[64][9] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return std::max(1, sm_count() / parts); }
-    std::lock_guard<std::mutex> lk(mu);
-    int& k = known[dev][parts];
-    if (k == 0) {
+    static std::atomic<int> known[64][9];
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+    if (dev < 0 || dev >= 64) return std::max(1, sm_count() / parts);
+    int n = known[dev][parts].load(std::memory_order_relaxed);
+    if (n == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned) parts); cfg.blockDim = dim3(TcShape<N>::THREADS); cfg.dynamicSmemBytes = TcShape<N>::SMEM;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned) parts; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, q4k_gemm_tc_kernel<N>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = std::max(1, sm_count() / parts); }
-        k = n;
+        if (ensure_dynamic_smem((const void*) q4k_gemm_tc_kernel<N>, TcShape<N>::SMEM) != SKAINET_CUDA_OK ||
+            cudaOccupancyMaxActiveClusters(&n, q4k_gemm_tc_kernel<N>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = std::max(1, sm_count() / parts); }
+        known[dev][parts].store(n, std::memory_order_relaxed);
     }
-    return k;
+    return n;
 }
 
 // Microseconds fitted to calls of 1 K x 1 K to 22 K x 4 K weights: what precedes the kernel, a super-block, a round of CTAs (prologue, first
@@ -535,16 +540,24 @@ float mma_cost(const Weight& w, int m) {
     return 3.5f + std::max(rate, chain);
 }
 
+// Parts of a tile for m rows where this kernel is expected to cost less than the mma.sync one; 0 where it is not.
 template <int N>
-int32_t launch_tc_n(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s) {
+int tc_plan_n(const Weight& w, int m) {
+    const float other = m < TC_ALWAYS_ROWS ? mma_cost(w, m) : 1e30f;
+    if (other <= TC_BEFORE + TC_ROUND + tc_unit<N>()) return 0;              // below any call of this kernel
+    float cost;
+    const int parts = tc_parts<N>((int64_t) ((w.rows + TC_M - 1) / TC_M) * ((m + N - 1) / N), w.bpr, &cost);
+    return cost > other ? 0 : parts;
+}
+
+// 1 = not taken: scratch that cannot be had (or would have to grow while the stream is being captured), or a weight no tensor map describes
+template <int N>
+int32_t launch_tc_n(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int parts, cudaStream_t s) {
     typedef TcShape<N> S;
     const int m_pad = (m + N - 1) / N * N, m_tiles = (w.rows + TC_M - 1) / TC_M, n_tiles = m_pad / N;
-    const float other = m < TC_ALWAYS_ROWS ? mma_cost(w, m) : 1e30f;
-    if (other <= TC_BEFORE + TC_ROUND + tc_unit<N>()) return 1;              // below any call of this kernel
+    CUtensorMap mq;
+    if (tensor_map_bytes(&mq, w.qs, w.rows, (int64_t) w.bpr * 128, TC_M) != SKAINET_CUDA_OK) return 1;
     SK_TRY(ensure_dynamic_smem((const void*) q4k_gemm_tc_kernel<N>, S::SMEM));
-    float cost;
-    const int parts = tc_parts<N>((int64_t) m_tiles * n_tiles, w.bpr, &cost);
-    if (cost > other) return 1;
     const size_t xh_bytes = (size_t) m_pad * w.cols * 2, hs_bytes = (size_t) m_pad * (w.cols / 16) * 2;
     const size_t need = gemm_tc_scratch_bytes(m, w.cols);
     // the operand tiles live in the calling stream's own scratch (calls on different streams do not share them)
@@ -553,13 +566,13 @@ int32_t launch_tc_n(const Weight& w, ActQ8K a, int m, float* y, const float* res
         if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) { cudaGetLastError(); return 1; }
     }
     void* base = nullptr;
-    SK_TRY(scratch_get(s, SCRATCH_GEMM, need, &base));
+    const int32_t st = scratch_get(s, SCRATCH_GEMM, need, &base);
+    if (st == SKAINET_CUDA_ERR_OOM) return 1;
+    if (st != SKAINET_CUDA_OK) return st;
     auto up = [](size_t v) { return (v + 255) & ~(size_t) 255; };
     __half* xh = (__half*) base;
     __half* hs = (__half*) ((uint8_t*) base + up(xh_bytes));
     float* dxt = (float*) ((uint8_t*) base + up(xh_bytes) + up(hs_bytes));
-    CUtensorMap mq;
-    SK_TRY(tensor_map_bytes(&mq, w.qs, w.rows, (int64_t) w.bpr * 128, TC_M));
     const int64_t n16 = (int64_t) m_pad * (w.cols / 16);
     SK_CUDA(launch_pdl(act_f16_tiles_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, s, a, m, m_pad, w.cols, N == 128 ? 7 : N == 64 ? 6 : 5, xh, hs, dxt));
     cudaLaunchConfig_t cfg = {};
@@ -583,12 +596,25 @@ size_t gemm_tc_scratch_bytes(int m, int cols) {
     return m_pad * cols * 2 + m_pad * (cols / 16) * 2 + m_pad * (cols / 256) * 4 + 3 * 256;
 }
 
-// y[m][w.rows] (= resid +) for m >= TC_MIN_ROWS quantized activation rows. Returns 1 when not taken (the caller
-// falls back to the mma.sync tile kernel): other encodings, few rows, shapes that kernel is quicker on, or scratch that would
-// have to grow while the stream is being captured.
+// The tile (32, 64 or 128 activation rows) and the parts that share one for m rows; 0 where the mma.sync tile kernel is the quicker.
+int gemm_tc_plan(const Weight& w, int m, int* parts) {
+    *parts = 0;
+    if (w.enc != SKAINET_ENC_Q4_K || m < TC_MIN_ROWS || w.bpr < 1) return 0;
+    const int tile = m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    *parts = tile == 32 ? tc_plan_n<32>(w, m) : tile == 64 ? tc_plan_n<64>(w, m) : tc_plan_n<128>(w, m);
+    return *parts ? tile : 0;
+}
+
+// y[m][w.rows] (= resid +) for quantized activation rows through tiles of 32, 64 or 128, `parts` CTAs a tile
+int32_t launch_gemm_tc_tiles(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int tile, int parts, cudaStream_t s) {
+    return tile == 32 ? launch_tc_n<32>(w, a, m, y, resid, parts, s) : tile == 64 ? launch_tc_n<64>(w, a, m, y, resid, parts, s) : launch_tc_n<128>(w, a, m, y, resid, parts, s);
+}
+
+// The same where it is the quicker. Returns 1 when not taken (the caller falls back to the mma.sync tile kernel).
 int32_t launch_gemm_tc(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s) {
-    if (w.enc != SKAINET_ENC_Q4_K || m < TC_MIN_ROWS || w.bpr < 1) return 1;
-    return m <= 32 ? launch_tc_n<32>(w, a, m, y, resid, s) : m <= 64 ? launch_tc_n<64>(w, a, m, y, resid, s) : launch_tc_n<128>(w, a, m, y, resid, s);
+    int parts;
+    const int tile = gemm_tc_plan(w, m, &parts);
+    return tile ? launch_gemm_tc_tiles(w, a, m, y, resid, tile, parts, s) : 1;
 }
 
 }  // namespace sk

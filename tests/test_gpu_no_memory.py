@@ -1,0 +1,64 @@
+"""What runs on when device memory is short: nearly all of it is taken by buffers that nothing touches, and given back at the end."""
+import gc
+
+import numpy as np
+import pytest
+
+from conftest import rel_err_ok
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def hog(gpu):
+    """hog(leave): takes device memory until about `leave` bytes are left (0: until a block of 2 MB is refused). release() ends it."""
+    import torch
+    held = []
+
+    def take(leave=0):
+        gc.collect()
+        size = torch.cuda.mem_get_info()[0] - leave
+        while size >= 2 << 20:
+            try:
+                held.append(gpu.DeviceBuffer(size))
+                if leave:
+                    return
+            except Exception:
+                size //= 2
+
+    def release():
+        for b in held:
+            b.free()
+        held.clear()
+
+    take.release = release
+    yield take
+    release()
+
+
+def test_rows_without_operand_scratch(gpu, hog):
+    """Rows for the tcgen05 kernel whose scratch cannot be had go to the kernel that needs none. (The quantized rows find theirs: a call over a
+    Q6_K weight of as many inputs left it.)"""
+    rng = np.random.default_rng(1)
+    m, n, k = 64, 1024, 22016
+    import ctypes as C
+    from skainet_b200 import _lib as L
+    stream = C.c_void_p()
+    L.check(L.lib().skainet_cuda_stream_create(C.byref(stream)))
+    w, other = gpu.Weight.synth("Q4_K", n, k, seed=5, std=0.02), gpu.Weight.upload(np.zeros(64 * (k // 256) * 210, np.uint8), "Q6_K", 64, k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    want = np.concatenate([gpu.matmul_host(w, x[i:i + 8]) for i in range(0, m, 8)])
+    dx, dy, dz = gpu.DeviceBuffer.from_host(x), gpu.DeviceBuffer(4 * m * n), gpu.DeviceBuffer(4 * m * 64)
+    gpu.matmul(other, dx.ptr, m, dz.ptr, stream=stream.value)
+    gpu.sync(stream.value)
+    hog()
+    gpu.matmul(w, dx.ptr, m, dy.ptr, stream=stream.value)
+    gpu.sync(stream.value)
+    hog.release()
+    rel_err_ok(dy.download(np.float32, m * n).reshape(m, n), want, 1e-5)
+    gpu.matmul(w, dx.ptr, m, dy.ptr, stream=stream.value)              # with memory, the tcgen05 kernel again
+    gpu.sync(stream.value)
+    rel_err_ok(dy.download(np.float32, m * n).reshape(m, n), want, 1e-5)
+    L.check(L.lib().skainet_cuda_stream_destroy(stream))
+    w.free()
+    other.free()
