@@ -519,6 +519,33 @@ int32_t skainet_cuda_probe_read_dev(skainet_weight_t h, skainet_stream_t stream)
     return launch_probe_read(*w, (uint32_t*) sink, as_stream(stream));
 }
 
+int32_t skainet_cuda_selftest_q4k_rows_plan(skainet_weight_t h, int32_t m, int32_t* out2) {
+    Weight* w = weight_from_handle(h);
+    if (!w) return SKAINET_CUDA_ERR_HANDLE;
+    SK_REQUIRE(out2 != nullptr && m >= 0, "q4k_rows_plan: null output or negative row count");
+    SK_TRY(ensure_device());
+    int parts = 0;
+    out2[0] = gemm_tc_plan(*w, m, &parts);
+    out2[1] = parts;
+    return SKAINET_CUDA_OK;
+}
+
+int32_t skainet_cuda_selftest_q4k_rows_dev(skainet_weight_t h, const float* x_dev, int32_t m, float* y_dev, int32_t tile, int32_t parts, skainet_stream_t stream) {
+    Weight* w = weight_from_handle(h);
+    if (!w) return SKAINET_CUDA_ERR_HANDLE;
+    SK_REQUIRE(w->enc == SKAINET_ENC_Q4_K, "q4k_rows: encoding %d", w->enc);
+    SK_REQUIRE((tile == 32 || tile == 64 || tile == 128) && parts >= 1 && parts <= 8 && parts <= w->bpr, "q4k_rows: tiles of %d rows in %d parts", tile, parts);
+    SK_REQUIRE(m >= 1 && x_dev && y_dev && ((uintptr_t) x_dev & 15) == 0, "q4k_rows: no rows, a null pointer, or x not 16-byte aligned");
+    SK_TRY(ensure_device());
+    cudaStream_t s = as_stream(stream);
+    void* scratch = nullptr;
+    SK_TRY(scratch_get(s, SCRATCH_ACT, act_scratch_bytes(w->enc, SKAINET_ACT_NATIVE, m, w->cols), &scratch));
+    SK_TRY(launch_act_quant(w->enc, SKAINET_ACT_NATIVE, x_dev, m, w->cols, scratch, s));
+    const int32_t st = launch_gemm_tc_tiles(*w, act_q8k_layout(scratch, m, w->cols), m, y_dev, nullptr, tile, parts, s);
+    SK_REQUIRE(st != 1, "q4k_rows: no scratch or no tensor map for %d rows", m);
+    return st;
+}
+
 int32_t skainet_cuda_matvec_fused_dev(skainet_weight_t h, const float* x_dev, const float* gamma_dev, float eps,
                                       const float* resid_dev, float* y_dev, skainet_stream_t stream) {
     Weight* w = weight_from_handle(h);

@@ -47,6 +47,8 @@ constexpr int TC_MIN_ROWS = 9, TC_ALWAYS_ROWS = 288;
 int32_t launch_rows_ring(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 // gemm_tc.cu: the same for m >= TC_MIN_ROWS on tcgen05 with TMEM accumulators; 1 = not taken
 size_t gemm_tc_scratch_bytes(int m, int cols);
+int gemm_tc_plan(const Weight& w, int m, int* parts);
+int32_t launch_gemm_tc_tiles(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int tile, int parts, cudaStream_t s);
 int32_t launch_gemm_tc(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 
 }  // namespace sk

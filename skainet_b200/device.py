@@ -125,6 +125,18 @@ def matmul(w: Weight, x_ptr: int, m: int, y_ptr: int, act_mode: int = L.ACT_NATI
     L.check(L.lib().skainet_cuda_matmul_dev(w.handle, x_ptr, m, y_ptr, act_mode, stream))
 
 
+def q4k_rows_plan(w: Weight, m: int) -> tuple[int, int]:
+    """(activation rows of a tcgen05 tile, CTAs that share one) that matmul takes for m rows; (0, 0) where another kernel does."""
+    out = (C.c_int32 * 2)()
+    L.check(L.lib().skainet_cuda_selftest_q4k_rows_plan(w.handle, m, out))
+    return out[0], out[1]
+
+
+def q4k_rows(w: Weight, x_ptr: int, m: int, y_ptr: int, tile: int, parts: int, stream: int = 0) -> None:
+    """matmul through the tcgen05 kernel with the given tile and parts."""
+    L.check(L.lib().skainet_cuda_selftest_q4k_rows_dev(w.handle, x_ptr, m, y_ptr, tile, parts, stream))
+
+
 def matvec_fused(w: Weight, x_ptr: int, gamma_ptr: int, eps: float, resid_ptr: int, y_ptr: int, stream: int = 0) -> None:
     """y = (resid +) W . quantize(rmsnorm(x) if gamma else x), one launch."""
     L.check(L.lib().skainet_cuda_matvec_fused_dev(w.handle, x_ptr, gamma_ptr or None, eps, resid_ptr or None, y_ptr, stream))

@@ -1,0 +1,75 @@
+"""One captured decode step of many sequences: its attention (rotation, append and, with more (sequence, cache head) pairs than SMs, four warps
+a CTA: csrc/attention.cu) against attention in 64 bits over each sequence's own history, and its linears where nine and more
+sequences send them to the tcgen05 kernel."""
+import numpy as np
+import pytest
+
+from test_gpu_llama import build, step_err
+
+pytestmark = pytest.mark.gpu
+
+
+def read(m, which, rows, width):
+    return m.peek(which, rows * width).reshape(rows, width).copy()
+
+
+def prompts(m, cfg, lengths, rng):
+    """Prompts of the given lengths into the sequences; their q | k | v rows."""
+    width, rows = (cfg.n_heads + 2 * cfg.n_kv_heads) * cfg.head_dim, []
+    for seq, n in enumerate(lengths):
+        m.forward(rng.integers(0, cfg.vocab, size=n).astype(np.int32), [n - 1], seq)
+        rows.append(read(m, 1, n, width))
+    return rows
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,batch,mode", [(64, 8, 64, 20, 0), (8, 8, 128, 20, 1), (32, 8, 64, 40, 0), (16, 8, 128, 19, 1), (8, 4, 128, 6, 0)])
+def test_attention_of_a_step(gpu, oracle, heads, kv_heads, dim, batch, mode):
+    """Bar: the keys and values that the cache holds are the binary16 of both sides' rotated rows, which may fall to a neighbouring value
+    (2^-11 of it): 2e-3 of the largest result, as for prompts; a lost or foreign key is worth 1e-2 and more."""
+    from skainet_b200.llama import LlamaConfig
+    cfg = LlamaConfig(1, 256, heads, kv_heads, dim, 256, 300, max_seq=330, max_batch=batch, rope_mode=mode)
+    m, _, _ = build(gpu, cfg, seed=heads + batch)
+    rng = np.random.default_rng(batch)
+    lengths = rng.integers(1, 90, batch)
+    lengths[:4] = 1, 320, 64, 17
+    history = prompts(m, cfg, lengths, rng)
+    m.decode(rng.integers(0, cfg.vocab, size=batch).astype(np.int32), np.zeros(batch, np.int32))
+    new, got = read(m, 1, batch, history[0].shape[1]), read(m, 2, batch, heads * dim).reshape(batch, heads, dim).astype(np.float64)
+    for b in range(batch):
+        qkv = np.concatenate([history[b], new[b:b + 1]]).reshape(lengths[b] + 1, -1, dim)
+        turned = np.stack([oracle.rope(row[:heads + kv_heads].copy(), heads + kv_heads, dim, p, mode=mode).reshape(-1, dim) for p, row in enumerate(qkv)])
+        half = lambda a: np.repeat(a.astype(np.float16).astype(np.float64), heads // kv_heads, 1)  # noqa: E731
+        q, k, v = turned[-1, :heads].astype(np.float64), half(turned[:, heads:]), half(qkv[:, heads + kv_heads:])
+        score = np.einsum("hd,jhd->hj", q, k) / np.sqrt(dim)
+        p = np.exp(score - score.max(-1, keepdims=True))
+        want = np.einsum("hj,jhd->hd", p / p.sum(-1, keepdims=True), v)
+        assert np.abs(got[b] - want).max() <= 2e-3 * np.abs(want).max(), b
+    m.free()
+
+
+def test_linears_of_a_step(gpu, oracle):
+    """Twenty sequences: the down projection of the step takes clusters of the tcgen05 kernel (asserted), from scratch that the model laid
+    out before the step was captured. Bar of the decoder tests (0.15 of the logits' root mean square, an activation code that falls
+    the other way); and the step repeats itself bit for bit."""
+    from skainet_b200.llama import LlamaConfig
+    from oracle.llama_cpu import CpuLlama
+    cfg = LlamaConfig(1, 512, 8, 8, 64, 11008, 300, max_seq=64, max_batch=20)
+    w = gpu.Weight.synth("Q4_K", 512, 11008, seed=1, std=0.02)
+    assert gpu.q4k_rows_plan(w, 20)[0] == 32
+    w.free()
+    m, weights, gam = build(gpu, cfg, norms=True)
+    rng = np.random.default_rng(4)
+    first, then = (rng.integers(0, cfg.vocab, size=20).astype(np.int32) for _ in range(2))
+    runs = []
+    for _ in range(3):
+        m.reset()
+        for seq in range(20):
+            m.forward(first[seq:seq + 1], [0], seq)
+        m.decode(then, np.zeros(20, np.int32))
+        runs.append(m.logits(20).copy())
+    assert np.array_equal(runs[0], runs[1]) and np.array_equal(runs[0], runs[2])
+    for seq in range(20):
+        cpu = CpuLlama(cfg, weights, gam)
+        cpu.step(int(first[seq]))
+        assert step_err(runs[0][seq], cpu.step(int(then[seq]))) < 0.15
+    m.free()

@@ -87,3 +87,39 @@ def test_largest_sums(gpu, m):
     got = gpu.matmul_host(w, x.reshape(m, -1)).astype(np.float64) * 2.0 ** 17
     assert np.abs(got - sums.astype(np.float32)).max() <= (32 if m == 128 else 0)
     w.free()
+
+
+@pytest.mark.parametrize("tile,parts", [(32, 1), (32, 3), (32, 8), (64, 1), (64, 2), (64, 5), (128, 1), (128, 4), (128, 7)])
+@pytest.mark.parametrize("n,k", [(1, 256), (127, 768), (128, 1280), (300, 2304), (129, 4352)])
+def test_tiles_and_parts(gpu, oracle, tile, parts, n, k):
+    """Every tile and cluster at its edges, whatever the plan would take: the same rows, one short of a tile to one more, through the
+    kernel itself; queued behind one another with other rows, each result that of the call made alone."""
+    parts = min(parts, k // 256)
+    rng = np.random.default_rng(n + k + tile + parts)
+    w_bytes = oracle.quantize_q4k((0.02 * rng.standard_normal((n, k))).astype(np.float32))
+    w = gpu.Weight.upload(w_bytes, "Q4_K", n, k)
+    calls = []
+    for m in (1, tile - 1, tile, tile + 1):
+        x = ((10.0 ** (m % 3)) * rng.standard_normal((m, k))).astype(np.float32)
+        x[0, :256] = 0.0
+        dx, dy = gpu.DeviceBuffer.from_host(x), gpu.DeviceBuffer(4 * m * n)
+        gpu.q4k_rows(w, dx.ptr, m, dy.ptr, tile, parts)
+        got = dy.download(np.float32, m * n).reshape(m, n)
+        rel_err_ok(got, oracle.matmul("Q4_K", x, w_bytes, k, n, "rm", use_ref=oracle.ref() is not None), 1e-5)
+        calls.append((m, dx, dy, got))
+    for _ in range(4):
+        for m, dx, dy, _ in calls:
+            gpu.q4k_rows(w, dx.ptr, m, dy.ptr, tile, parts)
+    for m, _, dy, got in calls:
+        assert np.array_equal(dy.download(np.float32, m * n).reshape(m, n), got)
+    w.free()
+
+
+@pytest.mark.parametrize("n,k,m,tile,cluster", [(11008, 4096, 64, 64, False), (11008, 4096, 32, 32, False), (4096, 11008, 64, 64, True), (4096, 11008, 20, 32, True), (512, 11008, 20, 32, True),
+                                                (11008, 4096, 128, 128, False), (11008, 1024, 512, 128, False), (300, 4352, 64, 64, True), (1, 256, 64, 0, False), (127, 768, 64, 0, False)])
+def test_which_calls_take_the_kernel(gpu, n, k, m, tile, cluster):
+    """The shapes that the tests here rely on reach the tiles (and clusters) they are meant for, or another kernel."""
+    w = gpu.Weight.synth("Q4_K", n, k, seed=5, std=0.02)
+    got, parts = gpu.q4k_rows_plan(w, m)
+    assert got == tile and (parts > 1) == cluster
+    w.free()
