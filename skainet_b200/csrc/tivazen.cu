@@ -96,22 +96,32 @@ struct Tivazen : Decoder {
         return expand_weights();
     }
     // W_uk back in its own orientation, with W_uv below it, for the layers whose prompts take the expanded form of attention; the room
-    // for the widest of their caches is shared, since a layer uses it within its own attention only.
+    // for the widest of their caches is shared, since a layer uses it within its own attention only. A layer whose copy finds no memory,
+    // or would take all copies past LATENT_EXPAND_COPY_BYTES, keeps the folded form.
     int32_t expand_weights() {
-        size_t room = 0;
+        auto none = [&]() { for (auto& L : layers) if (L.ukv) { weight_release(L.ukv); L.ukv = nullptr; } };
+        auto room_of = [&](const TvLayer& L) -> size_t {
+            const size_t bytes = (size_t) L.cache.cap * L.geom.heads * 2 * L.geom.dim * 2;
+            return f32 || !latent_expands(L.geom) || max_rows < LATENT_EXPAND_ROWS || bytes > LATENT_EXPAND_MAX_BYTES ? 0 : bytes;
+        };
+        none();                                                          // laid out by an earlier call that failed behind it, from weights set since
+        size_t room = 0, copies = 0;
+        for (auto& L : layers) room = std::max(room, room_of(L));
+        if (room == 0) return SKAINET_CUDA_OK;
+        int32_t st = kv ? SKAINET_CUDA_OK : alloc(&kv, room);
         for (auto& L : layers) {
+            if (st != SKAINET_CUDA_OK) break;
             const LatentGeom& g = L.geom;
-            const size_t bytes = (size_t) L.cache.cap * g.heads * 2 * g.dim * 2;
-            if (f32 || L.ukv || !latent_expands(g) || max_rows < LATENT_EXPAND_ROWS || bytes > LATENT_EXPAND_MAX_BYTES) continue;
-            SK_TRY(weight_alloc(SKAINET_ENC_BF16, g.heads * 2 * g.dim, g.kv_rank, &L.ukv));
+            copies += (size_t) g.heads * 2 * g.dim * g.rank_ld() * 2;
+            if (room_of(L) == 0 || copies > LATENT_EXPAND_COPY_BYTES) continue;
+            if ((st = weight_alloc(SKAINET_ENC_BF16, g.heads * 2 * g.dim, g.kv_rank, &L.ukv)) != SKAINET_CUDA_OK) { L.ukv = nullptr; break; }
             bf16* dst = (bf16*) L.ukv->qs;
             SK_TRY(launch_transpose_heads(data(L.uk), dst, g.heads, g.kv_rank, g.dim, nullptr));
             SK_CUDA(cudaMemcpy(dst + (size_t) g.heads * g.dim * g.rank_ld(), L.uv->qs, (size_t) g.heads * g.vdim * g.rank_ld() * 2, cudaMemcpyDeviceToDevice));
-            room = std::max(room, bytes);
         }
-        if (room && !kv) SK_TRY(alloc(&kv, room));
+        if (!kv) none();
         SK_CUDA(cudaStreamSynchronize(nullptr));
-        return SKAINET_CUDA_OK;
+        return st == SKAINET_CUDA_ERR_OOM ? SKAINET_CUDA_OK : st;
     }
     int32_t enqueue_decode(int batch, int kv_bound, cudaStream_t s) override {
         SK_TRY(body(batch, RowMap{pos, -1}, kv_bound, s));

@@ -1,10 +1,16 @@
 """What runs on when device memory is short: nearly all of it is taken by buffers that nothing touches, and given back at the end."""
+import ctypes as C
 import gc
+import os
 
 import numpy as np
 import pytest
 
+import tivazen_models as M
 from conftest import rel_err_ok
+from oracle import tivazen as F
+from skainet_b200 import _lib as L
+from test_gpu_tivazen import TOL
 
 pytestmark = pytest.mark.gpu
 
@@ -41,8 +47,6 @@ def test_rows_without_operand_scratch(gpu, hog):
     Q6_K weight of as many inputs left it.)"""
     rng = np.random.default_rng(1)
     m, n, k = 64, 1024, 22016
-    import ctypes as C
-    from skainet_b200 import _lib as L
     stream = C.c_void_p()
     L.check(L.lib().skainet_cuda_stream_create(C.byref(stream)))
     w, other = gpu.Weight.synth("Q4_K", n, k, seed=5, std=0.02), gpu.Weight.upload(np.zeros(64 * (k // 256) * 210, np.uint8), "Q6_K", 64, k)
@@ -62,3 +66,31 @@ def test_rows_without_operand_scratch(gpu, hog):
     L.check(L.lib().skainet_cuda_stream_destroy(stream))
     w.free()
     other.free()
+
+
+def loaded(path, cfg, **runtime):
+    """A Tivazen model with its weights, not finalized."""
+    from skainet_b200 import tivazen as T
+    from skainet_b200.safetensors import SafetensorsReader
+    m = T.Tivazen(T.TivazenConfig.from_json(cfg, **runtime))
+    r = SafetensorsReader(os.path.join(path, "model.safetensors"))
+    m.load(r)
+    r.close()
+    return m
+
+
+def test_prompts_without_room_for_expanded_weights(gpu, hog, tmp_path):
+    """Where finalize finds no memory for the weights of the expanded form of latent attention, prompts take the folded form."""
+    cfg = M.config([(M.attn(heads=16, dim=128, rot_dim=64, vdim=128, kv_rank=512, scale=0.08, window=100), None)], width=64)
+    w = M.random_weights(cfg, 7)
+    path, t, out = M.save(tmp_path, cfg, w), M.tokens(cfg, 400), []
+    for short in (True, False):
+        m = loaded(path, cfg, max_seq=600, prefill_rows=300)
+        if short:
+            hog()
+        m.finalize()
+        hog.release()
+        out.append(m.forward(t, list(range(400))))
+        assert M.error(out[-1], F.forward(cfg, w, t)) < TOL["bfloat16"]
+        m.free()
+    assert not np.array_equal(*out)
