@@ -687,10 +687,17 @@ int32_t launch_latent_attention(const LatentArgs& args, cudaStream_t s) {
         else SK_CUDA(launch_pdl(latent_prep_kernel<bf16>, dim3(a.rows), dim3(256), 0, s, a));
         LinearArgs l;
         if (a.kv && a.map.seq >= 0 && a.rows >= LATENT_EXPAND_ROWS) {
-            // keys and values of the cache slots in use, then attention over them; out is final
-            l.w = a.ukv; l.w_rows = g.heads * 2 * g.dim; l.ldw = g.rank_ld(); l.x = (const bf16*) a.cache.rows + (size_t) a.map.seq * a.cache.cap * g.key_ld(); l.ldx = g.key_ld();
-            l.x_rows_alloc = a.cache.cap; l.rows = std::min(a.cache.cap, a.kv_bound); l.y = a.kv; l.ldy = l.w_rows; l.out = LIN_OUT_ACT;
-            SK_TRY(launch_linear_bf16(l, s));
+            // keys and values of the positions that a row of the pass sees, in the one or two runs of slots they lie in, then attention over
+            // them; out is final
+            const int cap = a.cache.cap, last = a.kv_bound, first = (int) std::max<int64_t>(0, (int64_t) last - a.rows - a.window + 1);
+            const int n = std::min(cap, last - first), slot = n == cap ? 0 : first % cap;
+            l.w = a.ukv; l.w_rows = g.heads * 2 * g.dim; l.ldw = g.rank_ld(); l.ldx = g.key_ld(); l.ldy = l.w_rows; l.out = LIN_OUT_ACT;
+            for (int at = slot, left = n; left > 0; at = 0) {
+                l.rows = std::min(left, cap - at); l.x_rows_alloc = cap - at;
+                l.x = (const bf16*) a.cache.rows + ((size_t) a.map.seq * cap + at) * g.key_ld(); l.y = (bf16*) a.kv + (size_t) at * l.ldy;
+                SK_TRY(launch_linear_bf16(l, s));
+                left -= l.rows;
+            }
             SK_TRY(ensure_dynamic_smem((const void*) latent_attn_expanded_kernel, EX_SMEM));
             SK_CUDA(launch_pdl(latent_attn_expanded_kernel, dim3(g.heads, (a.rows + EX_ROWS - 1) / EX_ROWS), dim3(256), EX_SMEM, s, a));
             return SKAINET_CUDA_OK;
