@@ -54,9 +54,32 @@ struct Decoder {
     virtual const float* buffer(int which) const = 0;
 };
 
+// Rows of one prompt pass of the BF16 designs unless the configuration says otherwise, and where memory is short: buffers and ring caches grow
+// with them. 2048 tokens in one pass instead of two take 9.8 ms instead of 12.8 (2B Tivazen shape) and 11.4 instead of 14.5 (2B Fomalix
+// shape): the 128-row tiles of the linears fill 4.8 rounds of SMs instead of 2.4, and half as many kernels are started. The Tivazen shape
+// takes 0.3 GB more for it, and 28 MB more of caches per sequence.
+constexpr int PROMPT_PASS_ROWS = 2048, PROMPT_PASS_ROWS_SHORT = 1024;
+constexpr size_t PROMPT_PASS_SPARE = (size_t) 2 << 30;        // left behind a model with the larger passes: weights on their way in, scratch
+
 int32_t decoder_init(Decoder* m);                     // allocates what the base owns and registers the handle
-skainet_model_t decoder_handle(Decoder* m);
 void decoder_destroy(Decoder* m);                     // unregisters and deletes
+// A model by make(rows of a pass), registered and laid out by lay_out(model): of asked rows, or of the library's choice for 0.
+template <typename M, typename Make, typename LayOut>
+int32_t decoder_create(int asked, Make&& make, LayOut&& lay_out, M** out) {
+    for (int rows : {asked ? asked : PROMPT_PASS_ROWS, PROMPT_PASS_ROWS_SHORT}) {
+        M* m = make(rows);
+        int32_t st = decoder_init(m);
+        if (st == SKAINET_CUDA_OK) st = lay_out(m);
+        size_t free = 0, total = 0;
+        const bool tight = st == SKAINET_CUDA_ERR_OOM || (st == SKAINET_CUDA_OK && cudaMemGetInfo(&free, &total) == cudaSuccess && free < PROMPT_PASS_SPARE);
+        const bool again = !asked && tight && m->max_rows > PROMPT_PASS_ROWS_SHORT && m->max_rows > m->max_batch;
+        if (st == SKAINET_CUDA_OK && !again) { *out = m; return st; }
+        decoder_destroy(m);
+        if (!again) return st;
+    }
+    return SKAINET_CUDA_ERR_OOM;
+}
+skainet_model_t decoder_handle(Decoder* m);
 Decoder* decoder_from_handle(skainet_model_t h);      // nullptr (+ error set) when unknown
 int32_t decoder_require_ready(Decoder* m, const char* who);
 int32_t flag_fetch(Decoder& m, cudaStream_t s);

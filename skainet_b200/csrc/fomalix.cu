@@ -26,10 +26,6 @@ namespace sk {
 
 namespace {
 
-// Rows of one prompt pass unless the configuration says otherwise. 2048 tokens in one pass instead of two take 11.44 ms instead of
-// 14.5 (2B shape): the 128-row tiles of the linears fill 4.8 rounds of SMs instead of 2.4, and half as many kernels are started.
-constexpr int PREFILL_ROWS = 2048;
-
 // Where a matrix or vector of the checkpoint goes.
 struct MatrixSlot { Weight* w = nullptr; int row0 = 0, rows = 0, cols = 0; };
 struct VectorSlot { float* p = nullptr; int n = 0; };
@@ -344,15 +340,16 @@ int32_t skainet_cuda_fomalix_create(const skainet_fomalix_config* cfg, const ska
         SK_REQUIRE(l.type != SKAINET_FX_MAMBA2 || (l.norm_groups >= 1 && (l.heads * l.vdim) % l.norm_groups == 0), "fomalix_create: layer %d: norm in %d parts", i, l.norm_groups);
     }
     SK_TRY(ensure_device());
-    Fomalix* m = new Fomalix();
-    m->cfg = c;
-    m->f32 = c.act_f32 != 0; m->act_size = m->f32 ? 4 : 2;
-    m->vocab = m->vocab_l = c.vocab; m->d_model = c.width; m->width_ld = bf16_ld(c.width); m->max_seq = c.max_seq; m->max_batch = c.max_batch;
-    m->max_rows = std::max(c.max_batch, std::min(c.prefill_rows ? c.prefill_rows : PREFILL_ROWS, c.max_seq));
-    m->layers.resize(c.n_layers);
-    int32_t st = decoder_init(m);
-    if (st == SKAINET_CUDA_OK) st = m->create(ls);
-    if (st != SKAINET_CUDA_OK) { decoder_destroy(m); return st; }
+    Fomalix* m = nullptr;
+    SK_TRY(decoder_create<Fomalix>(c.prefill_rows, [&](int rows) {
+        Fomalix* n = new Fomalix();
+        n->cfg = c;
+        n->f32 = c.act_f32 != 0; n->act_size = n->f32 ? 4 : 2;
+        n->vocab = n->vocab_l = c.vocab; n->d_model = c.width; n->width_ld = bf16_ld(c.width); n->max_seq = c.max_seq; n->max_batch = c.max_batch;
+        n->max_rows = std::max(c.max_batch, std::min(rows, c.max_seq));
+        n->layers.resize(c.n_layers);
+        return n;
+    }, [&](Fomalix* n) { return n->create(ls); }, &m));
     *out = decoder_handle(m);
     return SKAINET_CUDA_OK;
 }

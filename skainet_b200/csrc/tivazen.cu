@@ -24,10 +24,6 @@ namespace sk {
 
 namespace {
 
-// Rows of one prompt pass unless the configuration says otherwise. 2048 tokens in one pass instead of two take 9.77 ms instead of
-// 12.76 (2B shape): the 128-row tiles of the linears fill 4.8 rounds of SMs instead of 2.4, and half as many kernels are started.
-constexpr int PREFILL_ROWS = 2048;
-
 // Seeded noise in a sequence's cache rows; the zero tails stay zero.
 template <typename T>
 __global__ void fill_latent_kernel(T* rows, int cap, int key_ld, int rank, int rank_pad, int rot, uint64_t seed) {
@@ -364,15 +360,16 @@ int32_t skainet_cuda_tivazen_create(const skainet_tivazen_config* cfg, const ska
         }
     }
     SK_TRY(ensure_device());
-    Tivazen* m = new Tivazen();
-    m->cfg = c;
-    m->f32 = c.act_f32 != 0; m->act_size = m->f32 ? 4 : 2;
-    m->vocab = m->vocab_l = c.vocab; m->d_model = c.width; m->width_ld = bf16_ld(c.width); m->max_seq = c.max_seq; m->max_batch = c.max_batch;
-    m->max_rows = std::max(c.max_batch, std::min(c.prefill_rows ? c.prefill_rows : PREFILL_ROWS, c.max_seq));
-    m->layers.resize(c.n_layers);
-    int32_t st = decoder_init(m);
-    if (st == SKAINET_CUDA_OK) st = m->create(ls);
-    if (st != SKAINET_CUDA_OK) { decoder_destroy(m); return st; }
+    Tivazen* m = nullptr;
+    SK_TRY(decoder_create<Tivazen>(c.prefill_rows, [&](int rows) {
+        Tivazen* n = new Tivazen();
+        n->cfg = c;
+        n->f32 = c.act_f32 != 0; n->act_size = n->f32 ? 4 : 2;
+        n->vocab = n->vocab_l = c.vocab; n->d_model = c.width; n->width_ld = bf16_ld(c.width); n->max_seq = c.max_seq; n->max_batch = c.max_batch;
+        n->max_rows = std::max(c.max_batch, std::min(rows, c.max_seq));
+        n->layers.resize(c.n_layers);
+        return n;
+    }, [&](Tivazen* n) { return n->create(ls); }, &m));
     *out = decoder_handle(m);
     return SKAINET_CUDA_OK;
 }

@@ -94,3 +94,20 @@ def test_prompts_without_room_for_expanded_weights(gpu, hog, tmp_path):
         assert M.error(out[-1], F.forward(cfg, w, t)) < TOL["bfloat16"]
         m.free()
     assert not np.array_equal(*out)
+
+
+def test_shorter_passes_where_memory_is_short(gpu, hog, tmp_path):
+    """The library's choice of a pass is 2048 rows, and 1024 where those would leave too little memory: the model then is the one that asks for
+    passes of 1024 rows (same logits, bit for bit, of a prompt that the two choices cut differently), and it is created at all."""
+    cfg = M.config([(M.attn(heads=16, dim=128, rot_dim=64, vdim=128, kv_rank=512, scale=0.08, window=64), None) for _ in range(3)], width=64)
+    path, t, out = M.save(tmp_path, cfg, M.random_weights(cfg, 7)), M.tokens(cfg, 1500), {}
+    for rows, left in ((1024, 0), (2048, 0), (0, 0), (0, 1 << 30)):
+        if left:
+            hog(left)
+        m = loaded(path, cfg, max_seq=1600, max_batch=8, prefill_rows=rows)
+        hog.release()
+        m.finalize()
+        out[rows, left] = m.forward(t, [700, 1100, 1499])
+        m.free()
+    assert not np.array_equal(out[1024, 0], out[2048, 0])
+    assert np.array_equal(out[0, 0], out[2048, 0]) and np.array_equal(out[0, 1 << 30], out[1024, 0])
