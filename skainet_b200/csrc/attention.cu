@@ -829,11 +829,11 @@ attn_prefill_mma_kernel(const float* q, const __half* kc, const __half* vc, floa
 }
 
 // =================================================================================================
-// The same for many rows of a prompt: CTA = 64 consecutive queries of one head, a warp 16 of them, over tiles of 64 keys that the four
+// The same for many rows of one sequence's prompt, without a window: CTA = 64 consecutive queries of one head, a warp 16 of them, over tiles of 64 keys that the four
 // warps share through shared memory. q and the probabilities are carried as two f16 terms, one MMA each against the f16 cache rows.
 // With eight queries a CTA, each fetching all keys into registers by itself, the L2 reads bounded it: 512 rows x 32 heads
 // 82 us (a 512-token prompt of the 7B shape 21.5 ms, 20.1 with this kernel). Few queries over many keys leave SMs idle: then a cluster of `parts` CTAs shares the keys of a tile of queries, and their
-// records meet in shared memory, folded in the order of the parts. grid (heads * parts, ceil(seq_q / 64), batch), the queries with
+// records meet in shared memory, folded in the order of the parts. grid (heads * parts, ceil(seq_q / 64)), the queries with
 // the most keys first.
 // =================================================================================================
 constexpr int AP_ROWS = 64, AP_BK = 64, AP_THREADS = 128;
@@ -842,27 +842,27 @@ template <int D> constexpr int ap_smem() { return 2 * 2 * AP_BK * (D + 8) * 2; }
 template <int D>
 __global__ void __launch_bounds__(AP_THREADS, 2)
 attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __restrict__ out,
-                   int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* q_abs_base, float scale, int window, int parts) {
+                   int heads, int kv_heads, int seq_q, int64_t cache_stride, const int32_t* q_base, float scale, int parts) {
     constexpr int KS = D / 16, NT = D / 8, LD = D + 8, STAGE = 2 * AP_BK * LD, OLD = D + 4;
     static_assert(AP_ROWS * (OLD + 2) * 4 <= 2 * STAGE * 2, "the records take the place of the ring");
     extern __shared__ __align__(16) uint8_t smem[];
     __half* ring = (__half*) smem;
     skd::pdl_launch_dependents();
     skd::pdl_wait();
-    const int h = blockIdx.x / parts, part = blockIdx.x % parts, q0 = (gridDim.y - 1 - blockIdx.y) * AP_ROWS, b = blockIdx.z, kvh = h / (heads / kv_heads);
+    const int h = blockIdx.x / parts, part = blockIdx.x % parts, q0 = (gridDim.y - 1 - blockIdx.y) * AP_ROWS, kvh = h / (heads / kv_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int base = skd::ld_dep(q_abs_base + b), q_last = min(q0 + AP_ROWS, seq_q) - 1;
-    const int hi = base + q_last, lo = window > 0 ? max(0, base + q0 - window + 1) : 0, n_all = (hi - lo) / AP_BK + 1;
+    const int base = skd::ld_dep(q_base), q_last = min(q0 + AP_ROWS, seq_q) - 1;
+    const int hi = base + q_last, n_all = hi / AP_BK + 1;
     const int t_first = (int) ((int64_t) n_all * part / parts), t_end = (int) ((int64_t) n_all * (part + 1) / parts);      // this part's tiles
-    const __half* kb = kc + ((int64_t) b * kv_heads + kvh) * cache_stride * D;
-    const __half* vb = vc + ((int64_t) b * kv_heads + kvh) * cache_stride * D;
+    const __half* kb = kc + (int64_t) kvh * cache_stride * D;
+    const __half* vb = vc + (int64_t) kvh * cache_stride * D;
 
     auto fetch = [&](int i) {                             // keys past hi repeat the newest one; their scores are masked
         if (i < t_end) {
             __half* kd = ring + (i & 1) * STAGE;
             for (int c = threadIdx.x; c < AP_BK * (D / 8); c += AP_THREADS) {
                 const int j = c / (D / 8), x = c % (D / 8) * 8;
-                const int64_t src = (int64_t) min(lo + i * AP_BK + j, hi) * D + x;
+                const int64_t src = (int64_t) min(i * AP_BK + j, hi) * D + x;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(skd::smem_u32(kd + j * LD + x)), "l"(kb + src) : "memory");
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(skd::smem_u32(kd + (AP_BK + j) * LD + x)), "l"(vb + src) : "memory");
             }
@@ -873,8 +873,8 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
     const int ra = q0 + warp * 16 + g, rb = ra + 8, pa = base + ra, pb = base + rb;       // this lane's queries and their positions
     uint32_t qh[KS][4], ql[KS][4];
     {
-        const float* qa = q + (((int64_t) b * seq_q + min(ra, q_last)) * heads + h) * D + 2 * t;
-        const float* qb = q + (((int64_t) b * seq_q + min(rb, q_last)) * heads + h) * D + 2 * t;
+        const float* qa = q + ((int64_t) min(ra, q_last) * heads + h) * D + 2 * t;
+        const float* qb = q + ((int64_t) min(rb, q_last) * heads + h) * D + 2 * t;
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
             const float2 f[4] = {skd::ld_dep((const float2*) (qa + ks * 16)), skd::ld_dep((const float2*) (qb + ks * 16)), skd::ld_dep((const float2*) (qa + ks * 16 + 8)), skd::ld_dep((const float2*) (qb + ks * 16 + 8))};
@@ -891,9 +891,9 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                  // tile i is staged; every warp is done with tile i - 1
         fetch(i + 1);
-        const int k0 = lo + i * AP_BK;
+        const int k0 = i * AP_BK;
         // no query in the warp, or no key of the tile that one of its queries sees
-        if (q0 + warp * 16 > q_last || k0 > last || (window > 0 && k0 + AP_BK - 1 <= first - window)) continue;
+        if (q0 + warp * 16 > q_last || k0 > last) continue;
         const __half* kt = ring + (i & 1) * STAGE;
         const __half* vt = kt + AP_BK * LD;
         float s[8][4];
@@ -911,15 +911,14 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
                 mma_f16(s[n], qh[ks], f[0], f[1]);
                 mma_f16(s[n + 1], qh[ks], f[2], f[3]);
             }
-        // masked where the tile crosses the newest position or the window's far edge of a query
-        const bool edge = k0 + AP_BK - 1 > first || (window > 0 && k0 <= last - window);
+        const bool edge = k0 + AP_BK - 1 > first;         // the tile crosses the newest position of a query
         float mx[2] = {m[0], m[1]};
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = k0 + n * 8 + 2 * t + (j & 1), p = j < 2 ? pa : pb;
-                s[n][j] = !edge || (key <= p && (window <= 0 || p - key < window)) ? s[n][j] * scale : MASKED;
+                s[n][j] = !edge || key <= p ? s[n][j] * scale : MASKED;
                 mx[j >> 1] = fmaxf(mx[j >> 1], s[n][j]);
             }
         bool moved = false;
@@ -966,7 +965,7 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
             const int row = r ? rb : ra;
             if (row > q_last) continue;
             const float inv = l[r] > 0.0f ? 1.0f / l[r] : 0.0f;
-            float* d = out + (((int64_t) b * seq_q + row) * heads + h) * D + 2 * t;
+            float* d = out + ((int64_t) row * heads + h) * D + 2 * t;
 #pragma unroll
             for (int n = 0; n < NT; ++n) *(float2*) (d + n * 8) = make_float2(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
         }
@@ -1000,7 +999,7 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
             const float f = fast_exp(peer(rec_m + row, p) - mm);
             lt += f * peer(rec_l + row, p); at += f * peer(rec_o + row * OLD + d, p);
         }
-        out[(((int64_t) b * seq_q + q0 + row) * heads + h) * D + d] = lt > 0.0f ? at / lt : 0.0f;
+        out[((int64_t) (q0 + row) * heads + h) * D + d] = lt > 0.0f ? at / lt : 0.0f;
     }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody leaves while its records are read
@@ -1008,15 +1007,14 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
 
 // Parts of the keys: as many as keep all CTAs of the pass resident (two an SM), each with two tiles and more.
 template <int D>
-static int32_t launch_prompt(const float* q, const __half* k, const __half* v, float* out, int batch, int heads, int kv_heads, int seq_q, int seq_kv, int64_t cache_stride,
-                             float scale, int window, const int32_t* q_abs_base, cudaStream_t s) {
+static int32_t launch_prompt(const float* q, const __half* k, const __half* v, float* out, int heads, int kv_heads, int seq_q, int seq_kv, int64_t cache_stride,
+                             float scale, const int32_t* q_base, cudaStream_t s) {
     SK_TRY(ensure_dynamic_smem((const void*) attn_prompt_kernel<D>, ap_smem<D>()));
-    const int64_t tiles = (int64_t) heads * batch * ((seq_q + AP_ROWS - 1) / AP_ROWS);
-    const int keys = window > 0 ? std::min(seq_kv, window + AP_ROWS) : seq_kv;
+    const int64_t tiles = (int64_t) heads * ((seq_q + AP_ROWS - 1) / AP_ROWS);
     int parts = 1;
-    while (parts < 8 && tiles * parts * 2 <= 2 * sm_count() && parts * 2 * 2 * AP_BK <= keys) parts *= 2;
+    while (parts < 8 && tiles * parts * 2 <= 2 * sm_count() && parts * 2 * 2 * AP_BK <= seq_kv) parts *= 2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned) (heads * parts), (unsigned) ((seq_q + AP_ROWS - 1) / AP_ROWS), (unsigned) batch); cfg.blockDim = dim3(AP_THREADS);
+    cfg.gridDim = dim3((unsigned) (heads * parts), (unsigned) ((seq_q + AP_ROWS - 1) / AP_ROWS)); cfg.blockDim = dim3(AP_THREADS);
     cfg.dynamicSmemBytes = (size_t) ap_smem<D>(); cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1024,7 +1022,7 @@ static int32_t launch_prompt(const float* q, const __half* k, const __half* v, f
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = (unsigned) parts; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    SK_CUDA(cudaLaunchKernelEx(&cfg, attn_prompt_kernel<D>, q, k, v, out, heads, kv_heads, seq_q, cache_stride, q_abs_base, scale, window, parts));
+    SK_CUDA(cudaLaunchKernelEx(&cfg, attn_prompt_kernel<D>, q, k, v, out, heads, kv_heads, seq_q, cache_stride, q_base, scale, parts));
     return SKAINET_CUDA_OK;
 }
 // Fewest rows for the tiles of 64 queries: below, eight warps on the keys of eight queries finish sooner. Four layers of the 7B shape,
@@ -1038,9 +1036,9 @@ int32_t launch_sdpa_cache(const float* q, const __half* k, const __half* v, floa
                           int kv_heads, int seq_q, int seq_kv, int64_t cache_stride, int d, float scale, int window,
                           const int32_t* q_abs_base, cudaStream_t s) {
     if ((d == 128 || d == 64) && batch > 0 && seq_q > 0 && heads % kv_heads == 0 && batch <= 65535 && heads <= 65535) {
-        if (seq_q >= PROMPT_TILE_ROWS)
-            return d == 128 ? launch_prompt<128>(q, k, v, out, batch, heads, kv_heads, seq_q, seq_kv, cache_stride, scale, window, q_abs_base, s)
-                            : launch_prompt<64>(q, k, v, out, batch, heads, kv_heads, seq_q, seq_kv, cache_stride, scale, window, q_abs_base, s);
+        if (seq_q >= PROMPT_TILE_ROWS && batch == 1 && window <= 0)
+            return d == 128 ? launch_prompt<128>(q, k, v, out, heads, kv_heads, seq_q, seq_kv, cache_stride, scale, q_abs_base, s)
+                            : launch_prompt<64>(q, k, v, out, heads, kv_heads, seq_q, seq_kv, cache_stride, scale, q_abs_base, s);
         dim3 grid((seq_q + 7) / 8, heads, batch);
         if (d == 128) SK_CUDA(launch_pdl(attn_prefill_mma_kernel<128>, grid, dim3(AM_WARPS * 32), 0, s, q, k, v, out, heads, kv_heads, seq_q, cache_stride, q_abs_base, scale, window));
         else SK_CUDA(launch_pdl(attn_prefill_mma_kernel<64>, grid, dim3(AM_WARPS * 32), 0, s, q, k, v, out, heads, kv_heads, seq_q, cache_stride, q_abs_base, scale, window));
