@@ -259,18 +259,18 @@ attn_decode_mma_kernel(const float* q, int64_t q_row_stride, const __half* __res
     if (FUSE) {
         // score of head hg against the new key (fp32 rotated q, the cache's binary16 key), a warp per head at a time
         for (int hg = warp; hg < 8; hg += W) {
-        float sc_new = MASKED;
-        if (owner && hg < G) {
-            const float* qrow = q + (int64_t) b * q_row_stride + (int64_t) (kvh * G + hg) * D;
-            float p = 0.0f;
+            float sc_new = MASKED;
+            if (owner && hg < G) {
+                const float* qrow = q + (int64_t) b * q_row_stride + (int64_t) (kvh * G + hg) * D;
+                float p = 0.0f;
 #pragma unroll
-            for (int e0 = lane * 4; e0 < D; e0 += 128) {
-                const float4 f = rope_load4<D>(qrow, e0, step.cos_t, step.sin_t, pos_new, step.rope_mode);
-                p += f.x * sm_knew[e0] + f.y * sm_knew[e0 + 1] + f.z * sm_knew[e0 + 2] + f.w * sm_knew[e0 + 3];
+                for (int e0 = lane * 4; e0 < D; e0 += 128) {
+                    const float4 f = rope_load4<D>(qrow, e0, step.cos_t, step.sin_t, pos_new, step.rope_mode);
+                    p += f.x * sm_knew[e0] + f.y * sm_knew[e0 + 1] + f.z * sm_knew[e0 + 2] + f.w * sm_knew[e0 + 3];
+                }
+                sc_new = skd::warp_sum(p) * scale;
             }
-            sc_new = skd::warp_sum(p) * scale;
-        }
-        if (lane == 0) { sm_m[W][hg] = sc_new; sm_l[W][hg] = (owner && hg < G) ? 1.0f : 0.0f; }
+            if (lane == 0) { sm_m[W][hg] = sc_new; sm_l[W][hg] = (owner && hg < G) ? 1.0f : 0.0f; }
         }
     }
     uint32_t qa[KS][4];
@@ -982,15 +982,9 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
 #pragma unroll
         for (int n = 0; n < NT; ++n) *(float2*) (rec_o + row * OLD + n * 8 + 2 * t) = make_float2(o[n][2 * r], o[n][2 * r + 1]);
     }
-    auto peer = [](const float* p, int rank) {
-        uint32_t a;
-        float v;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(skd::smem_u32(p)), "r"(rank));
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-        return v;
-    };
+    auto peer = [](const float* p, int rank) { return skd::ld_cluster(skd::smem_u32(p), rank); };
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    skd::cluster_sync_all();
     for (int row = part * (AP_THREADS / D) + threadIdx.x / D; row <= q_last - q0; row += parts * (AP_THREADS / D)) {
         const int d = threadIdx.x % D;
         float mm = MASKED, lt = 0.0f, at = 0.0f;
@@ -1002,7 +996,7 @@ attn_prompt_kernel(const float* q, const __half* kc, const __half* vc, float* __
         out[((int64_t) (q0 + row) * heads + h) * D + d] = lt > 0.0f ? at / lt : 0.0f;
     }
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody leaves while its records are read
+    skd::cluster_sync_all();      // nobody leaves while its records are read
 }
 
 // Parts of the keys: as many as keep all CTAs of the pass resident (two an SM), each with two tiles and more.

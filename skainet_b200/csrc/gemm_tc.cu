@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "actquant.cuh"
 #include "tma.cuh"
+#include "f32x2.cuh"
 #include "matvec_fused.cuh"
 #include "tensor_map.cuh"
 
@@ -148,24 +149,6 @@ __device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[4 + i]); w[i] = __uint_as_float(r[8 + i]); }
 }
-// packed fp32 pairs, each half rounded as the scalar operation
-__device__ __forceinline__ uint64_t pk2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float2 up2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {      // the same shared-memory address in CTA `rank` of the cluster
-    uint32_t a;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-
 // ---- activation side: int8 codes -> f16 in core-matrix order, sums of 16 codes, transposed block scales (tile = N = 1 << nlog rows) ----
 //   xh  [m_pad/N][cols/64][N/8][8 rows][8][8]  f16: the N x 64 k pieces of a super-block are contiguous, rows of 128 B
 //                                               whose 16-byte chunks are XOR-swizzled with the row (128B swizzle);
@@ -415,7 +398,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             tc_fence_after();
             const uint32_t dd = *reinterpret_cast<const uint32_t*>(smem + S::OFF_DD + ((i & 3) * TC_M + r) * 4);
             const float dw = __half2float(__ushort_as_half((unsigned short) (dd & 0xffff))), dminw = __half2float(__ushort_as_half((unsigned short) (dd >> 16)));
-            const uint64_t dw2 = pk2(dw, dw), nd2 = pk2(-dminw, -dminw);
+            const uint64_t dw2 = skd::pk2(dw, dw), nd2 = skd::pk2(-dminw, -dminw);
             const float* dx = (const float*) (smem + S::OFF_DX) + (i & 3) * N + ch * NC;
             const uint32_t t0 = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + ch * NC, t2 = t0 + S::COL_S2 + (S::S2_SETS == 2 ? set * N : 0);
 #pragma unroll
@@ -431,10 +414,10 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
 #pragma unroll
                 for (int j = 0; j < LD; j += 2) {
                     const float2 x2 = *reinterpret_cast<const float2*>(dx + c + j);
-                    uint64_t sum = pk2(s1[j], s1[j + 1]);
-                    if (S::S1_ACC == 2) sum = add2(sum, pk2(s1b[j], s1b[j + 1]));
+                    uint64_t sum = skd::pk2(s1[j], s1[j + 1]);
+                    if (S::S1_ACC == 2) sum = skd::add2(sum, skd::pk2(s1b[j], s1b[j + 1]));
                     uint64_t& y2 = yacc[(c + j) / 2];
-                    y2 = fma2(pk2(x2.x, x2.y), fma2(dw2, sum, mul2(nd2, pk2(s2[j], s2[j + 1]))), y2);
+                    y2 = skd::fma2(skd::pk2(x2.x, x2.y), skd::fma2(dw2, sum, skd::mul2(nd2, skd::pk2(s2[j], s2[j + 1]))), y2);
                 }
             }
         }
@@ -444,7 +427,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             float* mine = (float*) (smem + S::OFF_B) + (ch * NC) * TC_M + r;
 #pragma unroll
             for (int c = 0; c < NC / 2; ++c) {
-                const float2 v = up2(yacc[c]);
+                const float2 v = skd::up2(yacc[c]);
                 mine[(2 * c) * TC_M] = v.x; mine[(2 * c + 1) * TC_M] = v.y;
             }
         } else {
@@ -452,7 +435,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
             if (ok && row0 + r < rows) {
 #pragma unroll
                 for (int c = 0; c < NC / 2; ++c) {
-                    const float2 v = up2(yacc[c]);
+                    const float2 v = skd::up2(yacc[c]);
                     const int col = col0 + ch * NC + 2 * c;
                     const size_t o = (size_t) col * rows + row0 + r;
                     if (col < m) y[o] = resid ? resid[o] + v.x : v.x;
@@ -469,22 +452,22 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     }
     if (parts > 1) {
         __syncwarp();
-        cluster_sync_all();                            // every part's sums are in place
+        skd::cluster_sync_all();                            // every part's sums are in place
         skd::pdl_wait();
         const uint32_t base = skd::smem_u32(smem + S::OFF_B);
         bool whole = true;
-        for (int p = 0; p < parts; ++p) whole = whole && ld_cluster(skd::smem_u32(gave_up), p) == 0.0f;
+        for (int p = 0; p < parts; ++p) whole = whole && skd::ld_cluster(skd::smem_u32(gave_up), p) == 0.0f;
         const int per = (N * TC_M / 4 + parts - 1) / parts * 4, e0 = part * per, e1 = min(N * TC_M, e0 + per);
         for (int e = e0 + tid; e < e1; e += S::THREADS) {
             const int row = row0 + (e & (TC_M - 1)), col = col0 + e / TC_M;
             if (!whole || row >= rows || col >= m) continue;
             float v = 0.0f;
-            for (int p = 0; p < parts; ++p) v += ld_cluster(base + e * 4, p);
+            for (int p = 0; p < parts; ++p) v += skd::ld_cluster(base + e * 4, p);
             const size_t o = (size_t) col * rows + row;
             y[o] = resid ? resid[o] + v : v;           // resid may be y itself: read and written by this thread only
         }
         __syncwarp();
-        cluster_sync_all();                            // nobody leaves while its sums are still read
+        skd::cluster_sync_all();                            // nobody leaves while its sums are still read
     }
 }
 

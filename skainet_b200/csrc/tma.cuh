@@ -42,14 +42,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// The bounded wait by a whole warp, with one verdict for all its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* timeout_flag) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, timeout_flag));
+}
+
 // Programmatic dependent launch: let the next kernel in the stream start its independent prologue
 // now; and wait until every kernel this one depends on has completed and flushed its writes.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// The same by a whole warp, with one verdict for all its lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* timeout_flag) {
-    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, timeout_flag));
+// The CTAs of a cluster: a barrier of all their threads (warps whole), and a read of the same shared-memory address in CTA `rank`.
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
 // One lane of a converged warp. Loops that issue tcgen05 or TMA instructions are run by the whole warp, with only the instructions

@@ -12,6 +12,7 @@
 #include "turboquant.cuh"
 #include "attn_frag.cuh"
 #include "tma.cuh"
+#include "f32x2.cuh"
 
 #include <algorithm>
 
@@ -20,12 +21,6 @@ namespace sk {
 namespace {
 
 constexpr int TA_WARPS = 8;
-
-__device__ __forceinline__ uint64_t pk2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float2 up2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 // Half a row's block as it lies in the store: EL elements
 template <int EL>
@@ -60,7 +55,7 @@ __device__ __forceinline__ void load_packed(Packed<EL>& p, const TqPlane& pl, in
 template <int EL, int BITS>
 __device__ __forceinline__ void scaled_codes(const Packed<EL>& p, uint64_t (&v)[EL / 2]) {
     constexpr float BIAS = 8388608.0f + (float) (1 << (BITS - 1));       // 2^23 + u has u in its low mantissa bits
-    const uint64_t nb = pk2(-BIAS, -BIAS);
+    const uint64_t nb = skd::pk2(-BIAS, -BIAS);
 #pragma unroll
     for (int i = 0; i < EL / 2; ++i) {
         uint32_t u[2];
@@ -73,8 +68,8 @@ __device__ __forceinline__ void scaled_codes(const Packed<EL>& p, uint64_t (&v)[
                 u[k] = (x & ((1u << BITS) - 1)) | 0x4b000000u;
             }
         }
-        const uint64_t sc = pk2(p.scale[i / 16], p.scale[i / 16]);
-        v[i] = mul2(add2(pk2(__uint_as_float(u[0]), __uint_as_float(u[1])), nb), sc);
+        const uint64_t sc = skd::pk2(p.scale[i / 16], p.scale[i / 16]);
+        v[i] = skd::mul2(skd::add2(skd::pk2(__uint_as_float(u[0]), __uint_as_float(u[1])), nb), sc);
     }
 }
 
@@ -88,21 +83,21 @@ __device__ __forceinline__ void decode_half_row(const Packed<EL>& p, int bits, i
         case 4: scaled_codes<EL, 4>(p, v); break;
         default: scaled_codes<EL, 8>(p, v); break;
     }
-    const uint64_t minus = pk2(-1.0f, -1.0f);
+    const uint64_t minus = skd::pk2(-1.0f, -1.0f);
 #pragma unroll
-    for (int i = 0; i < EL / 2; ++i) { const float2 a = up2(v[i]); v[i] = pk2(__fadd_rn(a.x, a.y), __fsub_rn(a.x, a.y)); }
+    for (int i = 0; i < EL / 2; ++i) { const float2 a = skd::up2(v[i]); v[i] = skd::pk2(__fadd_rn(a.x, a.y), __fsub_rn(a.x, a.y)); }
 #pragma unroll
     for (int h = 1; h < EL / 2; h <<= 1) {
 #pragma unroll
         for (int i = 0; i < EL / 2; ++i) {
             if ((i & h) == 0) {
                 const uint64_t a = v[i], b = v[i + h];
-                v[i] = add2(a, b); v[i + h] = fma2(b, minus, a);
+                v[i] = skd::add2(a, b); v[i + h] = skd::fma2(b, minus, a);
             }
         }
     }
     const float s = half ? -1.0f : 1.0f, nf = __fdiv_rn(1.0f, __fsqrt_rn((float) (2 * EL)));
-    const uint64_t s2 = pk2(s, s), norm = pk2(nf, nf);
+    const uint64_t s2 = skd::pk2(s, s), norm = skd::pk2(nf, nf);
     uint32_t z[EL / 32];                               // signs of the even elements in the low half, of the odd ones in the high half
 #pragma unroll
     for (int g = 0; g < EL / 32; ++g) {
@@ -117,9 +112,9 @@ __device__ __forceinline__ void decode_half_row(const Packed<EL>& p, int bits, i
     uint32_t out[EL / 2];
 #pragma unroll
     for (int i = 0; i < EL / 2; ++i) {
-        const float2 a = up2(v[i]);
-        const uint64_t o = pk2(__shfl_xor_sync(0xffffffffu, a.x, 1), __shfl_xor_sync(0xffffffffu, a.y, 1));
-        const float2 r = up2(mul2(fma2(v[i], s2, o), norm));       // the lower half takes the sums, the upper the differences
+        const float2 a = skd::up2(v[i]);
+        const uint64_t o = skd::pk2(__shfl_xor_sync(0xffffffffu, a.x, 1), __shfl_xor_sync(0xffffffffu, a.y, 1));
+        const float2 r = skd::up2(skd::mul2(skd::fma2(v[i], s2, o), norm));       // the lower half takes the sums, the upper the differences
         const __half2 h = __floats2half2_rn(r.x, r.y);
         out[i] = *reinterpret_cast<const uint32_t*>(&h) ^ ((z[i / 16] << (15 - i % 16)) & 0x80008000u);
     }
