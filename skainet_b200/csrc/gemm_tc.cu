@@ -393,8 +393,8 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
         bool ok = true;
         for (int i = 0; i < nk; ++i) {
             const int set = i & 1;
-            if (!(ok = skd::mbar_wait_warp(acc_full + set, (i >> 1) & 1, timeout_flag))) break;
-            if (!(ok = skd::mbar_wait_warp(s2_full + (i & 3), (i >> 2) & 1, timeout_flag))) break;      // long complete; observed for what it guards
+            // the second long complete; observed for what it guards
+            if (!(ok = skd::mbar_wait_warp(acc_full + set, (i >> 1) & 1, timeout_flag) && skd::mbar_wait_warp(s2_full + (i & 3), (i >> 2) & 1, timeout_flag))) { *gave_up = 1; break; }
             tc_fence_after();
             const uint32_t dd = *reinterpret_cast<const uint32_t*>(smem + S::OFF_DD + ((i & 3) * TC_M + r) * 4);
             const float dw = __half2float(__ushort_as_half((unsigned short) (dd & 0xffff))), dminw = __half2float(__ushort_as_half((unsigned short) (dd >> 16)));
@@ -423,7 +423,6 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
         }
         if (parts > 1) {
             // this part's sums into shared memory, [column][row], where the activation tiles were (all MMAs have read them)
-            if (!ok) *gave_up = 1;
             float* mine = (float*) (smem + S::OFF_B) + (ch * NC) * TC_M + r;
 #pragma unroll
             for (int c = 0; c < NC / 2; ++c) {
