@@ -829,12 +829,12 @@ attn_prefill_mma_kernel(const float* q, const __half* kc, const __half* vc, floa
 }
 
 // =================================================================================================
-// The same for many rows of one sequence's prompt, without a window: CTA = 64 consecutive queries of one head, a warp 16 of them, over tiles of 64 keys that the four
-// warps share through shared memory. q and the probabilities are carried as two f16 terms, one MMA each against the f16 cache rows.
-// With eight queries a CTA, each fetching all keys into registers by itself, the L2 reads bounded it: 512 rows x 32 heads
-// 82 us (a 512-token prompt of the 7B shape 21.5 ms, 20.1 with this kernel). Few queries over many keys leave SMs idle: then a cluster of `parts` CTAs shares the keys of a tile of queries, and their
-// records meet in shared memory, folded in the order of the parts. grid (heads * parts, ceil(seq_q / 64)), the queries with
-// the most keys first.
+// The same for many rows of one sequence's prompt, without a window: CTA = 64 consecutive queries of one head, a warp 16 of them, over
+// tiles of 64 keys that the four warps share through shared memory. q and the probabilities are carried as two f16 terms, one MMA each
+// against the f16 cache rows. With eight queries a CTA, each fetching all keys into registers by itself, the L2 reads bounded it: 512 rows
+// x 32 heads 82 us, 38 with this kernel (a 512-token prompt of the 7B shape 1.4 ms less). Few queries over many keys leave SMs idle: then
+// a cluster of `parts` CTAs shares the keys of a tile of queries, and their records meet in shared memory, folded in the order of the
+// parts. grid (heads * parts, ceil(seq_q / 64)), the queries with the most keys first.
 // =================================================================================================
 constexpr int AP_ROWS = 64, AP_BK = 64, AP_THREADS = 128;
 template <int D> constexpr int ap_smem() { return 2 * 2 * AP_BK * (D + 8) * 2; }       // two stages of keys | values
