@@ -672,6 +672,20 @@ int32_t launch_mma(const LatentArgs& a, const SplitArgs& sp, dim3 grid, cudaStre
     return nt <= 1 ? run_mma<MW, 1>(a, sp, grid, s) : nt <= 2 ? run_mma<MW, 2>(a, sp, grid, s) : nt <= 4 ? run_mma<MW, 4>(a, sp, grid, s) : run_mma<MW, 8>(a, sp, grid, s);
 }
 
+// Whether forming the keys and values of `slots` positions costs a prompt pass less than folding W_uk into its queries. Microseconds a layer,
+// fitted to both forms over ranks 64 to 512, windows 64 to 4096, 4 and 16 heads, 64 to 2048 rows: the expanded form walks the keys tile by
+// tile in one CTA per 128 rows and head (3.4 a tile), the folded one splits them and is bound by its (row, key, head) triples whatever the
+// rank, behind three more launches. Expanded / folded, eight layers of rank 512 in us: 200 rows behind a window of 4096 with 16 heads
+// 2422 / 2046, with 4 heads 2263 / 972; 400 rows with 16 heads 2448 / 4576; 192 rows behind 64 keys 557 / 755, behind 1024 with 4 heads
+// 887 / 721; 2048 rows behind 1024 with 16 heads 1757 / 5319.
+bool expanding_pays(const LatentArgs& a, int slots) {
+    const int heads = a.g.heads, ctas = heads * ((a.rows + EX_ROWS - 1) / EX_ROWS), reach = std::min(a.window, a.kv_bound);
+    const float tiles = (float) ((reach + std::min(a.rows, EX_ROWS) + EX_BK - 1) / EX_BK), rounds = (float) ((ctas + sm_count() - 1) / sm_count());
+    const float keys = (float) std::min(a.window, a.kv_bound - a.rows / 2);          // that a row sees, on average
+    const float expanded = 3.4f * tiles * rounds + (float) slots * (float) heads * 2.0f * EX_DIM * (float) a.g.kv_rank / 350e6f;
+    return expanded < 28.0f + (float) a.rows * keys * (float) heads / 90e3f;
+}
+
 }  // namespace
 
 int32_t launch_latent_attention(const LatentArgs& args, cudaStream_t s) {
@@ -686,11 +700,11 @@ int32_t launch_latent_attention(const LatentArgs& args, cudaStream_t s) {
         if (a.f32_act) SK_CUDA(launch_pdl(latent_prep_kernel<float>, dim3(a.rows), dim3(256), 0, s, a));
         else SK_CUDA(launch_pdl(latent_prep_kernel<bf16>, dim3(a.rows), dim3(256), 0, s, a));
         LinearArgs l;
-        if (a.kv && a.map.seq >= 0 && a.rows >= LATENT_EXPAND_ROWS) {
-            // keys and values of the positions that a row of the pass sees, in the one or two runs of slots they lie in, then attention over
-            // them; out is final
-            const int cap = a.cache.cap, last = a.kv_bound, first = (int) std::max<int64_t>(0, (int64_t) last - a.rows - a.window + 1);
-            const int n = std::min(cap, last - first), slot = n == cap ? 0 : first % cap;
+        // the positions that a row of the pass sees, in the one or two runs of slots they lie in
+        const int cap = a.cache.cap, first = (int) std::max<int64_t>(0, (int64_t) a.kv_bound - a.rows - a.window + 1);
+        const int n = std::min(cap, a.kv_bound - first), slot = n == cap ? 0 : first % cap;
+        if (a.kv && a.map.seq >= 0 && a.rows >= LATENT_EXPAND_ROWS && expanding_pays(a, n)) {
+            // their keys and values, then attention over them; out is final
             l.w = a.ukv; l.w_rows = g.heads * 2 * g.dim; l.ldw = g.rank_ld(); l.ldx = g.key_ld(); l.ldy = l.w_rows; l.out = LIN_OUT_ACT;
             for (int at = slot, left = n; left > 0; at = 0) {
                 l.rows = std::min(left, cap - at); l.x_rows_alloc = cap - at;

@@ -56,7 +56,7 @@ struct LatentArgs {
 };
 
 constexpr int LATENT_FUSED_ROWS = 4;      // rows up to which the folds of W_uk and W_uv run inside the kernels around attention
-// The expanded form's geometry, and the prompt rows from which forming the keys and values pays.
+// The expanded form's geometry, and the prompt rows from which it is considered.
 constexpr bool latent_expands(const LatentGeom& g) { return g.dim == 128 && g.rot_dim == 64 && g.vdim == 128 && g.kv_rank % 64 == 0; }
 constexpr int LATENT_EXPAND_ROWS = 192;
 constexpr size_t LATENT_EXPAND_MAX_BYTES = (size_t) 256 << 20, LATENT_EXPAND_COPY_BYTES = (size_t) 1 << 30;      // of keys and values, of weights laid out for them

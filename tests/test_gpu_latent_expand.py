@@ -14,7 +14,7 @@ from test_gpu_tivazen import TOL, make  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("window,kv_rank,heads", [(1, 64, 2), (63, 64, 3), (64, 128, 1), (65, 64, 2), (200, 192, 2), (700, 64, 3)])
+@pytest.mark.parametrize("window,kv_rank,heads", [(1, 64, 2), (63, 64, 3), (64, 128, 1), (65, 64, 2), (200, 192, 2), (700, 64, 3), (700, 64, 16)])
 def test_windows_and_cuts(make, window, kv_rank, heads):  # noqa: F811
     a = dict(heads=heads, dim=128, rot_dim=64, vdim=128, kv_rank=kv_rank, scale=0.08)
     cfg = M.config([(M.attn(window=window, **a), M.dense(40)), (M.attn(window=min(window, 90), kv_from=0, **a), None)], width=64)
