@@ -198,6 +198,8 @@ SKAINET_CUDA_API int32_t skainet_cuda_weight_dequant(skainet_weight_t w, float* 
 
 /* y[m, rows] = x[m, cols] . W^T on the device. Q4_K / Q8_0: the dequant-fused matvec for m = 1 (and Q4_K up to
  * 2 rows), tensor-core tile kernels above that (mma.sync; tcgen05 with TMEM accumulators for Q4_K, from 9 rows where it is the quicker).
+ * The fp32 sums over the blocks of a Q4_K or Q8_0 row run in an order that depends on the number of rows of the call (its kernel, and
+ * how many CTAs share a tile), so a row's result may differ in its last places from that of the same row in another call.
  * Q6_K (native mode = int8 activations per 256 like skainet_q6k_matmul_rm, native/src/q6k_matmul.c:344-357): one warp
  * per output row and up to eight activation rows per pass over the weight, an mma.sync tile kernel from nine rows,
  * every row bit-identical to the single-row result. Q5_K (fp32 activations in both modes, native/src/q5k_matmul.c):
