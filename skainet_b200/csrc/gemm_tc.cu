@@ -121,21 +121,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t tb, float (&u)[8]
 #pragma unroll
     for (int i = 0; i < 8; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(q[i]); }
 }
-// the same of three places, eight or four columns each
-__device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, float (&u)[8], float (&v)[8], float (&w)[8]) {
-    uint32_t r[24];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%24];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%25];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%26];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
-        : "r"(ta), "r"(tb), "r"(tc)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[8 + i]); w[i] = __uint_as_float(r[16 + i]); }
-}
+// the same of three places, four columns each
 __device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, float (&u)[4], float (&v)[4], float (&w)[4]) {
     uint32_t r[12];
     asm volatile(
@@ -386,7 +372,7 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     } else {
         // ------------------------------- epilogue: fold every super-block out of TMEM -------------------------------
         const int r = tid & 127, ch = (warp - S::PROD_WARPS) >> 2;      // TMEM lane = weight row; which half of the columns
-        constexpr int NC = N / 2, LD = N == 64 ? 4 : 8;                 // columns a load: as many as the registers take
+        constexpr int NC = N / 2, LD = S::S1_ACC == 2 ? 4 : 8;          // columns a load: what the registers take (eight are no faster at N = 32)
         uint64_t yacc[NC / 2];
 #pragma unroll
         for (int c = 0; c < NC / 2; ++c) yacc[c] = 0;
