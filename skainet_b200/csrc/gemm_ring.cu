@@ -110,6 +110,7 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
     const int8_t* act_q = skd::behind_wait(act.q);
     const int16_t* act_bsums = skd::behind_wait(act.bsums);
     const float* act_d = skd::behind_wait(act.d);
+    const float* res = skd::behind_wait(resid);
     if (!XG) {
         const int ct = (grp * GR_BLKS + warp) * 32 + lane, nct = NG * GR_BLKS * 32;          // this thread among the consumer threads of the CTA
         for (int c = ct; c < GR_MT * (cols >> 4); c += nct) {                 // 16 codes
@@ -234,7 +235,7 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
                 const int row = row0 + g + 8 * (j >> 1), col = 2 * t + (j & 1);
                 if (row < rows && col < m) {
                     const size_t o = (size_t) col * rows + row;
-                    y[o] = EPI == EPI_ADD ? resid[o] + out[j] : out[j];
+                    y[o] = EPI == EPI_ADD ? skd::ld_free(res + o) + out[j] : out[j];
                 }
             }
         }

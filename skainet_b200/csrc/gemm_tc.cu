@@ -440,8 +440,8 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
         skd::cluster_sync_all();                            // every part's sums are in place
         skd::pdl_wait();
         const uint32_t base = skd::smem_u32(smem + S::OFF_B);
-        bool whole = true;
-        for (int p = 0; p < parts; ++p) whole = whole && skd::ld_cluster(skd::smem_u32(gave_up), p) == 0.0f;
+        // one flag a lane: read in turn they cost 0.4 us a call of four parts
+        const bool whole = !__any_sync(0xffffffffu, lane < parts && skd::ld_cluster(skd::smem_u32(gave_up), lane) != 0.0f);
         const int per = (N * TC_M / 4 + parts - 1) / parts * 4, e0 = part * per, e1 = min(N * TC_M, e0 + per);
         for (int e = e0 + tid; e < e1; e += S::THREADS) {
             const int row = row0 + (e & (TC_M - 1)), col = col0 + e / TC_M;
