@@ -245,10 +245,10 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
 
 template <int NG, bool XG>
 int32_t launch_rows_ring_ng(const Weight& w, ActQ8K a, int m, float* y, const float* resid, size_t fixed, int x_stride, cudaStream_t s) {
-    if (GR_BUDGET <= fixed) return 1;
-    const int ns = (int) std::min<size_t>(GR_MAX_STAGES, (GR_BUDGET - fixed - (size_t) NG * (2 * GR_BLKS * 128 * 4 + 2 * GR_MAX_STAGES * 8)) / ((size_t) NG * GR_STAGE));
-    if (ns < 3) return 1;
-    const size_t smem = (size_t) NG * ns * GR_STAGE + fixed + (size_t) NG * (2 * GR_BLKS * 128 * 4 + 2 * GR_MAX_STAGES * 8) + 128;
+    const size_t beside = fixed + (size_t) NG * (2 * GR_BLKS * 128 * 4 + 2 * GR_MAX_STAGES * 8);      // rows, partial tiles, barriers
+    if (GR_BUDGET < beside + 3 * (size_t) NG * GR_STAGE) return 1;
+    const int ns = (int) std::min<size_t>(GR_MAX_STAGES, (GR_BUDGET - beside) / ((size_t) NG * GR_STAGE));
+    const size_t smem = (size_t) NG * ns * GR_STAGE + beside + 128;
     const int nrg = (w.rows + GR_ROWS - 1) / GR_ROWS, grid = std::min(sm_count(), (nrg + NG - 1) / NG);
     int* flag = device_timeout_flag();
     if (resid) {
