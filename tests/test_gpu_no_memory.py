@@ -1,0 +1,123 @@
+"""What runs on when device memory is short: nearly all of it is taken by buffers that nothing touches, and given back at the end."""
+import ctypes as C
+import gc
+import os
+
+import numpy as np
+import pytest
+
+import tivazen_models as M
+from conftest import rel_err_ok
+from oracle import tivazen as F
+from skainet_b200 import _lib as L
+from test_gpu_tivazen import TOL
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def hog(gpu):
+    """hog(leave): takes device memory until about `leave` bytes are left. release() ends it."""
+    import torch
+    held = []
+
+    def take(leave):
+        gc.collect()
+        part = 1
+        while part <= 1 << 16:
+            size = (torch.cuda.mem_get_info()[0] - leave) // part
+            if size < 2 << 20:
+                return
+            try:
+                held.append(gpu.DeviceBuffer(size))
+            except Exception:
+                part *= 2
+
+    def release():
+        for b in held:
+            b.free()
+        held.clear()
+
+    take.release = release
+    yield take
+    release()
+
+
+def test_rows_without_operand_scratch(gpu, hog):
+    """Rows for the tcgen05 kernel whose scratch cannot be had go to the kernel that needs none. (The quantized rows find theirs: a call over a
+    Q6_K weight of as many inputs left it.)"""
+    rng = np.random.default_rng(1)
+    m, n, k = 64, 1024, 22016
+    stream = C.c_void_p()
+    L.check(L.lib().skainet_cuda_stream_create(C.byref(stream)))
+    w, other = gpu.Weight.synth("Q4_K", n, k, seed=5, std=0.02), gpu.Weight.upload(np.zeros(64 * (k // 256) * 210, np.uint8), "Q6_K", 64, k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    want = np.concatenate([gpu.matmul_host(w, x[i:i + 8]) for i in range(0, m, 8)])
+    dx, dy, dz = gpu.DeviceBuffer.from_host(x), gpu.DeviceBuffer(4 * m * n), gpu.DeviceBuffer(4 * m * 64)
+    gpu.matmul(other, dx.ptr, m, dz.ptr, stream=stream.value)
+    small = gpu.Weight.synth("Q4_K", 64, 256, seed=5, std=0.02)        # the kernel that takes over is loaded
+    assert gpu.q4k_rows_plan(small, m)[0] == 0 and gpu.q4k_rows_plan(w, m)[0] == 64
+    gpu.matmul(small, dx.ptr, m, dz.ptr, stream=stream.value)
+    gpu.sync(stream.value)
+    hog(3 << 20)
+    gpu.matmul(w, dx.ptr, m, dy.ptr, stream=stream.value)
+    gpu.sync(stream.value)
+    hog.release()
+    rel_err_ok(dy.download(np.float32, m * n).reshape(m, n), want, 1e-5)
+    gpu.matmul(w, dx.ptr, m, dy.ptr, stream=stream.value)              # with memory, the tcgen05 kernel again
+    gpu.sync(stream.value)
+    rel_err_ok(dy.download(np.float32, m * n).reshape(m, n), want, 1e-5)
+    L.check(L.lib().skainet_cuda_stream_destroy(stream))
+    for each in (w, other, small):
+        each.free()
+
+
+def loaded(path, cfg, **runtime):
+    """A Tivazen model with its weights, not finalized."""
+    from skainet_b200 import tivazen as T
+    from skainet_b200.safetensors import SafetensorsReader
+    m = T.Tivazen(T.TivazenConfig.from_json(cfg, **runtime))
+    r = SafetensorsReader(os.path.join(path, "model.safetensors"))
+    m.load(r)
+    r.close()
+    return m
+
+
+def test_prompts_without_room_for_expanded_weights(gpu, hog, tmp_path):
+    """Where finalize finds no memory for the weights of the expanded form of latent attention, prompts take the folded form."""
+    cfg = M.config([(M.attn(heads=16, dim=128, rot_dim=64, vdim=128, kv_rank=512, scale=0.08, window=100), None)], width=64)
+    w = M.random_weights(cfg, 7)
+    path, t, out = M.save(tmp_path, cfg, w), M.tokens(cfg, 400), []
+    for short in (True, False):
+        m = loaded(path, cfg, max_seq=600, prefill_rows=300)
+        if short:
+            hog(2 << 20)
+        m.finalize()
+        hog.release()
+        out.append(m.forward(t, list(range(400))))
+        assert M.error(out[-1], F.forward(cfg, w, t)) < TOL["bfloat16"]
+        m.free()
+    assert not np.array_equal(*out)
+
+
+def test_shorter_passes_where_memory_is_short(gpu, hog, tmp_path):
+    """The library's choice of a pass is 2048 rows, and 1024 where those would leave too little memory: the model then takes the memory of one that
+    asks for passes of 1024 rows, and reads a longer prompt."""
+    import torch
+    cfg = M.config([(M.attn(heads=16, dim=128, rot_dim=64, vdim=128, kv_rank=512, scale=0.08, window=64), None) for _ in range(2)], width=64)
+    w = M.random_weights(cfg, 7)
+    path, t, used = M.save(tmp_path, cfg, w), M.tokens(cfg, 1100), {}
+    want = F.forward(cfg, w, t)[[700, 1099]]
+    for rows, left in ((1024, 0), (2048, 0), (0, 0), (0, 1 << 30)):
+        if left:
+            hog(left)
+        before = torch.cuda.mem_get_info()[0]
+        m = loaded(path, cfg, max_seq=2400, max_batch=8, prefill_rows=rows)
+        used[rows, left] = before - torch.cuda.mem_get_info()[0]
+        hog.release()
+        m.finalize()
+        assert M.error(m.forward(t, [700, 1099]), want) < TOL["bfloat16"]
+        m.free()
+    small, large = used[1024, 0], used[2048, 0]
+    assert large - small > 32 << 20
+    assert abs(used[0, 0] - large) < 8 << 20 and abs(used[0, 1 << 30] - small) < 8 << 20
