@@ -221,6 +221,11 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
         // the eight warps' partial tiles -> one; two buffers, so one barrier per row group is enough
         float* part = s_part + pbuf * GR_BLKS * 128;
         *reinterpret_cast<float4*>(part + warp * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        float prior[4] = {0.f, 0.f, 0.f, 0.f};           // the residual, on its way while the partial tiles meet
+        if (EPI == EPI_ADD && warp == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) prior[j] = skd::ld_dep(res + (size_t) min(2 * t + (j & 1), m - 1) * rows + min(row0 + g + 8 * (j >> 1), rows - 1));
+        }
         gr_group_sync(grp);
         if (warp == 0) {
             float4 v = *reinterpret_cast<const float4*>(part + lane * 4);
@@ -235,7 +240,7 @@ q4k_rows_ring_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
                 const int row = row0 + g + 8 * (j >> 1), col = 2 * t + (j & 1);
                 if (row < rows && col < m) {
                     const size_t o = (size_t) col * rows + row;
-                    y[o] = EPI == EPI_ADD ? skd::ld_free(res + o) + out[j] : out[j];
+                    y[o] = EPI == EPI_ADD ? prior[j] + out[j] : out[j];
                 }
             }
         }
