@@ -93,7 +93,8 @@ struct Tivazen : Decoder {
     }
     // W_uk back in its own orientation, with W_uv below it, for the layers whose prompts take the expanded form of attention; the room
     // for the widest of their caches is shared, since a layer uses it within its own attention only. A layer whose copy finds no memory,
-    // or would take all copies past LATENT_EXPAND_COPY_BYTES, keeps the folded form.
+    // or would take all copies past LATENT_EXPAND_COPY_BYTES, keeps the folded form; so do all where little memory would be left behind the
+    // copies (scratch grows later; and whether a copy just fits would depend on how the free memory lies).
     int32_t expand_weights() {
         auto none = [&]() { for (auto& L : layers) if (L.ukv) { weight_release(L.ukv); L.ukv = nullptr; } };
         auto room_of = [&](const TvLayer& L) -> size_t {
@@ -115,7 +116,8 @@ struct Tivazen : Decoder {
             SK_TRY(launch_transpose_heads(data(L.uk), dst, g.heads, g.kv_rank, g.dim, nullptr));
             SK_CUDA(cudaMemcpy(dst + (size_t) g.heads * g.dim * g.rank_ld(), L.uv->qs, (size_t) g.heads * g.vdim * g.rank_ld() * 2, cudaMemcpyDeviceToDevice));
         }
-        if (!kv) none();
+        size_t free = 0, total = 0;
+        if (!kv || (cudaMemGetInfo(&free, &total) == cudaSuccess && free < LATENT_EXPAND_SPARE_BYTES)) none();
         SK_CUDA(cudaStreamSynchronize(nullptr));
         return st == SKAINET_CUDA_ERR_OOM ? SKAINET_CUDA_OK : st;
     }
