@@ -704,9 +704,9 @@ def run_gemm(args) -> None:
     peak, peak_kind = load_tensor_peak()
     achieved = ops / (ms_step * 1e-3) / 1e12
     if enc == "Q4_K":
-        kernel = "q4k_gemm_tc_kernel" if m >= 288 else "q4k_gemm_mma_kernel"
+        kernel = "kq_gemm_tc_kernel" if m >= 288 else "q4k_gemm_mma_kernel"
     elif enc == "Q6_K":
-        kernel = "q6k_gemm_mma_kernel" if m >= 9 else "q6k_rows_kernel"
+        kernel = "kq_gemm_tc_kernel" if m >= 9 else "q6k_rows_kernel"
     else:
         kernel = "q5k_gemm_mma_kernel" if m >= 5 else "q5k_rows_kernel"
     line = {"metric": f"{args.workload}_tflops", "value": achieved, "unit": "TFLOP/s", "n_gpus": 1, "steps": args.steps, "warmup": warm,

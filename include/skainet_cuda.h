@@ -201,7 +201,7 @@ SKAINET_CUDA_API int32_t skainet_cuda_weight_dequant(skainet_weight_t w, float* 
  * The fp32 sums over the blocks of a Q4_K or Q8_0 row run in an order that depends on the number of rows of the call (its kernel, and
  * how many CTAs share a tile), so a row's result may differ in its last places from that of the same row in another call.
  * Q6_K (native mode = int8 activations per 256 like skainet_q6k_matmul_rm, native/src/q6k_matmul.c:344-357): one warp
- * per output row and up to eight activation rows per pass over the weight, an mma.sync tile kernel from nine rows,
+ * per output row and up to eight activation rows per pass over the weight, a tcgen05 tile kernel for more (and where it is the quicker),
  * every row bit-identical to the single-row result. Q5_K (fp32 activations in both modes, native/src/q5k_matmul.c):
  * one warp per output row, up to four activation rows per pass; from five rows (native mode) an mma.sync tile kernel
  * with the activation carried as two f16 terms.

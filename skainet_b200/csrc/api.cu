@@ -534,7 +534,7 @@ int32_t skainet_cuda_selftest_q4k_rows_dev(skainet_weight_t h, const float* x_de
     Weight* w = weight_from_handle(h);
     if (!w) return SKAINET_CUDA_ERR_HANDLE;
     SK_REQUIRE(w->enc == SKAINET_ENC_Q4_K, "q4k_rows: encoding %d", w->enc);
-    SK_REQUIRE((tile == 32 || tile == 64 || tile == 128) && parts >= 1 && parts <= 8 && parts <= w->bpr, "q4k_rows: tiles of %d rows in %d parts", tile, parts);
+    SK_REQUIRE((tile == 16 || tile == 32 || tile == 64 || tile == 128) && parts >= 1 && parts <= 8 && parts <= w->bpr, "q4k_rows: tiles of %d rows in %d parts", tile, parts);
     SK_REQUIRE(m >= 1 && x_dev && y_dev && ((uintptr_t) x_dev & 15) == 0, "q4k_rows: no rows, a null pointer, or x not 16-byte aligned");
     SK_TRY(ensure_device());
     cudaStream_t s = as_stream(stream);
@@ -542,7 +542,7 @@ int32_t skainet_cuda_selftest_q4k_rows_dev(skainet_weight_t h, const float* x_de
     SK_TRY(scratch_get(s, SCRATCH_ACT, act_scratch_bytes(w->enc, SKAINET_ACT_NATIVE, m, w->cols), &scratch));
     SK_TRY(launch_act_quant(w->enc, SKAINET_ACT_NATIVE, x_dev, m, w->cols, scratch, s));
     const int32_t st = launch_gemm_tc_tiles(*w, act_q8k_layout(scratch, m, w->cols), m, y_dev, nullptr, tile, parts, s);
-    SK_REQUIRE(st != 1, "q4k_rows: no scratch or no tensor map for %d rows", m);
+    SK_REQUIRE(st != 1, "q4k_rows: no tensor map for %d rows", m);
     return st;
 }
 

@@ -84,8 +84,8 @@ void scratch_release(cudaStream_t stream);                // frees every slot of
 // Entry points that take HOST pointers stage through the default stream's scratch slots: one such call at a time per process.
 std::mutex& twin_mutex();
 enum { SCRATCH_ACT = 0, SCRATCH_ATTN = 1, SCRATCH_TWIN_A = 2, SCRATCH_TWIN_B = 3, SCRATCH_TWIN_C = 4,
-       SCRATCH_TWIN_D = 5, SCRATCH_TWIN_E = 6, SCRATCH_TWIN_F = 7, SCRATCH_FUSED = 8, SCRATCH_FUSED2 = 9, SCRATCH_GEMM = 10,
-       SCRATCH_FFN = 11, SCRATCH_SLOTS = 12 };
+       SCRATCH_TWIN_D = 5, SCRATCH_TWIN_E = 6, SCRATCH_TWIN_F = 7, SCRATCH_FUSED = 8, SCRATCH_FUSED2 = 9, SCRATCH_FFN = 10,
+       SCRATCH_SLOTS = 11 };
 
 int sm_count();
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` on the CURRENT device, once per (kernel, device):
@@ -118,8 +118,6 @@ int32_t launch_act_quant(int enc, int act_mode, const float* x, int m, int cols,
 struct ActQ8K;
 // matvec_kq.cu: Q6_K (int8-per-256 or fp32 activations) and Q5_K (fp32 activations) over resident planes
 int32_t launch_matvec_kq(const Weight& w, const float* x, ActQ8K a, int m, float* y, int act_mode, cudaStream_t s, const float* resid = nullptr);
-// gemm_kq.cu: Q6_K weights x m quantized activation rows on the tensor cores (mma.sync); 1 = not taken
-int32_t launch_gemm_q6k(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 // gemm_kq.cu: Q5_K weights x m fp32 activation rows carried as two f16 terms (hi + lo) plus per-32 sums, on the tensor cores.
 // Activation rows from which a Q5_K product takes this path (fewer rows: the row kernel of matvec_kq.cu, four per pass).
 // 11008 x 4096: 47 us here for up to 32 rows against 42 us for four rows and 83 us for eight through the row kernel.

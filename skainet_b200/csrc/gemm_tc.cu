@@ -1,34 +1,32 @@
-// Batched rows on the 5th-generation tensor cores (tcgen05.mma, accumulators and A operand in TMEM) for Q4_K weights: prompts,
-// and decode steps of many sequences.
+// Batched rows on the 5th-generation tensor cores (tcgen05.mma, accumulators and A operand in TMEM) for Q4_K and Q6_K weights: prompts,
+// and decode steps of several sequences.
 //
-// The reference's arithmetic for one 256-element super-block (native/src/q4k_matmul.c:143-251) is
-//     y += d_x * ( d_w * S1 - dmin_w * S2 ),   S1 = sum_sb sc[sb] * <codes_sb, xq_sb>,   S2 = sum_sb mn[sb] * sum(xq_sb)
-// with 4-bit codes, 6-bit sc / mn and int8 activation codes xq. Both sums are products of small integers, exact in f16 x f16 -> f32
-// as long as their sums stay below 2^24: the A operand carries code*sc (<= 945 < 2048, exact in f16), the
-// B operand the activation codes, and one super-block is 16 MMAs of K = 16 accumulated in TMEM. S2 is one
-// more K = 16 MMA of (mn[sb] twice) x (sums of 16 codes, <= 2032). |S1| can reach 945 * 127 * 256 = 1.83 * 2^24: tiles of 32 and 64 rows
-// accumulate its halves (128 products, below 2^24) apart and add them once, which gives the integer sum rounded to fp32 as the
-// mma.sync kernel has it; tiles of 128 rows have no TMEM left for that and may lose last places of sums beyond 2^24 (all codes and
-// scales near their largest and activations of one sign: error 9.1e-8 of the result instead of 5.9e-8; normal data is not affected).
-// The CUDA cores only unpack nibbles into
-// the A operand (one LOP3 + one HFMA2 per two elements, using the 0x6400|n trick: f16(1024+n)*s - 1024*s
-// is n*s exactly under the fused rounding) and apply the three fp32 block scales once per super-block.
+// The reference's arithmetic for one 256-element super-block is integer until its scales are applied:
+//     Q4_K (native/src/q4k_matmul.c:143-251)   y += d_x * (d_w * S1 - dmin_w * S2),   S1 = sum_sb sc[sb] * <codes_sb, xq_sb>,  S2 = sum_sb mn[sb] * sum(xq_sb)
+//     Q6_K (native/src/q6k_matmul.c:155-215)   y += d_w * d_x * S,                    S = sum_g sc[g] * <codes_g - 32, xq_g>
+// with int8 activation codes xq. So the main sums run on the integer MMA (kind::i8, s8 x s8 -> s32), whose B operand is the quantizer's
+// output as it lies in memory: no conversion launch, and half the bytes of 16-bit operands. A product code * scale does not fit eight
+// bits; it goes in as two planes, each a byte an element, with an accumulator each:
+//     Q4_K   code * sc = 8 * (code * (sc >> 3)) + code * (sc & 7): both at most 105, four of them by one 32-bit multiplication
+//     Q6_K   (code - 32) * sc + 4096 = 256 * h + l with h in [0, 32], l in [-128, 127]; the 4096 is taken out with the sum of the
+//            activation codes when the accumulators are read
+// The sums are exact whatever the data, and (8 or 256) * high + low, an integer, is rounded once.
+// S2 is one f16 MMA of K = 16: mins (twice) times the sums of 32 codes, each in two parts that f16 holds.
 //
-// CTA = 128 weight rows (TMEM lanes) x N activation rows (TMEM columns; N = 32, 64 or 128 by the batch). Warps:
-//   producers   a thread owns a weight row and unpacks 64-element groups of a super-block into the row's TMEM lane
-//               (tcgen05.st): sets of four warps, one set per group (N <= 64) or per two groups (N = 128, whose epilogue needs the
-//               registers). Half a super-block, two groups, is one stage: the MMAs of one half run while the other is written.
-//   epilogue    eight warps fold a finished super-block out of TMEM (tcgen05.ld), N / 2 fp32 accumulators per thread;
-//   one warp    issues the MMAs and commits; two accumulators, so the MMAs of super-block i+1 overlap the fold of i;
-//   two warps   post the copies: packed weight tiles (128 rows x 128 B, a tensor map), activation tiles (bulk).
-// Few tiles leave SMs idle, so a cluster of CTAs may share a tile by parts of the contraction; their sums meet in shared memory
-// and are added in the order of the parts, whoever finishes first.
-// The activation side is prepared once per call by act_f16_tiles_kernel in the order of the operand (K-major, 128-byte swizzle).
-// Every mbarrier wait is bounded; a wait that runs out raises the device flag, and the CTA still reaches
+// Persistent CTA of 128 weight rows (TMEM lanes) x N activation rows (TMEM columns; N = 16, 32, 64 or 128 by the batch). Warps:
+//   producers   sets of four warps, a thread a weight row; a set unpacks half a super-block (128 elements) into a slot of the A ring
+//               in TMEM (tcgen05.st), the sets taking halves in turn;
+//   epilogue    eight or sixteen warps fold finished super-blocks out of TMEM (tcgen05.ld), up to 32 fp32 accumulators a thread;
+//   one warp    issues the MMAs and commits; two accumulator sets, so the MMAs of one overlap the fold of the other: super-blocks in
+//               turn, or, at N = 128, the two halves of the columns, which share the A operand;
+//   two warps   post the copies of weight tiles and activation tiles (tensor maps, 128-byte swizzle); one prepares S2's sums and the
+//               block scales of the columns.
+// Work: whole tiles in rounds of the grid; where the tiles left over are few, a cluster of CTAs shares each by parts of the contraction (Q4_K), whose
+// sums meet in shared memory and are added in the order of the parts, whoever finishes first. (Cut into equal runs over all SMs instead, with
+// the parts through global memory and the last to come adding them, 4096 x 4096 took 13.9 us at 16 rows, against 10.0 in four parts.) Q6_K rows
+// keep the bits of the single-row kernel, whose sum runs over the blocks in order, so its tiles stay whole and are made narrower instead.
+// Every mbarrier wait is bounded; a wait that runs out raises the device flag, nothing of the tile is stored, and the CTA still reaches
 // the common exit where TMEM is freed.
-//
-// What bounds it: the chain of barrier waits between the roles (a wait on a phase that is already complete takes 60 to 120 cycles),
-// so a super-block takes few of them and large stages.
 #include "common.cuh"
 #include "actquant.cuh"
 #include "tma.cuh"
@@ -45,26 +43,55 @@ namespace sk {
 namespace {
 
 constexpr int TC_M = 128;                       // weight rows of a tile
-constexpr int TC_W_BYTES = TC_M * 128, TC_S2A_BYTES = TC_M * 32;      // codes and mins of a super-block
-constexpr int TC_EPI_WARPS = 8;
+constexpr int TC_QS_BYTES = TC_M * 128, TC_QH_BYTES = TC_M * 64, TC_S2A_BYTES = TC_M * 32;      // codes, high bits (Q6_K) and mins (Q4_K) of a super-block
+constexpr int TC_MISC_WARPS = 4, TC_AUX = 4;
 
-template <int N>
+template <int ENC, int N>
 struct TcShape {
-    static constexpr int SETS = N == 128 ? 2 : 4, PROD_WARPS = 4 * SETS, THREADS = (PROD_WARPS + TC_EPI_WARPS + 3) * 32;
-    static constexpr int WS = N == 128 ? 3 : N == 64 ? 5 : 6, BS = N == 128 ? 2 : N == 64 ? 3 : 4;      // super-blocks of weights, of activations in flight
-    static constexpr int B_BYTES = N * 512, S2B_BYTES = N * 32, SLOT = B_BYTES + S2B_BYTES;
-    static constexpr int OFF_B = WS * TC_W_BYTES, OFF_S2A = OFF_B + BS * SLOT, OFF_DX = OFF_S2A + 4 * TC_S2A_BYTES, OFF_DD = OFF_DX + 4 * N * 4;
-    static constexpr int OFF_BAR = OFF_DD + 4 * TC_M * 4, BARS = 2 * WS + 2 * BS + 4 + 4 + 4;
-    static constexpr int SMEM = OFF_BAR + BARS * 8 + 16 + 1024;             // the dynamic area is aligned to 1024 by hand
-    // TMEM columns: two sets of S1 accumulators, one for each half of a super-block where there is room, one or two of S2, four A groups of 32
-    static constexpr int S1_ACC = N == 128 ? 1 : 2, S2_SETS = N == 128 ? 1 : 2;
-    static constexpr int COL_S2 = 2 * S1_ACC * N, COL_A = COL_S2 + S2_SETS * N;
-    static_assert(COL_A + 128 <= 512, "TMEM");
-    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (TC_M >> 4) << 24);   // f16 x f16 -> f32, K-major both
+    static constexpr bool Q4 = ENC == SKAINET_ENC_Q4_K;
+    static constexpr int PROD_WARPS = 16, EPI_WARPS = 8, THREADS = (PROD_WARPS + EPI_WARPS + TC_MISC_WARPS) * 32;
+    // super-blocks of weights and of activations in flight
+    static constexpr int WS = Q4 && N < 64 ? 8 : 6, BS = 4;
+    static_assert(WS % 2 == 0, "a weight slot belongs to one pair of producer sets, which sees all its phases");
+    static constexpr int W_BYTES = TC_QS_BYTES + (Q4 ? 0 : TC_QH_BYTES), B_BYTES = N * 256, S2B_BYTES = Q4 ? N * 32 : 0;
+    static constexpr int OFF_B = WS * W_BYTES, OFF_S2A = OFF_B + BS * B_BYTES, OFF_S2B = OFF_S2A + (Q4 ? TC_AUX * TC_S2A_BYTES : 0);
+    static constexpr int OFF_DX = OFF_S2B + TC_AUX * S2B_BYTES, OFF_XS = OFF_DX + TC_AUX * N * 4, OFF_BAR = OFF_XS + (Q4 ? 0 : TC_AUX * N * 4);
+    // TMEM columns: two sets of accumulators (low plane, high plane, S2), then the A operand of RING super-blocks in halves of 64 columns
+    // (per 64 elements 16 columns of either plane)
+    static constexpr int SET = (Q4 ? 3 : 2) * N, COL_A = 2 * SET, RING = COL_A + 256 <= 512 ? 2 : 1;
+    static_assert(COL_A + RING * 128 <= 512, "TMEM");
+    static constexpr int BARS = 2 * WS + 2 * BS + 8 + 2 * TC_AUX + 4;
+    static constexpr int SMEM = OFF_BAR + BARS * 8 + 16 + 1024;         // the dynamic area is aligned to 1024 by hand
+    static_assert(SMEM <= 227 * 1024, "shared memory");
+    // registers a thread after the split; their sum over the warpgroups is that of the launch (setmaxnreg waits for ever otherwise)
+    static constexpr int R_LAUNCH = 72, R_PROD = 64, R_EPI = 104, R_MISC = 40;
+    static_assert(PROD_WARPS / 4 * R_PROD + EPI_WARPS / 4 * R_EPI + TC_MISC_WARPS / 4 * R_MISC <= THREADS / 128 * R_LAUNCH, "registers");
+    static constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (TC_M >> 4) << 24);   // s8 x s8 -> s32, K-major both
+    static constexpr uint32_t IDESC_F16 = (1u << 4) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (TC_M >> 4) << 24);                          // f16 x f16 -> f32
 };
 
-// K-major operand in the 128-byte swizzle: rows of 128 B (64 f16), groups of 8 rows 1024 B apart; a K = 16 step
-// moves the start address by 32 B inside the swizzle atom.
+// What a launch works on: tiles from `tile0` on, tile = weight tile * n_tiles + activation tile. One part: CTA c takes c, c + grid, ...; more:
+// cluster c / parts takes tile c / parts, each CTA its run of the super-blocks.
+struct TcWork {
+    int rows, bpr, n_tiles, m;
+    int tile0, tiles, grid, parts;
+};
+struct TcSeg { int tile, kb, ke; };                    // super-blocks [kb, ke) of a tile; kb == ke: there is no such segment
+__device__ __forceinline__ TcSeg tc_segment(const TcWork& w, int b, int idx) {
+    if (w.parts > 1) {
+        const int t = b / w.parts, p = b - t * w.parts;
+        return idx == 0 ? TcSeg{w.tile0 + t, w.bpr * p / w.parts, w.bpr * (p + 1) / w.parts} : TcSeg{0, 0, 0};
+    }
+    const int t = idx * w.grid + b;
+    return t < w.tiles ? TcSeg{w.tile0 + t, 0, w.bpr} : TcSeg{0, 0, 0};
+}
+__device__ __forceinline__ int tc_total(const TcWork& w, int b) {      // super-blocks of a CTA
+    if (w.parts > 1) { const TcSeg s = tc_segment(w, b, 0); return s.ke - s.kb; }
+    return b < w.tiles ? ((w.tiles - 1 - b) / w.grid + 1) * w.bpr : 0;
+}
+
+// K-major operand in the 128-byte swizzle: rows of 128 B, groups of 8 rows 1024 B apart; a K step of 32 bytes moves the start address inside
+// the swizzle atom.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     return (uint64_t) ((saddr & 0x3ffffu) >> 4) | (1ull << 16) | ((uint64_t) (1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
@@ -72,27 +99,29 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
     return (uint64_t) ((saddr & 0x3ffffu) >> 4) | ((uint64_t) (lbo_bytes >> 4) << 16) | ((uint64_t) (sbo_bytes >> 4) << 32) | (1ull << 46);
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc) : "memory");
 }
-// A operand in TMEM: lane = row, a 32-bit column holds two consecutive k
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// A operand in TMEM: lane = row, a 32-bit column holds four consecutive k
+__device__ __forceinline__ void umma_i8_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t ta, const uint32_t (&v)[32]) {
+__device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t* v) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n\t"
-        "tcgen05.wait::st.sync.aligned;"
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(ta), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
-          "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]),
-          "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+          "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t ta, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(ta), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(skd::smem_u32(bar)) : "memory");
 }
@@ -101,109 +130,143 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {      // volatile: sta
     asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
     return r;
 }
+__device__ __forceinline__ uint32_t ld_nc_u32(const void* p) { uint32_t r; asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r) : "l"(p)); return r; }
+__device__ __forceinline__ uint32_t ld_nc_u16(const void* p) { uint16_t r; asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(r) : "l"(p)); return r; }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive1(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(skd::smem_u32(bar)) : "memory");
 }
-// TMEM loads of eight columns each and the wait for them in ONE asm statement: the destination registers are only defined
-// for the compiler once the wait has been issued, so no use of them can be scheduled ahead of it.
-__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t tb, float (&u)[8], float (&v)[8]) {
-    uint32_t r[8], q[8];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
-        : "r"(ta), "r"(tb)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(q[i]); }
-}
-// the same of three places, four columns each
-__device__ __forceinline__ void tmem_ld3(uint32_t ta, uint32_t tb, uint32_t tc, float (&u)[4], float (&v)[4], float (&w)[4]) {
-    uint32_t r[12];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%12];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%13];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%14];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11])
-        : "r"(ta), "r"(tb), "r"(tc)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[4 + i]); w[i] = __uint_as_float(r[8 + i]); }
-}
-// ---- activation side: int8 codes -> f16 in core-matrix order, sums of 16 codes, transposed block scales (tile = N = 1 << nlog rows) ----
-//   xh  [m_pad/N][cols/64][N/8][8 rows][8][8]  f16: the N x 64 k pieces of a super-block are contiguous, rows of 128 B
-//                                               whose 16-byte chunks are XOR-swizzled with the row (128B swizzle);
-//                                               inside every group of four k the order is (0,2,1,3), matching the
-//                                               order in which the weight nibbles leave a 32-bit word
-//   hs  [m_pad/N][bpr][N/8][2][8 rows][8]      f16 sums of 16 consecutive codes: 32 N bytes per (tile, super-block)
-//   dxt [bpr][m_pad]                            fp32 block scales
-__global__ void __launch_bounds__(256)
-act_f16_tiles_kernel(ActQ8K act, int m, int m_pad, int cols, int nlog, __half* __restrict__ xh, __half* __restrict__ hs, float* __restrict__ dxt) {
-    skd::pdl_launch_dependents();
-    skd::pdl_wait();
-    const int per_row = cols >> 4;
-    const int64_t idx = (int64_t) blockIdx.x * 256 + threadIdx.x;
-    if (idx >= (int64_t) m_pad * per_row) return;
-    const int n = (int) (idx / per_row), seg = (int) (idx % per_row);        // 16 codes: elements 16*seg ..
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (n < m) raw = *reinterpret_cast<const uint4*>(act.q + (size_t) n * cols + (size_t) seg * 16);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    int sum = 0;
-    __half out[16];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int b0 = (int8_t) (w[j] & 0xff), b1 = (int8_t) ((w[j] >> 8) & 0xff), b2 = (int8_t) ((w[j] >> 16) & 0xff), b3 = (int8_t) (w[j] >> 24);
-        sum += b0 + b1 + b2 + b3;
-        out[4 * j] = __int2half_rn(b0); out[4 * j + 1] = __int2half_rn(b2); out[4 * j + 2] = __int2half_rn(b1); out[4 * j + 3] = __int2half_rn(b3);
+// The bounded wait of a whole warp. It asks to be put to sleep for up to TC_NAP ns a try: warps that spin take issue slots from those that
+// work (28 warps; the MMA warp's steps took twice as long).
+constexpr uint32_t TC_NAP = 1000000;
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, int* timeout_flag) {
+    uint32_t ok = 0;
+#pragma unroll 1
+    for (int i = 0; i < (1 << 12) && !ok; ++i) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(skd::smem_u32(bar)), "r"(parity), "r"(TC_NAP) : "memory");
+        ok = __all_sync(0xffffffffu, ok != 0);
     }
-    const int groups = 1 << (nlog - 3), tile = n >> nlog, ng = (n >> 3) & (groups - 1), r = n & 7;
+    if (!ok && timeout_flag) *timeout_flag = 1;
+    return ok != 0;
+}
+// Whether the phases are complete: asked together, since each answer takes 60 cycles and a warp waits for it in place.
+__device__ __forceinline__ bool mbar_test2(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+                 "and.pred p, p, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(skd::smem_u32(a)), "r"(pa), "r"(skd::smem_u32(b)), "r"(pb) : "memory");
+    return __all_sync(0xffffffffu, ok != 0);
+}
+// The same of five, the first two apart from the others: bit 0 of b to d and `a`, bit 1 of `late`. Waits in turn cost 100 to 200 cycles each,
+// complete or not.
+__device__ __forceinline__ uint32_t mbar_test5(uint64_t* a, uint64_t* late, uint32_t pa, uint64_t* b, uint32_t pb, uint64_t* c, uint32_t pc, uint64_t* d, uint32_t pd) {
+    uint32_t x, y;
+    asm volatile("{\n\t.reg .pred p, q, r, s, t;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%2], %4;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 s, [%7], %8;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 t, [%9], %10;\n\t"
+                 "and.pred p, p, r;\n\tand.pred s, s, t;\n\tand.pred p, p, s;\n\tselp.u32 %0, 1, 0, p;\n\tselp.u32 %1, 2, 0, q;\n\t}"
+                 : "=r"(x), "=r"(y)
+                 : "r"(skd::smem_u32(a)), "r"(skd::smem_u32(late)), "r"(pa), "r"(skd::smem_u32(b)), "r"(pb), "r"(skd::smem_u32(c)), "r"(pc), "r"(skd::smem_u32(d)), "r"(pd)
+                 : "memory");
+    return __reduce_and_sync(0xffffffffu, x | y);
+}
+// A value that is the same in all lanes of a warp, as one the compiler knows to be: addresses made from it stay in uniform registers. Moved
+// there anew for each MMA, they made one take 50 cycles.
+__device__ __forceinline__ uint32_t warp_value(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
+
+template <int R> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+// Eight columns out of TMEM. They are there once tmem_ld_wait() has been passed; loaded8() behind it keeps the compiler from using one earlier.
+__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(ta) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void loaded8(uint32_t (&v)[8]) {
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int kcg = seg * 2 + c, it = kcg >> 3, kc = kcg & 7;            // 8-element chunk: 64-k piece it, chunk kc of the piece
-        *reinterpret_cast<uint4*>(xh + (((((size_t) tile * (cols >> 6) + it) * groups + ng) * 8 + r) * 8 + (kc ^ r)) * 8) = *reinterpret_cast<const uint4*>(out + 8 * c);
-    }
-    const int kb = seg >> 4, j = seg & 15;
-    hs[(((((size_t) tile * (cols >> 8) + kb) * groups + ng) * 2 + (j >> 3)) * 8 + r) * 8 + (j & 7)] = __int2half_rn(sum);
-    if (j == 0) dxt[(size_t) kb * m_pad + n] = n < m ? act.d[(size_t) n * (cols >> 8) + kb] : 0.0f;
+    for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(v[i]));
 }
 
-template <int N>
-__global__ void __launch_bounds__(TcShape<N>::THREADS, 1)
-q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __restrict__ hdr, int rows, int bpr, int parts,
-                   const __half* xh, const __half* hs, const float* dxt, int m, int m_pad,
-                   float* y, const float* resid, int* __restrict__ timeout_flag) {
-    typedef TcShape<N> S;
+// A quarter of a super-block's A operand, two planes of 64 elements. Q4_K: the low nibbles of the 32 bytes are its first 32 elements, the
+// high ones the others; scw holds their two scales.
+struct TcA {
+    uint32_t lo[16], hi[16];
+};
+__device__ __forceinline__ void q4_group(const uint4 (&q)[2], uint32_t scw, TcA& o) {
+    const uint32_t s0 = scw & 7, s1 = (scw >> 3) & 7, t0 = (scw >> 8) & 7, t1 = (scw >> 11) & 7;
+    const uint32_t wv[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t x = wv[k] & 0x0f0f0f0fu, y = (wv[k] >> 4) & 0x0f0f0f0fu;
+        o.lo[k] = x * s0; o.hi[k] = x * s1; o.lo[8 + k] = y * t0; o.hi[8 + k] = y * t1;
+    }
+}
+// Four Q6_K codes of a group with scale s: (code - 32) * s + 4096 = 256 * h + l in each byte, l signed. Two products a multiplication, 4224 = 4096 + 128
+// more than they are: each 16-bit lane is at least 160 and at most 8320, so none borrows from or runs into the other, and h is its upper byte.
+__device__ __forceinline__ void q6_word(uint32_t w, int s, uint32_t& lo, uint32_t& hi) {
+    const uint32_t add = (uint32_t) (4224 - 32 * s) * 0x10001u;
+    const uint32_t e = __byte_perm(w, 0u, 0x4240) * (uint32_t) s + add, o = __byte_perm(w, 0u, 0x4341) * (uint32_t) s + add;
+    lo = __byte_perm(e, o, 0x6240) ^ 0x80808080u;
+    hi = __byte_perm(e, o, 0x7351);
+}
+// A thread's headers (d, dmin and scales of Q4_K; the sixteen scales of Q6_K) of its weight row, 16 bytes a super-block, through the CTA's segments
+struct TcHeaders {
+    const uint8_t* hrow;
+    int idx, left;                                     // segment; super-blocks of it from this one on
+};
+__device__ __forceinline__ void tc_headers_at(const TcWork& w, int b, const uint8_t* hdr, int r, TcHeaders& i, int over) {
+    const TcSeg s = tc_segment(w, b, i.idx);
+    i.left = s.ke - s.kb - over;
+    i.hrow = hdr + ((size_t) min(s.tile / w.n_tiles * TC_M + r, w.rows - 1) * w.bpr + s.kb + over) * 16;
+}
+__device__ __forceinline__ void tc_headers_next(const TcWork& w, int b, const uint8_t* hdr, int r, TcHeaders& i, int by) {
+    i.left -= by; i.hrow += by * 16;
+#pragma unroll 1
+    while (i.left <= 0) { ++i.idx; tc_headers_at(w, b, hdr, r, i, -i.left); }
+}
+
+template <int ENC, int N>
+__global__ void __launch_bounds__((TcShape<ENC, N>::THREADS), 1)
+kq_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_constant__ CUtensorMap map_qh, const __grid_constant__ CUtensorMap map_x,
+                  const uint8_t* __restrict__ hdr, const uint8_t* __restrict__ dd, const float* act_d, const int16_t* act_sums,
+                  const __grid_constant__ TcWork wk, float* y, const float* resid, int* __restrict__ timeout_flag) {
+    typedef TcShape<ENC, N> S;
+    constexpr bool Q4 = S::Q4;
     extern __shared__ uint8_t raw[];
     uint8_t* smem = raw + ((1024 - (skd::smem_u32(raw) & 1023)) & 1023);
     uint64_t* w_full = (uint64_t*) (smem + S::OFF_BAR);      // weight tile landed (bytes)
-    uint64_t* w_empty = w_full + S::WS;                      // read by all producer warps
-    uint64_t* b_full = w_empty + S::WS;                      // activation tile and its sums landed (bytes)
+    uint64_t* w_empty = w_full + S::WS;                      // read by the producers of both halves
+    uint64_t* b_full = w_empty + S::WS;                      // activation tile landed (bytes)
     uint64_t* b_empty = b_full + S::BS;                      // read by the MMAs
-    uint64_t* a_full = b_empty + S::BS;                      // half a super-block of A written, the second half with the mins
-    uint64_t* a_empty = a_full + 2;                          // read by the MMAs
-    uint64_t* s2_full = a_empty + 2;                         // scales of a super-block for the epilogue: (d, dmin) of the rows, block scales of the columns
-    uint64_t* acc_full = s2_full + 4;
-    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* a_full = b_empty + S::BS;                      // half a super-block of A written, the second with the mins: [super-block & 1][half]
+    uint64_t* a_empty = a_full + 4;                          // read by the MMAs, likewise
+    uint64_t* x_full = a_empty + 4;                          // what the columns need beside the codes
+    uint64_t* x_empty = x_full + TC_AUX;                     // folded
+    uint64_t* acc_full = x_empty + TC_AUX;
+    uint64_t* acc_empty = acc_full + 2;                      // read by the eight warps of the fold
     uint32_t* tmem_slot = (uint32_t*) (acc_empty + 2);
-    uint32_t* gave_up = tmem_slot + 1;                       // a wait of the fold ran out: this part's sums are not whole
+    uint32_t* gave_up = tmem_slot + 1;                       // a wait of the fold ran out: the sums are not whole
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int MMA_WARP = S::PROD_WARPS + TC_EPI_WARPS;
-    const int part = blockIdx.x % parts, row0 = blockIdx.x / parts * TC_M, tile_n = blockIdx.y, col0 = tile_n * N;
-    const int kb0 = (int) ((int64_t) bpr * part / parts), nk = (int) ((int64_t) bpr * (part + 1) / parts) - kb0;      // this CTA's super-blocks
+    const int tid = threadIdx.x, lane = tid & 31, cta = blockIdx.x;
+    const int warp = warp_value(tid >> 5);
+    constexpr int MMA_WARP = 0, PROD_WARP = TC_MISC_WARPS, EPI_WARP = PROD_WARP + S::PROD_WARPS;      // the warps that all wait for come first: they are the ones preferred
     skd::pdl_launch_dependents();
 
     if (warp == MMA_WARP) {
         if (lane == 0) {
-            for (int i = 0; i < S::WS; ++i) { skd::mbar_init(w_full + i, 1); skd::mbar_init(w_empty + i, S::PROD_WARPS); }
+            for (int i = 0; i < S::WS; ++i) { skd::mbar_init(w_full + i, 1); skd::mbar_init(w_empty + i, 8); }
             for (int i = 0; i < S::BS; ++i) { skd::mbar_init(b_full + i, 1); skd::mbar_init(b_empty + i, 1); }
-            for (int i = 0; i < 2; ++i) { skd::mbar_init(a_full + i, 8); skd::mbar_init(a_empty + i, 1); skd::mbar_init(acc_full + i, 1); skd::mbar_init(acc_empty + i, TC_EPI_WARPS); }
-            for (int i = 0; i < 4; ++i) skd::mbar_init(s2_full + i, 8);
+            for (int i = 0; i < 4; ++i) { skd::mbar_init(a_full + i, 4); skd::mbar_init(a_empty + i, 1); }
+            for (int i = 0; i < TC_AUX; ++i) { skd::mbar_init(x_full + i, 1); skd::mbar_init(x_empty + i, S::EPI_WARPS); }
+            for (int i = 0; i < 2; ++i) { skd::mbar_init(acc_full + i, 1); skd::mbar_init(acc_empty + i, 8); }
             skd::mbar_fence_init();
             *gave_up = 0;
         }
@@ -214,245 +277,394 @@ q4k_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const uint8_t* __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_value(*tmem_slot);
 
-    if (warp == MMA_WARP) {
-        // ------------------------------------------------ MMA issuer ------------------------------------------------
-        const uint64_t d_b = smem_desc_sw128(skd::smem_u32(smem + S::OFF_B));
-        int s = 0, round = 0;
-        for (int i = 0; i < nk; ++i) {
-            const int set = i & 1;
-            if (i >= 2 && !skd::mbar_wait_warp(acc_empty + set, ((i >> 1) - 1) & 1, timeout_flag)) break;
-            if (!skd::mbar_wait_warp(b_full + s, round & 1, timeout_flag)) break;
-            bool ok = true;
+    if (warp < PROD_WARP) {
+        regs_down<S::R_MISC>();
+        if (warp == MMA_WARP) {
+            // ------------------------------------------------ MMA issuer ------------------------------------------------
+            const uint64_t d_b = smem_desc_sw128(skd::smem_u32(smem + S::OFF_B));
+            const uint32_t a2 = skd::smem_u32(smem + S::OFF_S2A), b2_at = skd::smem_u32(smem + S::OFF_S2B);
+            const int total = tc_total(wk, cta);
+            int s = 0, b_par = 0;                                  // activation slot and its round
+            auto mmas = [&](uint32_t acc, uint32_t ta, uint64_t db, bool first) {      // half a super-block
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (!(ok = skd::mbar_wait_warp(a_full + h, i & 1, timeout_flag))) break;
-                // the one S2 accumulator: super-block i - 1 has been folded
-                if (S::S2_SETS == 1 && h == 1 && i >= 1 && !(ok = skd::mbar_wait_warp(acc_empty + (set ^ 1), ((i - 1) >> 1) & 1, timeout_flag))) break;
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) umma_i8_ta(acc + p * N, ta + (j >> 1) * 32 + p * 16 + (j & 1) * 8, db + (uint64_t) (j * 2), S::IDESC_I8, first ? j : 1);
+            };
+#pragma unroll 1
+            for (int it = 0; it < total; ++it) {
+                const int sx = it & (TC_AUX - 1), x_par = (it / TC_AUX) & 1, odd = it & 1, par = (it >> 1) & 1;
+                uint64_t *const af = a_full + 2 * odd, *const ae = a_empty + 2 * odd, *const ac = acc_empty + odd;
+                // (Q6_K's columns need nothing more before the fold)
+                uint64_t* const x_or_b = Q4 ? x_full + sx : b_full + s;
+                const uint32_t x_or_b_par = Q4 ? x_par : b_par;
+                // The accumulators are free once the super-block before the last has been folded; the first two find them free: the parity before
+                // the first phase reads as complete. One warp may ask again and again.
+                uint32_t ready = 0;
+#pragma unroll 1
+                for (int i = 0; i < (1 << 24) && !(ready & 1); ++i) ready = mbar_test5(af, af + 1, par, b_full + s, b_par, x_or_b, x_or_b_par, ac, par ^ 1);
+                if (!(ready & 1)) { if (timeout_flag) *timeout_flag = 1; break; }
                 tc_fence_after();
-                if (skd::elect_one()) {
-                    // descriptors move in 16-byte units: a 64-k piece is 128 N bytes, a K = 16 step 32 bytes
-                    const uint64_t db = d_b + (uint64_t) ((s * S::SLOT + h * (S::B_BYTES / 2)) >> 4);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        umma_f16_ta(tmem + (set * S::S1_ACC + (S::S1_ACC == 2 ? h : 0)) * N, tmem + S::COL_A + h * 64 + j * 8, db + (uint64_t) (((j >> 2) * (S::B_BYTES / 4) + (j & 3) * 32) >> 4),
-                                    S::IDESC, (S::S1_ACC == 2 ? j : h | j) != 0 ? 1u : 0u);
-                    umma_commit(a_empty + h);
-                    if (h == 1) {
-                        const uint32_t a2 = skd::smem_u32(smem + S::OFF_S2A + (i & 3) * TC_S2A_BYTES), b2 = skd::smem_u32(smem + S::OFF_B + s * S::SLOT + S::B_BYTES);
-                        umma_f16(tmem + S::COL_S2 + (S::S2_SETS == 2 ? set * N : 0), smem_desc(a2, 128, 256), smem_desc(b2, 128, 256), S::IDESC, 0u);
-                        umma_commit(b_empty + s);
-                        umma_commit(acc_full + set);
-                    }
+                // descriptors move in 16-byte units: half a super-block of the tile is 128 N bytes, a K step 32 bytes
+                const uint64_t db = d_b + (uint64_t) ((s * S::B_BYTES) >> 4);
+                const uint32_t acc = tmem + odd * S::SET, ta = tmem + S::COL_A + (S::RING == 2 ? odd : 0) * 128;
+                if (!(ready & 2)) {
+                    if (skd::elect_one()) { mmas(acc, ta, db, true); umma_commit(ae); }
+                    __syncwarp();
+                    if (!mbar_wait_all(af + 1, par, timeout_flag)) break;
+                    tc_fence_after();
+                }
+                if (skd::elect_one()) {                            // all at once where it can be: every such block costs 200 cycles beside its instructions
+                    if (ready & 2) { mmas(acc, ta, db, true); umma_commit(ae); }
+                    mmas(acc, ta + 64, db + (uint64_t) (N * 128 >> 4), false);
+                    if (Q4) umma_f16(acc + 2 * N, smem_desc(a2 + sx * TC_S2A_BYTES, 128, 256), smem_desc(b2_at + sx * S::S2B_BYTES, 128, 256), S::IDESC_F16);
+                    umma_commit(ae + 1);
+                    umma_commit(b_empty + s);
+                    umma_commit(acc_full + odd);
                 }
                 __syncwarp();
+                if (++s == S::BS) { s = 0; b_par ^= 1; }
             }
-            if (!ok) break;
-            if (++s == S::BS) { s = 0; ++round; }
-        }
-    } else if (warp == MMA_WARP + 1) {
-        // ---------------------------------------- copies of weight tiles ----------------------------------------
-        bool ok = true;
-        for (int i = 0; i < nk; ++i) {
-            const int s = i % S::WS;
-            if (i >= S::WS && !(ok = skd::mbar_wait_warp(w_empty + s, (i / S::WS - 1) & 1, timeout_flag))) break;
-            if (skd::elect_one()) {
-                skd::mbar_expect_tx(w_full + s, TC_W_BYTES);
-                skd::tma_load_2d(smem + s * TC_W_BYTES, &map_qs, (kb0 + i) * 128, row0, w_full + s);
-            }
-            __syncwarp();
-        }
-        if (!ok)                                       // give copies in flight time to land before the CTA leaves
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    } else if (warp == MMA_WARP + 2) {
-        // ---------------------------------------- copies of activation tiles ----------------------------------------
-        skd::pdl_wait();                               // the activation side is the predecessor's output
-        bool ok = true;
-        int s = 0, round = 0;
-        for (int i = 0; i < nk; ++i) {
-            if (round > 0 && !(ok = skd::mbar_wait_warp(b_empty + s, (round - 1) & 1, timeout_flag))) break;
-            if (skd::elect_one()) {
-                const size_t blk = (size_t) tile_n * bpr + kb0 + i;
-                skd::mbar_expect_tx(b_full + s, S::SLOT);
-                skd::bulk_g2s(smem + S::OFF_B + s * S::SLOT, xh + blk * (S::B_BYTES / 2), S::B_BYTES, b_full + s);
-                skd::bulk_g2s(smem + S::OFF_B + s * S::SLOT + S::B_BYTES, hs + blk * (S::S2B_BYTES / 2), S::S2B_BYTES, b_full + s);
-            }
-            __syncwarp();
-            if (++s == S::BS) { s = 0; ++round; }
-        }
-        if (!ok)
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    } else if (warp < S::PROD_WARPS) {
-        // ------------------------------------------- producers of the A operand -------------------------------------------
-        constexpr int PER = 4 / S::SETS;                // groups a set unpacks: its number, and two further where it takes two
-        const int r = tid & 127, my = warp >> 2;        // weight row of the tile = TMEM lane (warp % 4 is its 32-lane quarter); set
-        const bool writes_mins = my == S::SETS - 1;     // the set whose last group is the super-block's last; set 0 writes the columns' block scales
-        const uint32_t a_lane = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + S::COL_A;
-        // headers straight from global memory, two super-blocks ahead (a tensor copy of 16-byte rows is no faster)
-        const uint8_t* hrow = hdr + ((size_t) min(row0 + r, rows - 1) * bpr + kb0) * 16;
-        uint4 hd1 = ld_nc_v4(hrow), hd2 = ld_nc_v4(hrow + (nk > 1 ? 16 : 0));
-        float dx = 0.0f;
-        for (int i = 0; i < nk; ++i) {
-            const int s = i % S::WS;
-            const uint4 hd = hd1;
-            hd1 = hd2;
-            if (i + 2 < nk) hd2 = ld_nc_v4(hrow + (size_t) (i + 2) * 16);
-            if (!skd::mbar_wait_warp(w_full + s, (i / S::WS) & 1, timeout_flag)) break;
-            const uint8_t* wrow = smem + s * TC_W_BYTES + r * 128;
-            uint4 q[PER][2];
-#pragma unroll
-            for (int e = 0; e < PER; ++e)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) q[e][c] = skd::lds128(wrow + (((2 * (my + 2 * e) + c) ^ (r & 7)) << 4));
-            uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
-            skd::k4_unpack(hd.y, hd.z, hd.w, sc_lo, sc_hi, mn_lo, mn_hi);
+        } else if (warp == MMA_WARP + 1) {
+            // ---------------------------------------- copies of weight tiles ----------------------------------------
             bool ok = true;
-#pragma unroll
-            for (int e = 0; e < PER; ++e) {
-                const int st = my + 2 * e, h = st >> 1;          // k 0..31 of the group = low nibbles x sc[2 st], k 32..63 = high nibbles x sc[2 st + 1]
-                // high nibbles stay in place (f16 1024 + 16 n) and take scale / 16, so only the odd bytes need a shift
-                const uint32_t scw = (h ? sc_hi : sc_lo) >> (16 * (st & 1));
-                const __half2 ml = __half2half2(__int2half_rn((int) (scw & 0xff))), mh = __half2half2(__hmul(__int2half_rn((int) ((scw >> 8) & 0xff)), __float2half_rn(0.0625f)));
-                const __half2 nl = __hmul2(ml, __float2half2_rn(-1024.0f)), nh = __hmul2(mh, __float2half2_rn(-1024.0f));
-                const uint32_t wv[8] = {q[e][0].x, q[e][0].y, q[e][0].z, q[e][0].w, q[e][1].x, q[e][1].y, q[e][1].z, q[e][1].w};
-                uint32_t out[32];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t w = wv[k], w8 = w >> 8;
-                    const uint32_t x02 = (w & 0x000f000fu) | 0x64006400u, x13 = (w8 & 0x000f000fu) | 0x64006400u;
-                    const uint32_t y02 = (w & 0x00f000f0u) | 0x64006400u, y13 = (w8 & 0x00f000f0u) | 0x64006400u;
-                    __half2 v;
-                    v = __hfma2(*reinterpret_cast<const __half2*>(&x02), ml, nl); out[2 * k] = *reinterpret_cast<uint32_t*>(&v);
-                    v = __hfma2(*reinterpret_cast<const __half2*>(&x13), ml, nl); out[2 * k + 1] = *reinterpret_cast<uint32_t*>(&v);
-                    v = __hfma2(*reinterpret_cast<const __half2*>(&y02), mh, nh); out[16 + 2 * k] = *reinterpret_cast<uint32_t*>(&v);
-                    v = __hfma2(*reinterpret_cast<const __half2*>(&y13), mh, nh); out[16 + 2 * k + 1] = *reinterpret_cast<uint32_t*>(&v);
+            int s = 0, par = 1;                                    // the first round finds the slots empty
+            bool first = true;
+            for (int idx = 0; ok; ++idx) {
+                const TcSeg sg = tc_segment(wk, cta, idx);
+                if (sg.kb >= sg.ke) break;
+                const int row0 = sg.tile / wk.n_tiles * TC_M;
+                for (int kb = sg.kb; kb < sg.ke; ++kb) {
+                    if (!first && !(ok = mbar_wait_all(w_empty + s, par, timeout_flag))) break;
+                    if (skd::elect_one()) {
+                        skd::mbar_expect_tx(w_full + s, S::W_BYTES);
+                        skd::tma_load_2d(smem + s * S::W_BYTES, &map_qs, kb * 128, row0, w_full + s);
+                        if (!Q4) skd::tma_load_2d(smem + s * S::W_BYTES + TC_QS_BYTES, &map_qh, kb * 64, row0, w_full + s);
+                    }
+                    __syncwarp();
+                    if (++s == S::WS) { s = 0; par ^= 1; first = false; }
                 }
-                if (i >= 1 && !(ok = skd::mbar_wait_warp(a_empty + h, (i - 1) & 1, timeout_flag))) break;
-                tc_fence_after();
-                tmem_st32(a_lane + st * 32, out);
-                // Scales and mins go to one of four slots. The slot's last use was super-block i - 4, folded before the MMAs of i - 2 were
-                // issued, and the wait above has seen MMAs of i - 1 complete.
-                if (writes_mins && e == PER - 1) {
-                    uint8_t* s2 = smem + S::OFF_S2A + (i & 3) * TC_S2A_BYTES + (r >> 3) * 256 + (r & 7) * 16;
+            }
+            if (!ok)                                       // give copies in flight time to land before the CTA leaves
+                for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        } else if (warp == MMA_WARP + 2) {
+            // ---------------------------------------- copies of activation tiles ----------------------------------------
+            skd::pdl_wait();                               // the activation side is the predecessor's output
+            bool ok = true, first = true;
+            int s = 0, par = 1;
+            for (int idx = 0; ok; ++idx) {
+                const TcSeg sg = tc_segment(wk, cta, idx);
+                if (sg.kb >= sg.ke) break;
+                const int col0 = sg.tile % wk.n_tiles * N;
+                for (int kb = sg.kb; kb < sg.ke; ++kb) {
+                    if (!first && !(ok = mbar_wait_all(b_empty + s, par, timeout_flag))) break;
+                    if (skd::elect_one()) {                // rows past the batch read as zeros
+                        skd::mbar_expect_tx(b_full + s, S::B_BYTES);
+                        skd::tma_load_2d(smem + S::OFF_B + s * S::B_BYTES, &map_x, kb * 256, col0, b_full + s);
+                        skd::tma_load_2d(smem + S::OFF_B + s * S::B_BYTES + N * 128, &map_x, kb * 256 + 128, col0, b_full + s);
+                    }
+                    __syncwarp();
+                    if (++s == S::BS) { s = 0; par ^= 1; first = false; }
+                }
+            }
+            if (!ok)
+                for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        } else {
+            // ------------------------- sums of the activation codes and block scales of the columns -------------------------
+            skd::pdl_wait();
+            constexpr int PER = (N + 31) / 32;             // columns a lane
+            bool ok = true;
+            int it = 0;
+            for (int idx = 0; ok; ++idx) {
+                const TcSeg sg = tc_segment(wk, cta, idx);
+                if (sg.kb >= sg.ke) break;
+                const int col0 = sg.tile % wk.n_tiles * N;
+                uint4 sums[PER];
+                float dx[PER];
+                auto fetch = [&](int q, int kb) {
+                    const int col = col0 + lane + 32 * q;
+                    sums[q] = make_uint4(0, 0, 0, 0); dx[q] = 0.0f;
+                    if (lane + 32 * q < N && col < wk.m) {
+                        sums[q] = skd::ld_dep(reinterpret_cast<const uint4*>(act_sums + ((size_t) col * wk.bpr + kb) * 8));
+                        dx[q] = skd::ld_dep(act_d + (size_t) col * wk.bpr + kb);
+                    }
+                };
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {       // mins, each twice, against the sums of 16 codes
-                        const uint32_t mnw = c ? mn_hi : mn_lo;
-                        uint32_t mm[4];
+                for (int q = 0; q < PER; ++q) fetch(q, sg.kb);
+                for (int kb = sg.kb; kb < sg.ke; ++kb, ++it) {
+                    const int s = it & 3;
+                    if (it >= TC_AUX && !(ok = mbar_wait_all(x_empty + s, ((it >> 2) - 1) & 1, timeout_flag))) break;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const __half2 vv = __half2half2(__int2half_rn((int) ((mnw >> (8 * j)) & 0xff)));
-                            mm[j] = *reinterpret_cast<const uint32_t*>(&vv);
+                    for (int q = 0; q < PER; ++q) {
+                        const int c = lane + 32 * q;
+                        const uint4 cs = sums[q];
+                        const float cd = dx[q];
+                        if (kb + 1 < sg.ke) fetch(q, kb + 1);
+                        if (c >= N) continue;
+                        const uint32_t w[4] = {cs.x, cs.y, cs.z, cs.w};
+                        if (Q4) {
+                            // a sum v in [-4064, 4064] as (64 t - 4096) + l with 4096 + v = 64 t + l, two at a time: f16 holds both parts
+                            uint32_t hi[4], lo[4];
+                            const __half2 k68 = __float2half2_rn(-68.0f), k1024 = __float2half2_rn(1024.0f), n1024 = __float2half2_rn(-1024.0f);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const uint32_t v = __vadd2(w[j], 0x10001000u), t = ((v >> 6) & 0x00ff00ffu) | 0x54005400u, l = (v & 0x003f003fu) | 0x64006400u;
+                                const __half2 h = __hmul2(__hadd2(*reinterpret_cast<const __half2*>(&t), k68), k1024), g = __hadd2(*reinterpret_cast<const __half2*>(&l), n1024);
+                                hi[j] = *reinterpret_cast<const uint32_t*>(&h); lo[j] = *reinterpret_cast<const uint32_t*>(&g);
+                            }
+                            uint8_t* at = smem + S::OFF_S2B + s * S::S2B_BYTES + (c >> 3) * 256 + (c & 7) * 16;
+                            *reinterpret_cast<uint4*>(at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                            *reinterpret_cast<uint4*>(at + 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        } else {
+                            int v = 0;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v += (int) (int16_t) (w[j] & 0xffff) + ((int) w[j] >> 16);
+                            *reinterpret_cast<int*>(smem + S::OFF_XS + (s * N + c) * 4) = -4096 * v;
                         }
-                        *reinterpret_cast<uint4*>(s2 + c * 128) = make_uint4(mm[0], mm[1], mm[2], mm[3]);
+                        *reinterpret_cast<float*>(smem + S::OFF_DX + (s * N + c) * 4) = cd;
                     }
-                    *reinterpret_cast<uint32_t*>(smem + S::OFF_DD + ((i & 3) * TC_M + r) * 4) = hd.x;
-                    fence_async_smem();
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive1(a_full + h);
-                    // The weight slot goes back only now that what was read from it lies in TMEM. Given back right behind the reads, the next
-                    // tile could overtake them: at 32 and 64 rows of 11008 x 4096 up to 15 of 100 queued calls had a warp's 32 rows of a
-                    // group from the super-block WS further on.
-                    if (e == PER - 1) mbar_arrive1(w_empty + s);
-                    if (writes_mins && e == PER - 1) mbar_arrive1(s2_full + (i & 3));
+                    if (Q4) fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive1(x_full + s);
                 }
             }
-            if (!ok) break;
-            if (my == 0) {
-                if (i == 0) { skd::pdl_wait(); if (r < N) dx = __ldcg(dxt + (size_t) kb0 * m_pad + col0 + r); }
-                if (r < N) *reinterpret_cast<float*>(smem + S::OFF_DX + ((i & 3) * N + r) * 4) = dx;
-                if (r < N && i + 1 < nk) dx = __ldcg(dxt + (size_t) (kb0 + i + 1) * m_pad + col0 + r);
-                __syncwarp();
-                if (lane == 0) mbar_arrive1(s2_full + (i & 3));
+        }
+    } else if (warp < EPI_WARP) {
+        // ------------------------------------------- producers of the A operand -------------------------------------------
+        regs_down<S::R_PROD>();
+        // weight row of the tile = TMEM lane (warp % 4 is its 32-lane quarter); the set unpacks half h of the even or odd super-blocks
+        const int r = tid & 127, h = ((warp - PROD_WARP) >> 2) & 1, odd = (warp - PROD_WARP) >> 3;
+        const uint32_t a_lane = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + S::COL_A + (S::RING == 2 ? odd : 0) * 128 + h * 64;
+        uint64_t *const af = a_full + 2 * odd + h, *const ae = a_empty + 2 * (S::RING == 2 ? odd : odd ^ 1) + h;      // the slot's last reader: RING super-blocks back
+        const int total = tc_total(wk, cta), r7 = r & 7;
+        TcHeaders ahead = {};
+        // headers straight from global memory, one of the set's super-blocks ahead
+        uint4 next = make_uint4(0, 0, 0, 0);
+        if (odd < total) {
+            tc_headers_at(wk, cta, hdr, r, ahead, 0);
+            tc_headers_next(wk, cta, hdr, r, ahead, odd);
+            const uint8_t* hrow = ahead.hrow;
+            next = ld_nc_v4(hrow);
+        }
+        int s = odd, w_par = 0;                                    // weight slot and its round
+        uint32_t a_par = S::RING == 2 || odd == 0 ? 1 : 0;         // the first RING super-blocks find the slots free
+#pragma unroll 1
+        for (int it = odd; it < total; it += 2) {
+            const uint4 hd = next;
+            if (it + 2 < total) {
+                tc_headers_next(wk, cta, hdr, r, ahead, 2);
+                const uint8_t* hrow = ahead.hrow;
+                next = ld_nc_v4(hrow);
             }
+            if (!mbar_wait_all(w_full + s, w_par, timeout_flag)) break;
+            const uint8_t* wt = smem + s * S::W_BYTES;
+            uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
+            if (Q4) skd::k4_unpack(hd.y, hd.z, hd.w, sc_lo, sc_hi, mn_lo, mn_hi);
+            const uint32_t sc4 = h ? sc_hi : sc_lo;
+            TcA o;
+            auto unpack = [&](int e) {                             // 64 elements
+                if constexpr (Q4) {
+                    const uint4 c[2] = {skd::lds128(wt + r * 128 + (((4 * h + 2 * e) ^ r7) << 4)), skd::lds128(wt + r * 128 + (((4 * h + 2 * e + 1) ^ r7) << 4))};
+                    q4_group(c, sc4 >> (16 * e), o);
+                } else {
+                    // 64 bytes of low nibbles (e = 0) or high ones, two bits of the half's 32 bytes of high bits
+                    const uint32_t scw = e ? (h ? hd.w : hd.y) : (h ? hd.z : hd.x);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {                  // sixteen bytes of each
+                        const int off = r * 64 + (2 * h + c) * 16;         // rows of 64 bytes in the 64-byte swizzle
+                        const uint4 hv = skd::lds128(wt + TC_QS_BYTES + (off ^ ((off >> 3) & 0x30)));
+                        const uint32_t h4[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            const uint4 lv = skd::lds128(wt + r * 128 + (((4 * h + 2 * q + c) ^ r7) << 4));
+                            const uint32_t l4[4] = {lv.x, lv.y, lv.z, lv.w};
+                            const int sc = (int) (int8_t) (scw >> (16 * q + 8 * c));
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                q6_word(((e ? l4[k] >> 4 : l4[k]) & 0x0f0f0f0fu) | ((e ? (q ? h4[k] >> 2 : h4[k]) : (q ? h4[k] << 2 : h4[k] << 4)) & 0x30303030u), sc, o.lo[8 * q + 4 * c + k], o.hi[8 * q + 4 * c + k]);
+                        }
+                    }
+                }
+            };
+            unpack(0);
+            // Mins go to one of four slots. Its last use was super-block it - 4: the wait for A at it - 2 was for the MMAs of it - 3 or it - 4.
+            if (Q4 && h == 1) {
+                uint32_t mm[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {                      // 1024 + n in f16, less 1024
+                    const uint32_t v = __byte_perm(j < 2 ? mn_lo : mn_hi, 0u, (j & 1) ? 0x4342 : 0x4140) | 0x64006400u;
+                    const __half2 f = __hadd2(*reinterpret_cast<const __half2*>(&v), __float2half2_rn(-1024.0f));
+                    mm[j] = *reinterpret_cast<const uint32_t*>(&f);
+                }
+                uint8_t* s2 = smem + S::OFF_S2A + (it & 3) * TC_S2A_BYTES + (r >> 3) * 256 + r7 * 16;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) *reinterpret_cast<uint4*>(s2 + c * 128) = make_uint4(mm[0], mm[1], mm[2], mm[3]);
+                fence_async_smem();
+            }
+            if (!mbar_wait_all(ae, a_par, timeout_flag)) break;
+            a_par ^= 1;
+            tc_fence_after();
+            tmem_st16(a_lane, o.lo); tmem_st16(a_lane + 16, o.hi);
+            unpack(1);
+            tmem_st16(a_lane + 32, o.lo); tmem_st16(a_lane + 48, o.hi);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive1(af);
+                // The weight slot goes back only now that what was read from it lies in TMEM: given back right behind the reads, the next tile
+                // could overtake them.
+                mbar_arrive1(w_empty + s);
+            }
+            if ((s += 2) >= S::WS) { s -= S::WS; w_par ^= 1; }
         }
     } else {
         // ------------------------------- epilogue: fold every super-block out of TMEM -------------------------------
-        const int r = tid & 127, ch = (warp - S::PROD_WARPS) >> 2;      // TMEM lane = weight row; which half of the columns
-        constexpr int NC = N / 2, LD = S::S1_ACC == 2 ? 4 : 8;          // columns a load: what the registers take (eight are no faster at N = 32)
-        uint64_t yacc[NC / 2];
-#pragma unroll
-        for (int c = 0; c < NC / 2; ++c) yacc[c] = 0;
+        regs_up<S::R_EPI>();
+        // TMEM lane = weight row; which half of an accumulator's columns
+        const int r = tid & 127, ch = (warp - EPI_WARP) >> 2;
+        constexpr int NC = N / 2, LD = 8;                          // columns of a thread, columns of a load
+        const int c0 = ch * NC;
+        const uint32_t t_lane = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + c0;
+        skd::pdl_wait();                                   // y, resid and the scratch may still be in use by kernels launched before this one
         bool ok = true;
-        for (int i = 0; i < nk; ++i) {
-            const int set = i & 1;
-            // the second long complete; observed for what it guards
-            if (!(ok = skd::mbar_wait_warp(acc_full + set, (i >> 1) & 1, timeout_flag) && skd::mbar_wait_warp(s2_full + (i & 3), (i >> 2) & 1, timeout_flag))) { *gave_up = 1; break; }
-            tc_fence_after();
-            const uint32_t dd = *reinterpret_cast<const uint32_t*>(smem + S::OFF_DD + ((i & 3) * TC_M + r) * 4);
-            const float dw = __half2float(__ushort_as_half((unsigned short) (dd & 0xffff))), dminw = __half2float(__ushort_as_half((unsigned short) (dd >> 16)));
-            const uint64_t dw2 = skd::pk2(dw, dw), nd2 = skd::pk2(-dminw, -dminw);
-            const float* dx = (const float*) (smem + S::OFF_DX) + (i & 3) * N + ch * NC;
-            const uint32_t t0 = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + ch * NC, t2 = t0 + S::COL_S2 + (S::S2_SETS == 2 ? set * N : 0);
+        int it = 0;
+        for (int idx = 0;; ++idx) {
+            const TcSeg sg = tc_segment(wk, cta, idx);
+            if (sg.kb >= sg.ke) break;
+            const int row = sg.tile / wk.n_tiles * TC_M + r, col0 = sg.tile % wk.n_tiles * N, valid = wk.m - col0;      // columns of the tile within the batch
+            const size_t blk = (size_t) min(row, wk.rows - 1) * wk.bpr;
+            uint64_t yacc[NC / 2];
 #pragma unroll
-            for (int c = 0; c < NC; c += LD) {
-                float s1[LD], s2[LD], s1b[LD];
-                if constexpr (S::S1_ACC == 2) tmem_ld3(t0 + 2 * set * N + c, t0 + (2 * set + 1) * N + c, t2 + c, s1, s1b, s2);
-                else tmem_ld8(t0 + set * N + c, t2 + c, s1, s2);
-                if (c + LD == NC) {                    // all accumulators have been read
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive1(acc_empty + set);
+            for (int c = 0; c < NC / 2; ++c) yacc[c] = 0;
+            uint32_t d_next = Q4 ? ld_nc_u32(hdr + (blk + sg.kb) * 16) : ld_nc_u16(dd + (blk + sg.kb) * 2);
+            for (int kb = sg.kb; ok && kb < sg.ke; ++kb, ++it) {
+                const uint32_t dv = d_next;
+                if (kb + 1 < sg.ke) d_next = Q4 ? ld_nc_u32(hdr + (blk + kb + 1) * 16) : ld_nc_u16(dd + (blk + kb + 1) * 2);
+                const float dw = __half2float(__ushort_as_half((unsigned short) (dv & 0xffff))), dminw = __half2float(__ushort_as_half((unsigned short) (dv >> 16)));
+                const uint64_t dw2 = skd::pk2(dw, dw), nd2 = skd::pk2(-dminw, -dminw);
+                const int sx = it & 3;
+                const int odd = it & 1, par = (it >> 1) & 1;
+                if (!mbar_test2(acc_full + odd, par, x_full + sx, (it >> 2) & 1)) {
+                    ok = mbar_wait_all(acc_full + odd, par, timeout_flag) && mbar_wait_all(x_full + sx, (it >> 2) & 1, timeout_flag);
+                    if (!ok) { *gave_up = 1; break; }
                 }
+                tc_fence_after();
+                const uint32_t t0 = t_lane + odd * S::SET;
+                const float* dx = (const float*) (smem + S::OFF_DX) + sx * N + c0;
+                const int* xs = (const int*) (smem + S::OFF_XS) + sx * N + c0;
+                if (c0 < valid) {                          // nothing is stored of columns past the batch
 #pragma unroll
-                for (int j = 0; j < LD; j += 2) {
-                    const float2 x2 = *reinterpret_cast<const float2*>(dx + c + j);
-                    uint64_t sum = skd::pk2(s1[j], s1[j + 1]);
-                    if (S::S1_ACC == 2) sum = skd::add2(sum, skd::pk2(s1b[j], s1b[j + 1]));
-                    uint64_t& y2 = yacc[(c + j) / 2];
-                    y2 = skd::fma2(skd::pk2(x2.x, x2.y), skd::fma2(dw2, sum, skd::mul2(nd2, skd::pk2(s2[j], s2[j + 1]))), y2);
+                    for (int c = 0; c < NC; c += LD) {
+                        uint32_t lo[LD], hi[LD], s2[LD];
+                        tmem_ld8(t0 + c, lo); tmem_ld8(t0 + N + c, hi);
+                        if (Q4) tmem_ld8(t0 + 2 * N + c, s2);
+                        tmem_ld_wait();
+                        loaded8(lo); loaded8(hi);
+                        if (Q4) loaded8(s2);
+#pragma unroll
+                        for (int j = 0; j < LD; j += 4) {
+                            const float4 x4 = *reinterpret_cast<const float4*>(dx + c + j);
+                            int4 z4 = make_int4(0, 0, 0, 0);
+                            if (!Q4) z4 = *reinterpret_cast<const int4*>(xs + c + j);
+#pragma unroll
+                            for (int f = 0; f < 4; f += 2) {
+                                uint64_t& y2 = yacc[(c + j + f) / 2];
+                                const uint64_t x2 = f ? skd::pk2(x4.z, x4.w) : skd::pk2(x4.x, x4.y);
+                                const int k = j + f;
+                                if constexpr (Q4) {
+                                    const uint64_t sum = skd::pk2((float) (int) (hi[k] * 8 + lo[k]), (float) (int) (hi[k + 1] * 8 + lo[k + 1]));
+                                    y2 = skd::fma2(x2, skd::fma2(dw2, sum, skd::mul2(nd2, skd::pk2(__uint_as_float(s2[k]), __uint_as_float(s2[k + 1])))), y2);
+                                } else {                   // in the order and with the roundings of the single-row kernel (a packed product and sum would be contracted)
+                                    const float a0 = (float) ((int) (hi[k] * 256 + lo[k]) + (f ? z4.z : z4.x)), a1 = (float) ((int) (hi[k + 1] * 256 + lo[k + 1]) + (f ? z4.w : z4.y));
+                                    y2 = skd::add2(y2, skd::pk2(__fmul_rn(__fmul_rn(dw, f ? x4.z : x4.x), a0), __fmul_rn(__fmul_rn(dw, f ? x4.w : x4.y), a1)));
+                                }
+                            }
+                        }
+                    }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) { mbar_arrive1(acc_empty + odd); mbar_arrive1(x_empty + sx); }
             }
-        }
-        if (parts > 1) {
-            // this part's sums into shared memory, [column][row], where the activation tiles were (all MMAs have read them)
-            float* mine = (float*) (smem + S::OFF_B) + (ch * NC) * TC_M + r;
-#pragma unroll
-            for (int c = 0; c < NC / 2; ++c) {
-                const float2 v = skd::up2(yacc[c]);
-                mine[(2 * c) * TC_M] = v.x; mine[(2 * c + 1) * TC_M] = v.y;
-            }
-        } else {
-            skd::pdl_wait();                           // y and resid may still be in use by kernels launched before this one
-            if (ok && row0 + r < rows) {
+            if (Q4 && wk.parts > 1) {
+                // this part's sums into shared memory, [column][row], where the activation tiles were (all MMAs have read them)
+                float* mine = (float*) (smem + S::OFF_B) + c0 * TC_M + r;
 #pragma unroll
                 for (int c = 0; c < NC / 2; ++c) {
                     const float2 v = skd::up2(yacc[c]);
-                    const int col = col0 + ch * NC + 2 * c;
-                    const size_t o = (size_t) col * rows + row0 + r;
-                    if (col < m) y[o] = resid ? resid[o] + v.x : v.x;
-                    if (col + 1 < m) y[o + rows] = resid ? resid[o + rows] + v.y : v.y;
+                    mine[2 * c * TC_M] = v.x; mine[(2 * c + 1) * TC_M] = v.y;
+                }
+                __syncwarp();
+                skd::cluster_sync_all();                   // every part's sums are in place
+                // one flag a lane: read in turn they cost 0.4 us a call of four parts
+                const bool whole = !__any_sync(0xffffffffu, lane < wk.parts && skd::ld_cluster(skd::smem_u32(gave_up), lane) != 0.0f);
+                const uint32_t base = skd::smem_u32(smem + S::OFF_B);
+                const int part = cta % wk.parts, per = (N * TC_M / 4 + wk.parts - 1) / wk.parts * 4, e0 = part * per, e1 = min(N * TC_M, e0 + per), row0 = row - r;
+#pragma unroll 1
+                for (int e = e0 + tid - EPI_WARP * 32; e < e1; e += S::EPI_WARPS * 32) {
+                    const int er = row0 + (e & (TC_M - 1)), ec = col0 + e / TC_M;
+                    if (!whole || er >= wk.rows || ec >= wk.m) continue;
+                    const size_t o = (size_t) ec * wk.rows + er;
+                    float v[8], sum = resid ? resid[o] : 0.0f;     // resid may be y itself: read and written by this thread only
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) v[p] = p < wk.parts ? skd::ld_cluster(base + e * 4, p) : 0.0f;
+                    float f = v[0];
+#pragma unroll
+                    for (int p = 1; p < 8; ++p) if (p < wk.parts) f += v[p];
+                    y[o] = resid ? sum + f : f;
+                }
+                __syncwarp();
+                skd::cluster_sync_all();                   // nobody leaves while its sums are still read
+                break;
+            }
+            if (ok && row < wk.rows) {
+                // few instructions, since they are fetched anew for each tile; resid may be y itself: read and written by this thread only
+                const size_t ld = wk.rows;
+                const size_t o = (size_t) (col0 + c0) * ld + row;
+                float* at = y + o;
+                if (valid - c0 >= NC && resid == nullptr) {
+#pragma unroll
+                    for (int c = 0; c < NC / 2; ++c) {
+                        const float2 v = skd::up2(yacc[c]);
+                        at[0] = v.x; at += ld;
+                        at[0] = v.y; at += ld;
+                    }
+                } else {
+                    const float* ra = resid ? resid + o : nullptr;
+#pragma unroll
+                    for (int c = 0; c < NC; c += 8) {
+                        if (c0 + c >= valid) break;
+                        float rv[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            rv[j] = 0.0f;
+                            if (ra) { if (c0 + c + j < valid) rv[j] = *ra; ra += ld; }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float2 v = skd::up2(yacc[(c + j) / 2]);
+                            const float f = j & 1 ? v.y : v.x;
+                            if (c0 + c + j < valid) *at = ra ? rv[j] + f : f;
+                            at += ld;
+                        }
+                    }
                 }
             }
         }
+    }
+    if (Q4 && wk.parts > 1 && warp < EPI_WARP) {                 // the epilogue's two, in which the parts meet; all threads of a cluster take part
+        __syncwarp();
+        skd::cluster_sync_all();
+        skd::cluster_sync_all();
     }
     tc_fence_before();
     __syncthreads();
     if (warp == MMA_WARP) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-    }
-    if (parts > 1) {
-        __syncwarp();
-        skd::cluster_sync_all();                            // every part's sums are in place
-        skd::pdl_wait();
-        const uint32_t base = skd::smem_u32(smem + S::OFF_B);
-        // one flag a lane: read in turn they cost 0.4 us a call of four parts
-        const bool whole = !__any_sync(0xffffffffu, lane < parts && skd::ld_cluster(skd::smem_u32(gave_up), lane) != 0.0f);
-        const int per = (N * TC_M / 4 + parts - 1) / parts * 4, e0 = part * per, e1 = min(N * TC_M, e0 + per);
-        for (int e = e0 + tid; e < e1; e += S::THREADS) {
-            const int row = row0 + (e & (TC_M - 1)), col = col0 + e / TC_M;
-            if (!whole || row >= rows || col >= m) continue;
-            float v = 0.0f;
-            for (int p = 0; p < parts; ++p) v += skd::ld_cluster(base + e * 4, p);
-            const size_t o = (size_t) col * rows + row;
-            y[o] = resid ? resid[o] + v : v;           // resid may be y itself: read and written by this thread only
-        }
-        __syncwarp();
-        skd::cluster_sync_all();                            // nobody leaves while its sums are still read
     }
 }
 
@@ -466,123 +678,145 @@ int tc_clusters(int parts) {
     if (dev < 0 || dev >= 64) return std::max(1, sm_count() / parts);
     int n = known[dev][parts].load(std::memory_order_relaxed);
     if (n == 0) {
+        typedef TcShape<SKAINET_ENC_Q4_K, N> S;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned) parts); cfg.blockDim = dim3(TcShape<N>::THREADS); cfg.dynamicSmemBytes = TcShape<N>::SMEM;
+        cfg.gridDim = dim3((unsigned) parts); cfg.blockDim = dim3(S::THREADS); cfg.dynamicSmemBytes = S::SMEM;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned) parts; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
-        if (ensure_dynamic_smem((const void*) q4k_gemm_tc_kernel<N>, TcShape<N>::SMEM) != SKAINET_CUDA_OK ||
-            cudaOccupancyMaxActiveClusters(&n, q4k_gemm_tc_kernel<N>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = std::max(1, sm_count() / parts); }
+        if (ensure_dynamic_smem((const void*) kq_gemm_tc_kernel<SKAINET_ENC_Q4_K, N>, S::SMEM) != SKAINET_CUDA_OK ||
+            cudaOccupancyMaxActiveClusters(&n, kq_gemm_tc_kernel<SKAINET_ENC_Q4_K, N>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = std::max(1, sm_count() / parts); }
         known[dev][parts].store(n, std::memory_order_relaxed);
     }
     return n;
 }
 
-// Microseconds fitted to calls of 1 K x 1 K to 22 K x 4 K weights: what precedes the kernel, a super-block, a round of CTAs (prologue, first
-// loads, store), the exchange of a cluster.
-constexpr float TC_BEFORE = 6.0f, TC_ROUND = 3.5f;
-template <int N> constexpr float tc_unit() { return N == 128 ? 1.7f : N == 64 ? 1.28f : 1.1f; }
-template <int N> constexpr float tc_exchange() { return N == 128 ? 3.5f : N == 64 ? 2.0f : 1.0f; }
+// Microseconds, fitted to calls of 1 K x 1 K to 22 K x 4 K weights: what precedes the first super-block of a launch and follows its last, a
+// super-block of a tile, the meeting of a cluster's parts, a second launch.
+constexpr float TC_BASE = 3.5f, TC_SECOND = 2.0f;
+template <int N> constexpr float tc_unit(bool q4) { return q4 ? (N == 64 ? 0.89f : N == 32 ? 0.78f : 0.62f) : N == 64 ? 1.21f : N == 32 ? 1.05f : 0.91f; }
+template <int N> constexpr float tc_meet() { return N == 64 ? 2.0f : 1.2f; }
+constexpr int TC_MAX_PARTS = 8;
 
-// Parts of the contraction that share a tile: the number whose rounds of CTAs cost least (512 rows of 11008 x 4096: three rounds of whole
-// tiles 100 us, five of halves 112). *cost is the whole call.
+// A call: whole tiles in rounds, then a launch of the tiles left over in parts, where that costs less than one more round of them.
+struct TcPlan { int tile, whole, parts; float cost; };     // activation rows of a tile; tiles of the first launch; parts of the others
 template <int N>
-int tc_parts(int64_t tiles, int bpr, float* cost) {
-    int best = 1;
-    *cost = 1e30f;
-    for (int p = 1; p <= 8 && p <= bpr; ++p) {
-        const int64_t slots = p == 1 ? sm_count() : tc_clusters<N>(p), rounds = (tiles + slots - 1) / slots;
-        const float c = TC_BEFORE + (float) rounds * (tc_unit<N>() * (float) ((bpr + p - 1) / p) + TC_ROUND + (p > 1 ? tc_exchange<N>() : 0.0f));
-        if (c < *cost) { *cost = c; best = p; }
+TcPlan tc_plan_n(const Weight& w, int m, bool cut) {
+    const int64_t tiles = (int64_t) ((w.rows + TC_M - 1) / TC_M) * ((m + N - 1) / N);
+    const int sms = sm_count();
+    const bool q4 = w.enc == SKAINET_ENC_Q4_K;
+    const int64_t rounds = (tiles + sms - 1) / sms;
+    TcPlan best = {N, (int) tiles, 1, TC_BASE + tc_unit<N>(q4) * (float) (w.bpr * rounds)};
+    if (!cut) return best;
+    const int64_t full = tiles / sms * sms, rest = tiles - full;
+    for (int p = 2; p <= TC_MAX_PARTS && p <= w.bpr && rest > 0 && rest * p <= sms; ++p) {
+        const int64_t turns = (rest + tc_clusters<N>(p) - 1) / tc_clusters<N>(p);
+        const float c = TC_BASE + (full ? tc_unit<N>(q4) * (float) (w.bpr * (full / sms)) + TC_SECOND : 0.0f) + (float) turns * (tc_unit<N>(q4) * (float) ((w.bpr + p - 1) / p) + tc_meet<N>());
+        if (c < best.cost) best = {N, (int) full, p, c};
     }
     return best;
 }
 
-// What the mma.sync tile kernel takes for fewer than TC_ALWAYS_ROWS rows, fitted alike: its throughput, or its chain over the super-blocks.
+// 1 = not taken: a matrix no tensor map describes
+template <int ENC, int N>
+int32_t launch_tc_n(const Weight& w, ActQ8K a, int m, const TcPlan& plan, float* y, const float* resid, cudaStream_t s) {
+    typedef TcShape<ENC, N> S;
+    CUtensorMap mq, mh, mx;
+    if (tensor_map_bytes(&mq, w.qs, w.rows, (int64_t) w.bpr * 128, TC_M, 128) != SKAINET_CUDA_OK) return 1;
+    mh = mq;
+    if (!S::Q4 && tensor_map_bytes(&mh, w.extra, w.rows, (int64_t) w.bpr * 64, TC_M, 64) != SKAINET_CUDA_OK) return 1;
+    if (tensor_map_bytes(&mx, (const uint8_t*) a.q, m, w.cols, N, 128) != SKAINET_CUDA_OK) return 1;
+    static const bool fits = [] {                      // the registers that the warps share out are those of the launch
+        cudaFuncAttributes at;
+        return cudaFuncGetAttributes(&at, kq_gemm_tc_kernel<ENC, N>) == cudaSuccess && at.numRegs == S::R_LAUNCH;
+    }();
+    SK_REQUIRE(fits, "gemm_tc: built with other registers than its warps share out");
+    SK_TRY(ensure_dynamic_smem((const void*) kq_gemm_tc_kernel<ENC, N>, S::SMEM));
+    TcWork wk = {};
+    wk.rows = w.rows; wk.bpr = w.bpr; wk.m = m; wk.n_tiles = (m + N - 1) / N;
+    const int64_t tiles = (int64_t) ((w.rows + TC_M - 1) / TC_M) * wk.n_tiles;
+    SK_REQUIRE(tiles * TC_MAX_PARTS < (1ll << 31), "gemm_tc: too many tiles");
+    for (int second = 0; second < 2; ++second) {
+        wk.tile0 = second ? plan.whole : 0;
+        wk.tiles = second ? (int) tiles - plan.whole : plan.whole;
+        if (wk.tiles == 0) continue;
+        wk.parts = second ? plan.parts : 1;
+        wk.grid = second ? wk.tiles * wk.parts : std::min(wk.tiles, sm_count());
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned) wk.grid); cfg.blockDim = dim3(S::THREADS); cfg.dynamicSmemBytes = S::SMEM; cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned) wk.parts; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        SK_CUDA(cudaLaunchKernelEx(&cfg, kq_gemm_tc_kernel<ENC, N>, mq, mh, mx, (const uint8_t*) w.hdr, (const uint8_t*) w.aux, (const float*) a.d, (const int16_t*) a.bsums, wk, y, resid,
+                                   device_timeout_flag()));
+    }
+    return SKAINET_CUDA_OK;
+}
+template <int ENC>
+int32_t launch_tc(const Weight& w, ActQ8K a, int m, const TcPlan& p, float* y, const float* resid, cudaStream_t s) {
+    return p.tile == 16 ? launch_tc_n<ENC, 16>(w, a, m, p, y, resid, s) : p.tile == 32 ? launch_tc_n<ENC, 32>(w, a, m, p, y, resid, s) : launch_tc_n<ENC, 64>(w, a, m, p, y, resid, s);
+}
+
+// The cheapest tile for m rows and how its tiles are dealt out. Where tiles may be cut, narrower ones than the rows need never pay.
+TcPlan tc_cheapest(const Weight& w, int m, bool cut) {
+    TcPlan best = tc_plan_n<64>(w, m, cut);
+    if (!cut || m <= 32) { const TcPlan p = tc_plan_n<32>(w, m, cut); if (p.cost < best.cost) best = p; }
+    if (!cut || m <= 16) { const TcPlan p = tc_plan_n<16>(w, m, cut); if (p.cost < best.cost) best = p; }
+    return best;
+}
+
+// What the mma.sync tile kernel takes for fewer than TC_ALWAYS_ROWS rows of Q4_K, fitted alike: its throughput, or its chain over the super-blocks.
 float mma_cost(const Weight& w, int m) {
     const int mp = m <= 16 ? 16 : (m + 31) / 32 * 32;
     const int64_t ctas = (int64_t) ((w.rows + 63) / 64);
     const float rate = 2.0f * (float) mp * (float) w.rows * (float) w.cols / 210e6f;
-    const float chain = (float) w.bpr * (m <= 16 ? 0.55f : m <= 32 ? 0.75f * (float) std::min<int64_t>(2, (ctas + sm_count() - 1) / sm_count()) : 1.2f);
+    const float chain = (float) std::max(0, w.bpr - 2) * (m <= 16 ? 0.55f : m <= 32 ? 0.75f * (float) std::min<int64_t>(2, (ctas + sm_count() - 1) / sm_count()) : 1.2f);
     return 3.5f + std::max(rate, chain);
 }
 
-// Parts of a tile for m rows where this kernel is expected to cost less than the mma.sync one; 0 where it is not.
-template <int N>
-int tc_plan_n(const Weight& w, int m) {
-    const float other = m < TC_ALWAYS_ROWS ? mma_cost(w, m) : 1e30f;
-    if (other <= TC_BEFORE + TC_ROUND + tc_unit<N>()) return 0;              // below any call of this kernel
-    float cost;
-    const int parts = tc_parts<N>((int64_t) ((w.rows + TC_M - 1) / TC_M) * ((m + N - 1) / N), w.bpr, &cost);
-    return cost > other ? 0 : parts;
-}
-
-// 1 = not taken: scratch that cannot be had (or would have to grow while the stream is being captured), or a weight no tensor map describes
-template <int N>
-int32_t launch_tc_n(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int parts, cudaStream_t s) {
-    typedef TcShape<N> S;
-    const int m_pad = (m + N - 1) / N * N, m_tiles = (w.rows + TC_M - 1) / TC_M, n_tiles = m_pad / N;
-    CUtensorMap mq;
-    if (tensor_map_bytes(&mq, w.qs, w.rows, (int64_t) w.bpr * 128, TC_M) != SKAINET_CUDA_OK) return 1;
-    SK_TRY(ensure_dynamic_smem((const void*) q4k_gemm_tc_kernel<N>, S::SMEM));
-    const size_t xh_bytes = (size_t) m_pad * w.cols * 2, hs_bytes = (size_t) m_pad * (w.cols / 16) * 2;
-    const size_t need = gemm_tc_scratch_bytes(m, w.cols);
-    // the operand tiles live in the calling stream's own scratch (calls on different streams do not share them)
-    if (scratch_capacity(s, SCRATCH_GEMM) < need) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) { cudaGetLastError(); return 1; }
-    }
-    void* base = nullptr;
-    const int32_t st = scratch_get(s, SCRATCH_GEMM, need, &base);
-    if (st == SKAINET_CUDA_ERR_OOM) return 1;
-    if (st != SKAINET_CUDA_OK) return st;
-    auto up = [](size_t v) { return (v + 255) & ~(size_t) 255; };
-    __half* xh = (__half*) base;
-    __half* hs = (__half*) ((uint8_t*) base + up(xh_bytes));
-    float* dxt = (float*) ((uint8_t*) base + up(xh_bytes) + up(hs_bytes));
-    const int64_t n16 = (int64_t) m_pad * (w.cols / 16);
-    SK_CUDA(launch_pdl(act_f16_tiles_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, s, a, m, m_pad, w.cols, N == 128 ? 7 : N == 64 ? 6 : 5, xh, hs, dxt));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned) (m_tiles * parts), (unsigned) n_tiles); cfg.blockDim = dim3(S::THREADS); cfg.dynamicSmemBytes = S::SMEM; cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned) parts; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 2;
-    SK_CUDA(cudaLaunchKernelEx(&cfg, q4k_gemm_tc_kernel<N>, mq, (const uint8_t*) w.hdr, w.rows, w.bpr, parts, (const __half*) xh, (const __half*) hs, (const float*) dxt, m, m_pad, y, resid,
-                               device_timeout_flag()));
-    return SKAINET_CUDA_OK;
+// tile 0 where the mma.sync kernel is the quicker
+TcPlan tc_plan(const Weight& w, int m) {
+    TcPlan p = {};
+    if (w.enc != SKAINET_ENC_Q4_K || m < TC_MIN_ROWS || w.bpr < 1) return p;
+    p = tc_cheapest(w, m, true);
+    if (m < TC_ALWAYS_ROWS && p.cost > mma_cost(w, m)) p.tile = 0;
+    return p;
 }
 
 }  // namespace
 
-// What launch_gemm_tc needs of SCRATCH_GEMM for m rows of cols inputs.
-size_t gemm_tc_scratch_bytes(int m, int cols) {
-    const size_t m_pad = (size_t) (m + 127) / 128 * 128;
-    return m_pad * cols * 2 + m_pad * (cols / 16) * 2 + m_pad * (cols / 256) * 4 + 3 * 256;
-}
-
-// The tile (32, 64 or 128 activation rows) and the parts that share one for m rows; 0 where the mma.sync tile kernel is the quicker.
+// The tile (16, 32 or 64 activation rows, 128 where more rows make several of 64) and the CTAs of a cluster that share each (1: some are whole), for m
+// rows; 0 where
+// the mma.sync tile kernel is the quicker.
 int gemm_tc_plan(const Weight& w, int m, int* parts) {
-    *parts = 0;
-    if (w.enc != SKAINET_ENC_Q4_K || m < TC_MIN_ROWS || w.bpr < 1) return 0;
-    const int tile = m <= 32 ? 32 : m <= 64 ? 64 : 128;
-    *parts = tile == 32 ? tc_plan_n<32>(w, m) : tile == 64 ? tc_plan_n<64>(w, m) : tc_plan_n<128>(w, m);
-    return *parts ? tile : 0;
+    const TcPlan p = tc_plan(w, m);
+    *parts = p.tile == 0 ? 0 : p.whole ? 1 : p.parts;
+    return p.tile == 64 && m > 64 ? 128 : p.tile;
 }
 
-// y[m][w.rows] (= resid +) for quantized activation rows through tiles of 32, 64 or 128, `parts` CTAs a tile
+// y[m][w.rows] (= resid +) for quantized activation rows through tiles of 16, 32, 64 or 128 (two of 64), `parts` CTAs a tile (1 for Q6_K)
 int32_t launch_gemm_tc_tiles(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int tile, int parts, cudaStream_t s) {
-    return tile == 32 ? launch_tc_n<32>(w, a, m, y, resid, parts, s) : tile == 64 ? launch_tc_n<64>(w, a, m, y, resid, parts, s) : launch_tc_n<128>(w, a, m, y, resid, parts, s);
+    if (tile == 128) tile = 64;
+    const int64_t tiles = (int64_t) ((w.rows + TC_M - 1) / TC_M) * ((m + tile - 1) / tile);
+    if (tiles > 1 << 28) return 1;
+    const TcPlan p = {tile, parts > 1 ? 0 : (int) tiles, parts, 0.0f};
+    return w.enc == SKAINET_ENC_Q4_K ? launch_tc<SKAINET_ENC_Q4_K>(w, a, m, p, y, resid, s) : launch_tc<SKAINET_ENC_Q6_K>(w, a, m, p, y, resid, s);
 }
 
-// The same where it is the quicker. Returns 1 when not taken (the caller falls back to the mma.sync tile kernel).
+// The same where it is the quicker. Returns 1 when not taken (the caller falls back to the mma.sync tile kernels).
 int32_t launch_gemm_tc(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s) {
-    int parts;
-    const int tile = gemm_tc_plan(w, m, &parts);
-    return tile ? launch_gemm_tc_tiles(w, a, m, y, resid, tile, parts, s) : 1;
+    if (w.enc == SKAINET_ENC_Q6_K) {
+        const TcPlan p = tc_cheapest(w, m, false);
+        // up to eight rows: one pass of the row kernel, fitted to 1 K x 1 K to 11 K x 4 K (11008 x 4096 at 2 / 4 / 8 rows 16.6 / 26.5 / 46.9 us, here 18.5)
+        if (m < TC_MIN_ROWS && p.cost > 7.0f + 0.11e-6f * (float) w.rows * (float) w.cols * (float) m) return 1;
+        return launch_tc<SKAINET_ENC_Q6_K>(w, a, m, p, y, resid, s);
+    }
+    const TcPlan p = tc_plan(w, m);
+    return p.tile ? launch_tc<SKAINET_ENC_Q4_K>(w, a, m, p, y, resid, s) : 1;
 }
 
 }  // namespace sk

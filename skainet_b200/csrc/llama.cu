@@ -384,13 +384,6 @@ int32_t Llama::finalize() {
             for (Weight** w : {&L.wgate, &L.wup}) { weight_release(*w); *w = nullptr; }
         }
     }
-    // Room for the activation tiles of the tcgen05 linears: a step's graph is captured, where scratch cannot grow, and takes the same
-    // kernels whatever ran before it.
-    if (cfg.linear_enc == SKAINET_ENC_Q4_K) {
-        void* room = nullptr;
-        const int32_t st = scratch_get(stream, SCRATCH_GEMM, gemm_tc_scratch_bytes(max_rows, std::max(std::max((int) cfg.d_model, ffn_l), heads_l * (int) cfg.head_dim)), &room);
-        if (st != SKAINET_CUDA_OK && st != SKAINET_CUDA_ERR_OOM) return st;       // without the room the mma.sync kernels take its place
-    }
     // rotation factors: angle = pos * theta^(-2i/d) in double, rounded once
     const int half = cfg.head_dim / 2;
     std::vector<float> cs((size_t) cfg.max_seq * half), sn(cs.size());

@@ -38,15 +38,15 @@ int32_t launch_matvec_ring(const Weight& w, const MatvecIn& in, int prep, float*
 // gemm_mma.cu: y[m][w.rows] (= resid +) for m >= 2 quantized activation rows on the tensor cores; 1 = not taken
 int32_t launch_gemm_mma(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
 int32_t launch_gemm_mma_q8(const Weight& w, ActSplit a, int m, float* y, const float* resid, cudaStream_t s);
-// Rows from which the tcgen05 kernel is considered (fewer: the matvec and ring kernels), and from which it is taken whatever the shape;
-// between them it is where its call is expected to cost less than the mma.sync tile kernel's. Measured per call, tcgen05 / mma.sync, us:
-// 4096 x 11008 at 64 rows 26.8 / 65.6, at 128 32.0 / 70.5; 4096 x 4096 at 64 rows 16.9 / 22.1; 11008 x 4096 at 32 rows 26.0 / 28.0, at 128
-// 37.3 / 53.9; the other way 22016 x 4096 at 32 rows 47.0 / 30.0, 4096 x 1024 at 64 rows 12.2 / 8.9.
+// Rows of Q4_K from which the tcgen05 kernel is considered (fewer: the matvec and ring kernels), and from which it is taken whatever the shape;
+// between them it is where its call is expected to cost less than the mma.sync tile kernel's. Measured per call, quantizer included, tcgen05 /
+// mma.sync, us: 4096 x 11008 at 64 rows 19.4 / 65.6; 4096 x 4096 at 16 rows 8.7 / 13.9, at 64 12.5 / 22.1; 11008 x 4096 at 32 rows 16.0 / 28.0; the
+// other way 11008 x 4096 at 16 rows 14.6 / 15.0, 4096 x 1024 at 64 rows 8.1 / 6.2. Q6_K rows take it from nine on, fewer
+// where a pass of the row kernel is expected to cost more (an mma.sync tile kernel it replaced took 70 us for 64 rows of 4096 x 11008, against 45).
 constexpr int TC_MIN_ROWS = 9, TC_ALWAYS_ROWS = 288;
 // gemm_ring.cu: 2..8 activation rows over a Q4_K weight through the persistent ring; 1 = not taken
 int32_t launch_rows_ring(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);
-// gemm_tc.cu: the same for m >= TC_MIN_ROWS on tcgen05 with TMEM accumulators; 1 = not taken
-size_t gemm_tc_scratch_bytes(int m, int cols);
+// gemm_tc.cu: the same of Q4_K for m >= TC_MIN_ROWS, and of Q6_K, on tcgen05 with TMEM accumulators; 1 = not taken
 int gemm_tc_plan(const Weight& w, int m, int* parts);
 int32_t launch_gemm_tc_tiles(const Weight& w, ActQ8K a, int m, float* y, const float* resid, int tile, int parts, cudaStream_t s);
 int32_t launch_gemm_tc(const Weight& w, ActQ8K a, int m, float* y, const float* resid, cudaStream_t s);

@@ -11,8 +11,9 @@ namespace sk {
 int32_t tensor_map_rows(CUtensorMap* map, const bf16* base, int64_t rows, int ld, int box_rows);
 // boxes of box_blocks blocks of 64 k, box_rows rows each, block-major; coordinates (0, row, block)
 int32_t tensor_map_k_blocks(CUtensorMap* map, const bf16* base, int64_t rows, int ld, int box_rows, int box_blocks);
-// a byte plane [rows][row_bytes] (row_bytes a multiple of 16) in boxes of box_rows x 128 bytes, coordinates (byte, row)
-int32_t tensor_map_bytes(CUtensorMap* map, const uint8_t* base, int64_t rows, int64_t row_bytes, int box_rows);
+// a byte plane [rows][row_bytes] (row_bytes a multiple of 16) in boxes of box_rows x box_bytes (128, or 64 in the 64-byte swizzle: chunk XORed
+// with row / 2), coordinates (byte, row)
+int32_t tensor_map_bytes(CUtensorMap* map, const uint8_t* base, int64_t rows, int64_t row_bytes, int box_rows, int box_bytes);
 
 }  // namespace sk
 
