@@ -7,11 +7,13 @@
 // Persistent CTA (static tile schedule, activation tiles fastest so that CTAs running together share weight tiles in L2):
 //   warp 0     posts the tensor copies of the stage ring
 //   warp 1     issues the MMAs and commits (stage barriers to the producer, accumulator barrier to the epilogue)
-//   warps 2-5  epilogue: TMEM -> registers -> global; two accumulator sets, so it overlaps the next tile's MMAs
+//   warps 2-9  epilogue: TMEM -> registers -> global; two accumulator sets, so it overlaps the next tile's MMAs
 // NA = 2 keeps two 128-row weight tiles per activation tile: twice the rows of one matrix, or the same rows of gate and up,
 // whose product act(gate) * up is then formed in the epilogue without a round trip.
-// Warps 0 and 1 run their loops whole, with one elected lane for the copies and MMAs (skd::elect_one): a 2048-token prompt of the 2B
-// Fomalix shape, in passes of 1024 rows, took 15.42 ms so and 15.64 under `lane == 0` (the Tivazen shape: no more than runs differ by).
+// Warps 0 and 1 run their loops whole, with one elected lane for the copies and MMAs (skd::elect_one), and the warp's number and the TMEM address
+// are values known to be the same in all lanes (skd::warp_value), so that the operands stay in uniform registers. A 2048-token prompt of the 2B
+// Fomalix shape: 11.42 ms without the latter, 11.05 with it, 10.74 with eight epilogue warps instead of four and the issuing loop in fewer
+// instructions; of the Tivazen shape 9.79, 9.36 and 9.15.
 // Every mbarrier wait is bounded; a wait that runs out raises the device flag and the CTA still frees its TMEM.
 #include "linear_bf16.cuh"
 #include "tensor_map.cuh"
@@ -26,7 +28,7 @@ namespace {
 constexpr int BM = 128, BKE = 64;            // weight rows of one tile, k elements of a stage (128 bytes)
 constexpr int A_BYTES = BM * BKE * 2;
 constexpr int SMEM_BUDGET = 200 * 1024;
-constexpr int EPI_WARPS = 4, TC_THREADS = (2 + EPI_WARPS) * 32;
+constexpr int EPI_WARPS = 8, TC_THREADS = (2 + EPI_WARPS) * 32;
 
 template <int NA, int BN>
 struct Shape {
@@ -110,7 +112,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* acc_full = empty + S::STAGES;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = (uint32_t*) (acc_empty + 2);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = skd::warp_value(threadIdx.x >> 5), lane = threadIdx.x & 31;
     skd::pdl_launch_dependents();
     if (warp == 1) {
         if (lane == 0) {
@@ -125,7 +127,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = skd::warp_value(*tmem_slot);
     skd::pdl_wait();
     const int total = a.m_tiles * (a.segs ? *a.n_segs : a.n_tiles * a.groups);
 
@@ -154,19 +156,20 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!skd::mbar_wait_warp(full + j % S::STAGES, (j / S::STAGES) & 1, a.timeout_flag)) break;
     } else if (warp == 1) {
         // ---------------------------------------------- MMA issuer ----------------------------------------------
-        int it = 0, n = 0;
+        int s = 0, par = 0, n = 0;                              // stage and its round
         bool ok = true;
+        const uint64_t d0 = desc_sw128(skd::smem_u32(smem));
+#pragma unroll 1
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++n) {
             const int set = n & 1;
             if (n >= 2 && !(ok = skd::mbar_wait_warp(acc_empty + set, ((n >> 1) + 1) & 1, a.timeout_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d = tmem + set * S::COLS;
-            for (int k = 0; k < a.ksteps; ++k, ++it) {
-                const int s = it % S::STAGES;
-                if (!(ok = skd::mbar_wait_warp(full + s, (it / S::STAGES) & 1, a.timeout_flag))) break;
+#pragma unroll 1
+            for (int k = 0; k < a.ksteps; ++k) {
+                if (!(ok = skd::mbar_wait_tight(full + s, par, a.timeout_flag))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t base = skd::smem_u32(smem + s * S::STAGE);
-                const uint64_t da = desc_sw128(base), db = desc_sw128(base + NA * A_BYTES);
+                const uint64_t da = d0 + (uint64_t) (s * (S::STAGE >> 4)), db = da + (uint64_t) (NA * A_BYTES >> 4);
                 if (skd::elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < BKE / 16; ++kk)             // a K = 16 step advances the start address by 32 bytes inside the swizzle atom
@@ -174,15 +177,15 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         for (int i = 0; i < NA; ++i)
                             umma_bf16(d + i * BN, da + (uint64_t) ((i * A_BYTES + kk * 32) >> 4), db + (uint64_t) (kk * 2), IDESC, (k | kk) != 0);
                     umma_commit(empty + s);
+                    if (k == a.ksteps - 1) umma_commit(acc_full + set);
                 }
                 __syncwarp();
+                if (++s == S::STAGES) { s = 0; par ^= 1; }
             }
-            if (ok && skd::elect_one()) umma_commit(acc_full + set);
-            __syncwarp();
         }
     } else if (warp >= 2) {
         // ---------------------------------------------- epilogue ----------------------------------------------
-        const int quad = warp & 3;                               // TMEM lanes 32 * quad .. + 31 belong to this warp
+        const int quad = warp & 3, first = (warp - 2) >> 2 ? 32 : 0;     // TMEM lanes 32 * quad .. + 31 are this warp's, every other 32 columns
         int n = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++n) {
             const int set = n & 1;
@@ -194,7 +197,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const uint32_t src = tmem + set * S::COLS + ((uint32_t) (quad * 32) << 16);
             const int wr = tl.m0 + quad * 32 + lane;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = first; c0 < BN; c0 += 64) {
                 if (c0 >= tl.n_valid) break;
                 float u[32], v[32];
                 tmem_ld32(src + c0, u);

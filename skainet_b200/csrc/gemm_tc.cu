@@ -178,10 +178,6 @@ __device__ __forceinline__ uint32_t mbar_test5(uint64_t* a, uint64_t* late, uint
                  : "memory");
     return __reduce_and_sync(0xffffffffu, x | y);
 }
-// A value that is the same in all lanes of a warp, as one the compiler knows to be: addresses made from it stay in uniform registers. Moved
-// there anew for each MMA, they made one take 50 cycles.
-__device__ __forceinline__ uint32_t warp_value(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
-
 template <int R> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 // Eight columns out of TMEM. They are there once tmem_ld_wait() has been passed; loaded8() behind it keeps the compiler from using one earlier.
@@ -256,7 +252,7 @@ kq_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_const
     uint32_t* gave_up = tmem_slot + 1;                       // a wait of the fold ran out: the sums are not whole
 
     const int tid = threadIdx.x, lane = tid & 31, cta = blockIdx.x;
-    const int warp = warp_value(tid >> 5);
+    const int warp = skd::warp_value(tid >> 5);
     constexpr int MMA_WARP = 0, PROD_WARP = TC_MISC_WARPS, EPI_WARP = PROD_WARP + S::PROD_WARPS;      // the warps that all wait for come first: they are the ones preferred
     skd::pdl_launch_dependents();
 
@@ -277,7 +273,7 @@ kq_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_qs, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = warp_value(*tmem_slot);
+    const uint32_t tmem = skd::warp_value(*tmem_slot);
 
     if (warp < PROD_WARP) {
         regs_down<S::R_MISC>();

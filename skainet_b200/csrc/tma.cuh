@@ -47,6 +47,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
     return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, timeout_flag));
 }
 
+// The same in few instructions, for loops whose warps share the instruction caches with others'.
+__device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity, int* timeout_flag) {
+    bool ok = false;
+#pragma unroll 1
+    for (int i = 0; i < (1 << 22) && !ok; ++i) ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity));
+    if (!ok && timeout_flag) *timeout_flag = 1;
+    return ok;
+}
+
 // Programmatic dependent launch: let the next kernel in the stream start its independent prologue
 // now; and wait until every kernel this one depends on has completed and flushed its writes.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -72,6 +81,10 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
+
+// A value that is the same in all lanes of a warp, as one the compiler knows to be: addresses made from it stay in uniform registers. Moved
+// there anew for each MMA, they made one take 50 cycles.
+__device__ __forceinline__ uint32_t warp_value(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
 
 __device__ __forceinline__ uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 
