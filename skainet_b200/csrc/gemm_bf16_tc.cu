@@ -28,6 +28,9 @@ namespace {
 constexpr int BM = 128, BKE = 64;            // weight rows of one tile, k elements of a stage (128 bytes)
 constexpr int A_BYTES = BM * BKE * 2;
 constexpr int SMEM_BUDGET = 200 * 1024;
+// times of tiles in terms of the 256 x 128 one: a pair's of 256 x 256, of 256 + 256 x 128, and 128 x 128 of one CTA
+constexpr float PAIR_TIME = 0.75f, PAIR_TIME_GATED = 0.9f, HALF_TIME = 0.6f;
+constexpr int PAIR_MIN_K = 1024;
 constexpr int EPI_WARPS = 8, TC_THREADS = (2 + EPI_WARPS) * 32;
 
 template <int NA, int BN>
@@ -97,6 +100,33 @@ __device__ __forceinline__ Tile tile_at(const TcArgs& a, int t) {
     }
     r.m0 *= BM + a.a2_rows;                   // 128 rows per tile, 256 when the second weight tile continues the first
     return r;
+}
+
+// A warp's share of a finished tile: weight row wr of the lane, every other 32 activation rows from `first` on.
+template <int NA, int BN, int OUT>
+__device__ __forceinline__ void store_tile(const TcArgs& a, const Tile& tl, uint32_t src, int wr, int first, int lane) {
+#pragma unroll 1
+    for (int c0 = first; c0 < BN; c0 += 64) {
+        if (c0 >= tl.n_valid) break;
+        float u[32], v[32];
+        tmem_ld32(src + c0, u);
+        if (NA == 2) tmem_ld32(src + BN + c0, v);
+        // lane j fetches the factor of column j once; a load per column in the loop below would serialise on its latency
+        const float fl = a.scale && c0 + lane < tl.n_valid ? a.scale[(size_t) (tl.x_row + c0 + lane) * a.scale_ld + tl.col_group] : 1.0f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float f = __shfl_sync(~0u, fl, j);
+            if (c0 + j >= tl.n_valid) break;
+            const int r = tl.x_row + c0 + j;
+            const size_t at = (size_t) r * a.ldy + (size_t) tl.col_group * a.y_group_stride + wr;
+            if (lin_gated(OUT)) {
+                if (wr < a.w_rows) ((bf16*) a.y)[at] = __float2bfloat16_rn(skd::lin_gate<OUT>(u[j] * f) * (v[j] * f));
+            } else {
+                if (wr < a.w_rows) { if (OUT == LIN_OUT_F32) ((float*) a.y)[at] = u[j] * f; else ((bf16*) a.y)[at] = __float2bfloat16_rn(u[j] * f); }
+                if (NA == 2 && wr + BM < a.w_rows) { if (OUT == LIN_OUT_F32) ((float*) a.y)[at + BM] = v[j] * f; else ((bf16*) a.y)[at + BM] = __float2bfloat16_rn(v[j] * f); }
+            }
+        }
+    }
 }
 
 template <int NA, int BN, int OUT>
@@ -194,30 +224,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ok = __all_sync(~0u, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t src = tmem + set * S::COLS + ((uint32_t) (quad * 32) << 16);
-            const int wr = tl.m0 + quad * 32 + lane;
-#pragma unroll 1
-            for (int c0 = first; c0 < BN; c0 += 64) {
-                if (c0 >= tl.n_valid) break;
-                float u[32], v[32];
-                tmem_ld32(src + c0, u);
-                if (NA == 2) tmem_ld32(src + BN + c0, v);
-                // lane j fetches the factor of column j once; a load per column in the loop below would serialise on its latency
-                const float fl = a.scale && c0 + lane < tl.n_valid ? a.scale[(size_t) (tl.x_row + c0 + lane) * a.scale_ld + tl.col_group] : 1.0f;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const float f = __shfl_sync(~0u, fl, j);
-                    if (c0 + j >= tl.n_valid) break;
-                    const int r = tl.x_row + c0 + j;
-                    const size_t at = (size_t) r * a.ldy + (size_t) tl.col_group * a.y_group_stride + wr;
-                    if (lin_gated(OUT)) {
-                        if (wr < a.w_rows) ((bf16*) a.y)[at] = __float2bfloat16_rn(skd::lin_gate<OUT>(u[j] * f) * (v[j] * f));
-                    } else {
-                        if (wr < a.w_rows) { if (OUT == LIN_OUT_F32) ((float*) a.y)[at] = u[j] * f; else ((bf16*) a.y)[at] = __float2bfloat16_rn(u[j] * f); }
-                        if (NA == 2 && wr + BM < a.w_rows) { if (OUT == LIN_OUT_F32) ((float*) a.y)[at + BM] = v[j] * f; else ((bf16*) a.y)[at + BM] = __float2bfloat16_rn(v[j] * f); }
-                    }
-                }
-            }
+            store_tile<NA, BN, OUT>(a, tl, tmem + set * S::COLS + ((uint32_t) (quad * 32) << 16), tl.m0 + quad * 32 + lane, first, lane);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) arrive(acc_empty + set);
@@ -226,6 +233,187 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM) : "memory");
+}
+
+// ---- pairs of SMs (cta_group::2): 256 weight rows, gate and up 256 of each, against 256 activation rows, gated 128 ---------------------------------
+// A single CTA's tile of 256 x 128 takes 48 KB a stage for 512 cycles of MMAs, 94 bytes a cycle where an SM's port to L2 gives 64: 62 % of the tensor
+// pipe at 60 bytes a cycle. Here each CTA of the pair brings its own 128 weight rows (gated: 128 of gate and of up) and half of the activation rows,
+// 32 KB (40 KB) for the same MMAs, which read the other half out of the peer's shared memory.
+//
+// The even CTA issues for both: its `full` barriers count the bytes of both CTAs' copies, its commits arrive on both CTAs' `empty` and `acc_full`
+// barriers, and the epilogue warps of both arrive on its `acc_empty`. Each CTA stores its own weight rows.
+template <int NA>
+struct PairShape {
+    static constexpr int BN = NA == 2 ? 128 : 256, B_ROWS = BN / 2;
+    static constexpr int STAGE = NA * A_BYTES + B_ROWS * BKE * 2, STAGES = SMEM_BUDGET / STAGE;
+    static constexpr int COLS = NA * BN;                            // 256: two sets are all of TMEM
+    static constexpr int BARS = 2 * STAGES + 4;
+    static constexpr int SMEM = STAGES * STAGE + BARS * 8 + 16 + 1024;
+    static_assert(SMEM <= 227 * 1024 && 2 * COLS == 512, "a pair's tile");
+};
+__device__ __forceinline__ uint32_t in_leader(uint64_t* bar) {      // the address of the even CTA's barrier of the pair
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(skd::smem_u32(bar)));
+    return a;
+}
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(skd::smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {        // on the barrier of both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(skd::smem_u32(bar)), "h"((uint16_t) 3) : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// A wait for what the peer CTA may have arrived on.
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, int* timeout_flag) {
+    uint32_t ok = 0;
+#pragma unroll 1
+    for (int i = 0; i < (1 << 22) && !ok; ++i) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(skd::smem_u32(bar)), "r"(parity) : "memory");
+        ok = __all_sync(0xffffffffu, ok != 0);
+    }
+    if (!ok && timeout_flag) *timeout_flag = 1;
+    return ok != 0;
+}
+
+template <int NA, int OUT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b,
+                      const TcArgs a) {
+    typedef PairShape<NA> S;
+    constexpr int BN = S::BN;
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (BN >> 3) << 17) | ((uint32_t) (2 * BM >> 4) << 24);
+    extern __shared__ uint8_t raw[];
+    uint8_t* smem = raw + ((1024 - (skd::smem_u32(raw) & 1023)) & 1023);      // the same offset in both CTAs
+    uint64_t* full = (uint64_t*) (smem + S::STAGES * S::STAGE);
+    uint64_t* empty = full + S::STAGES;
+    uint64_t* acc_full = empty + S::STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = (uint32_t*) (acc_empty + 2);
+    const int warp = skd::warp_value(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    skd::pdl_launch_dependents();
+    if (warp == 1) {
+        if (lane == 0) {
+            for (int s = 0; s < S::STAGES; ++s) { skd::mbar_init(full + s, 1); skd::mbar_init(empty + s, 1); }
+            for (int b = 0; b < 2; ++b) { skd::mbar_init(acc_full + b, 1); skd::mbar_init(acc_empty + b, 2 * EPI_WARPS); }
+            skd::mbar_fence_init();
+        }
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(skd::smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    skd::cluster_sync_all();                                    // both CTAs' barriers are there
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = skd::warp_value(*tmem_slot);
+    skd::pdl_wait();
+    const int total = a.m_tiles * a.n_tiles;
+
+    if (warp == 0) {
+        // ---------------------------------------------- producer ----------------------------------------------
+        int s = 0, par = 1;                                     // the first round finds the stages empty
+        bool ok = true;
+#pragma unroll 1
+        for (int t = pair; t < total && ok; t += pairs) {
+            const int wrow = t / a.n_tiles * 2 * BM + rank * BM, xrow = t % a.n_tiles * BN + rank * S::B_ROWS;
+#pragma unroll 1
+            for (int k = 0; k < a.ksteps; ++k) {
+                if (!(ok = wait_cluster(empty + s, par, a.timeout_flag))) break;
+                uint8_t* st = smem + s * S::STAGE;
+                if (skd::elect_one()) {
+                    const uint32_t bar = in_leader(full + s);
+                    if (rank == 0) skd::mbar_expect_tx(full + s, 2 * S::STAGE);
+                    tma_load_pair(st, &map_a, k * BKE, wrow, bar);
+                    if (NA == 2) tma_load_pair(st + A_BYTES, &map_a2, k * BKE, wrow, bar);
+                    tma_load_pair(st + NA * A_BYTES, &map_b, k * BKE, xrow, bar);
+                }
+                __syncwarp();
+                if (++s == S::STAGES) { s = 0; par ^= 1; }
+            }
+        }
+        if (!ok)                                                // give copies in flight time to land before the CTA leaves
+            for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    } else if (warp == 1 && rank == 0) {
+        // ------------------------------------- MMA issuer, of the even CTA -------------------------------------
+        int s = 0, par = 0, n = 0;
+        bool ok = true;
+        const uint64_t d0 = desc_sw128(skd::smem_u32(smem));
+#pragma unroll 1
+        for (int t = pair; t < total && ok; t += pairs, ++n) {
+            const int set = n & 1;
+            if (!(ok = wait_cluster(acc_empty + set, ((n >> 1) & 1) ^ 1, a.timeout_flag))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem + set * S::COLS;
+#pragma unroll 1
+            for (int k = 0; k < a.ksteps; ++k) {
+                if (!(ok = wait_cluster(full + s, par, a.timeout_flag))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t da = d0 + (uint64_t) (s * (S::STAGE >> 4)), db = da + (uint64_t) (NA * A_BYTES >> 4);
+                if (skd::elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < BKE / 16; ++kk)
+#pragma unroll
+                        for (int i = 0; i < NA; ++i)
+                            umma_bf16_pair(d + i * BN, da + (uint64_t) ((i * A_BYTES + kk * 32) >> 4), db + (uint64_t) (kk * 2), IDESC, (k | kk) != 0);
+                    commit_pair(empty + s);
+                    if (k == a.ksteps - 1) commit_pair(acc_full + set);
+                }
+                __syncwarp();
+                if (++s == S::STAGES) { s = 0; par ^= 1; }
+            }
+        }
+    } else if (warp >= 2) {
+        // ---------------------------------------------- epilogue ----------------------------------------------
+        const int quad = warp & 3, first = (warp - 2) >> 2 ? 32 : 0;
+        int n = 0;
+#pragma unroll 1
+        for (int t = pair; t < total; t += pairs, ++n) {
+            const int set = n & 1;
+            Tile tl;
+            tl.group = tl.col_group = 0;
+            tl.m0 = t / a.n_tiles * 2 * BM + rank * BM; tl.x_row = t % a.n_tiles * BN; tl.n_valid = min(BN, a.rows - tl.x_row);
+            if (!wait_cluster(acc_full + set, (n >> 1) & 1, a.timeout_flag)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            store_tile<NA, BN, OUT>(a, tl, tmem + set * S::COLS + ((uint32_t) (quad * 32) << 16), tl.m0 + quad * 32 + lane, first, lane);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) arrive_cluster(in_leader(acc_empty + set));
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    skd::cluster_sync_all();                                    // nobody leaves while the other may still arrive here or read here
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+template <int NA, int OUT>
+int32_t run_pair(const LinearArgs& l, cudaStream_t s) {
+    typedef PairShape<NA> S;
+    CUtensorMap ma, ma2, mb;
+    SK_TRY(tensor_map_rows(&ma, l.w, l.w_rows, l.ldw, BM));
+    if (lin_gated(OUT)) SK_TRY(tensor_map_rows(&ma2, l.w2, l.w_rows, l.ldw, BM)); else ma2 = ma;
+    SK_TRY(tensor_map_rows(&mb, (const bf16*) l.x, l.x_rows_alloc, l.ldx, S::B_ROWS));
+    TcArgs a = {};
+    a.y = l.y; a.ldy = l.ldy; a.y_group_stride = l.y_group_stride; a.scale = l.scale; a.scale_ld = l.scale_ld;
+    a.w_rows = l.w_rows; a.rows = l.rows; a.groups = 1; a.ksteps = l.ldw / BKE;
+    a.m_tiles = (l.w_rows + 2 * BM - 1) / (2 * BM); a.n_tiles = (l.rows + S::BN - 1) / S::BN;
+    a.timeout_flag = device_timeout_flag();
+    const int64_t tiles = (int64_t) a.m_tiles * a.n_tiles;
+    SK_REQUIRE(tiles < (1ll << 30), "gemm_bf16_tc: too many tiles");
+    SK_TRY(ensure_dynamic_smem((const void*) gemm_bf16_pair_kernel<NA, OUT>, S::SMEM));
+    const int grid = 2 * (int) std::min<int64_t>(tiles, sm_count() / 2);
+    SK_CUDA(launch_pdl(gemm_bf16_pair_kernel<NA, OUT>, dim3(grid), dim3(TC_THREADS), S::SMEM, s, ma, ma2, mb, a));
+    return SKAINET_CUDA_OK;
 }
 
 template <int NA, int BN, int OUT>
@@ -262,12 +450,27 @@ int32_t run_out(const LinearArgs& l, cudaStream_t s) {
 int32_t launch_gemm_bf16_tc(const LinearArgs& l, cudaStream_t s) {
     SK_REQUIRE(!l.f32_act && l.row_index == nullptr, "gemm_bf16_tc: bf16 rows in order only");
     const int rows = l.segs ? l.seg_rows : l.rows;
+    const int sms = sm_count();
+    auto rounds = [](int64_t tiles, int64_t at_once) { return (float) ((tiles + at_once - 1) / at_once); };
+    // pairs of SMs: one plain matrix, where the rounds of pair tiles, at PAIR_TIME of a 256 x 128 tile's time, cost less than those of single CTAs.
+    // 2048 rows of 5632 x 2048 with gate: 84.6 -> 70.5 us, 8192 x 2048 75.6 -> 62.1. A contraction of few steps is over before the wider tile's stores
+    // are hidden (4096 x 512: 18.9 -> 22.3).
+    const int64_t pair_rows = (l.w_rows + 2 * BM - 1) / (2 * BM);
+    const bool plain = !l.segs && l.groups == 1 && rows > 128 && l.x_group_stride == 0 && sms >= 2;
+    if (lin_gated(l.out) && plain &&
+        rounds(pair_rows * ((rows + 127) / 128), sms / 2) * PAIR_TIME_GATED <= rounds((int64_t) ((l.w_rows + BM - 1) / BM) * ((rows + 127) / 128), sms))
+        return l.out == LIN_OUT_GEGLU ? run_pair<2, LIN_OUT_GEGLU>(l, s) : run_pair<2, LIN_OUT_SWIGLU>(l, s);
     // a segment's rows past its end belong to the next one: their columns are computed and not stored
     if (l.out == LIN_OUT_GEGLU) return rows <= 32 ? run_tc<2, 32, LIN_OUT_GEGLU>(l, s) : run_tc<2, 128, LIN_OUT_GEGLU>(l, s);
     if (l.out == LIN_OUT_SWIGLU) return rows <= 32 ? run_tc<2, 32, LIN_OUT_SWIGLU>(l, s) : run_tc<2, 128, LIN_OUT_SWIGLU>(l, s);
     if (rows <= 32) return run_out<1, 32>(l, s);
     const int64_t wide = (int64_t) ((l.w_rows + 2 * BM - 1) / (2 * BM)) * (l.segs ? l.max_segs : (int64_t) ((l.rows + 127) / 128) * l.groups);
-    return l.w_rows > BM && wide * 5 >= (int64_t) sm_count() * 4 ? run_out<2, 128>(l, s) : run_out<1, 128>(l, s);
+    const bool two = l.w_rows > BM && wide * 5 >= (int64_t) sms * 4;
+    if (plain && l.ldw >= PAIR_MIN_K) {
+        const float single = two ? rounds(wide, sms) : rounds((int64_t) ((l.w_rows + BM - 1) / BM) * ((rows + 127) / 128), sms) * HALF_TIME;
+        if (rounds(pair_rows * ((rows + 255) / 256), sms / 2) * PAIR_TIME <= single) return l.out == LIN_OUT_ACT ? run_pair<1, LIN_OUT_ACT>(l, s) : run_pair<1, LIN_OUT_F32>(l, s);
+    }
+    return two ? run_out<2, 128>(l, s) : run_out<1, 128>(l, s);
 }
 
 }  // namespace sk
