@@ -280,27 +280,43 @@ struct ScanShape {
     static constexpr int STAGES = KT <= 2 ? 2 : 1, LV = VT + 8, LT = CH + 8, V_TERM = CH * LV * 2;
     static constexpr int INV = DELTA ? 3 * CH * LT * 2 : 0;
     static __host__ __device__ int stage(int kp) { return 2 * CH * (kp + 8) * 2 + V_TERM + INV; }        // q | k | v | T
-    static __host__ __device__ int smem(int kp) { return STAGES * stage(kp) + 3 * kp * LV * 2 + (DELTA ? 9 : 3) * V_TERM; }   // stages | S | U' | W | U
+    static __host__ __device__ int smem(int kp) { return STAGES * stage(kp) + 3 * kp * LV * 2 + (DELTA ? 9 : 3) * V_TERM + VT * 256; }   // stages | S | U' | W | U | S^T q
 };
 
+// The walk over the chunks is a chain of short products: nothing is busy (tensor pipe 24 %, issue slots 26 %), latency bounds it, so each step's
+// work is spread over three groups of four warps, a warp per 16 tokens: group 0 holds the state and walks the chain (k S, T W, the update),
+// group 1 forms q S, hands it on in fp32, and brings the next chunk, group 2 forms q k^T with its decays and the outputs. They meet at barriers of
+// their own, all of them once a chunk. 2048 tokens of the Fomalix shape, passes and all: 10.19 ms with two groups that met twice a chunk, 9.80 with three, 9.20 with the
+// products' loads ahead of them, 8.85 with the decays of a strong chunk from 16-token references (such chunks took 9.7 thousand cycles, others 6.0).
+constexpr int SCAN_THREADS = 384, SCAN_GROUP = 128;
+
+// The groups' own barriers; barrier 0 is the block's.
+template <int ID, int COUNT>
+__device__ __forceinline__ void group_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
+template <int ID, int COUNT>
+__device__ __forceinline__ void group_arrive() { asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
+
 template <bool DELTA, int VT, int KT>
-__global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, const Work w) {
+__global__ void __launch_bounds__(SCAN_THREADS, 1) recur_scan_kernel(const RecurArgs a, const Work w) {
     typedef ScanShape<DELTA, VT, KT> Z;
     constexpr int NT = VT / 8, LV = Z::LV, NF = NT < 4 ? NT : 4;      // NF: 8-column sums in flight
     const RecurGeom& g = a.g;
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ double sG[2][CH];
     __shared__ float s_step[2][CH], s_rq[2][CH], s_rk[2][CH], s_e[2][CH], s_f[2][CH], s_col[2][CH];      // e^G, e^(G_end - G), the latter with |k|^-1 (and the step)
+    __shared__ float s_ref[2][CH / 16 - 1][CH];                     // under a strong decay: e^(G_ref - G) for the last token before a block of 16, with the same
     const int kp = w.kp, lk = kp + 8, ksn = kp / 16, tiles = w.vp / VT, h = blockIdx.x / tiles, c0 = (blockIdx.x % tiles) * VT, grp = h / (g.heads / g.groups);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tq = lane & 3, n_chunks = w.rows / CH;
     const uint32_t base = skd::smem_u32(raw), s_at = base + Z::STAGES * Z::stage(kp), up_at = s_at + 3 * kp * LV * 2, w_at = up_at + 3 * Z::V_TERM, u_at = w_at + 3 * Z::V_TERM;
+    const uint32_t sq_at = up_at + (DELTA ? 9 : 3) * Z::V_TERM + (threadIdx.x % SCAN_GROUP) * 4;
     const int s_term = kp * LV * 2;
     float* state = a.state + (size_t) a.map.seq * g.state_size() + (size_t) h * g.kdim * g.vld();
     skd::pdl_launch_dependents();
     const int pos0 = a.map.pos[a.map.seq];
     const float skip = DELTA ? 0.0f : a.d[h];
-    const bool holder = warp < 4;                                   // warps 0-3 hold the state, 4-7 the outputs
-    const int mt = holder ? warp : 7 - warp;                        // the warp's 16 tokens; later tokens sum over more, so the two kinds run opposite ways
+    const int group = warp >> 2;
+    const bool holder = group == 0;
+    const int mt = holder ? warp : 3 - (warp & 3);                  // the warp's 16 tokens; later tokens sum over more, so the groups run opposite ways
 
     // state rows 16 (mt + 4 i) + gr (+ 8), columns 8 n + 2 tq (+ 1); left by an earlier pass
     float S[KT][NT][4];
@@ -317,20 +333,24 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 }
     skd::pdl_wait();
 
+    const int kc = kp / 8, kr = (threadIdx.x % SCAN_GROUP) / kc, kcol = (threadIdx.x % SCAN_GROUP) % kc, kdr = SCAN_GROUP / kc, kdc = SCAN_GROUP % kc;
     auto load_chunk = [&](int c, int stage) {
         const uint32_t q = base + stage * Z::stage(kp), k = q + CH * lk * 2, v = k + CH * lk * 2, t = v + Z::V_TERM;
         const bf16 *gq = w.qk + ((size_t) grp * w.rows + c * CH) * kp, *gk = w.qk + ((size_t) (g.groups + grp) * w.rows + c * CH) * kp;
         const bf16* gv = w.v + ((size_t) h * w.rows + c * CH) * w.vp + c0;
-        const int kc = kp / 8;
-        for (int i = threadIdx.x; i < CH * kc; i += 256) {
-            const uint32_t at = ((i / kc) * lk + (i % kc) * 8) * 2;
+        const int x = threadIdx.x % SCAN_GROUP;
+        int r = kr, col = kcol;
+        for (int i = x; i < CH * kc; i += SCAN_GROUP) {
+            const uint32_t at = (r * lk + col * 8) * 2;
             skd::cp16(q + at, gq + (size_t) i * 8);
             skd::cp16(k + at, gk + (size_t) i * 8);
+            r += kdr; col += kdc;
+            if (col >= kc) { col -= kc; ++r; }
         }
-        for (int i = threadIdx.x; i < CH * (VT / 8); i += 256) skd::cp16(v + ((i / (VT / 8)) * LV + (i % (VT / 8)) * 8) * 2, gv + (size_t) (i / (VT / 8)) * w.vp + (i % (VT / 8)) * 8);
+        for (int i = x; i < CH * (VT / 8); i += SCAN_GROUP) skd::cp16(v + ((i / (VT / 8)) * LV + (i % (VT / 8)) * 8) * 2, gv + (size_t) (i / (VT / 8)) * w.vp + (i % (VT / 8)) * 8);
         if (DELTA) {
             const bf16* gt = w.inv + ((size_t) h * n_chunks + c) * 3 * CH * CH;
-            for (int i = threadIdx.x; i < 3 * CH * (CH / 8); i += 256) skd::cp16(t + ((i / (CH / 8)) * Z::LT + (i % (CH / 8)) * 8) * 2, gt + (size_t) i * 8);
+            for (int i = x; i < 3 * CH * (CH / 8); i += SCAN_GROUP) skd::cp16(t + ((i / (CH / 8)) * Z::LT + (i % (CH / 8)) * 8) * 2, gt + (size_t) i * 8);
         }
         skd::cp_commit();
     };
@@ -355,6 +375,14 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
             s_e[b][t] = expf((float) d[i]); s_f[b][t] = expf((float) (end - d[i]));
             s_col[b][t] = s_f[b][t] * rk[i] * (DELTA ? 1.0f : st[i]);
         }
+        if (end > -MILD_DECAY) return;
+#pragma unroll
+        for (int j = 0; j < CH / 16 - 1; ++j) {
+            const double ref = __shfl_sync(~0u, d[1], 8 * j + 7);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (2 * lane + i < 16 * (j + 1)) s_ref[b][j][2 * lane + i] = expf((float) (ref - d[i])) * rk[i] * (DELTA ? 1.0f : st[i]);
+        }
     };
     // three bf16 terms of a value pair into the terms' tiles
     auto put3 = [&](uint32_t at, int term, float x, float y) {
@@ -376,8 +404,8 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
     const int lr = lane & 7, l8 = (lane >> 3) & 1, l16 = lane >> 4;
     const uint32_t bt_off = ((lr + l8 * 8) * LV + l16 * 8) * 2;     // B fragments of a [k][columns] tile, transposed on load
 
-    load_chunk(0, 0);
-    if (warp == 7) store_scal(fetch_scal(0), 0);
+    if (group == 1) load_chunk(0, 0);
+    if (warp == 4) store_scal(fetch_scal(0), 0);
     if (holder) put_state();
 
     for (int c = 0; c < n_chunks; ++c) {
@@ -385,9 +413,6 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
         const uint32_t q = base + stage * Z::stage(kp), k = q + CH * lk * 2, v = k + CH * lk * 2, t_at = v + Z::V_TERM;
         skd::cp_wait<0>();
         __syncthreads();
-        if (Z::STAGES == 2 && c + 1 < n_chunks) load_chunk(c + 1, b ^ 1);
-        Scal next = {};
-        if (warp == 7 && c + 1 < n_chunks) next = fetch_scal(c + 1);
         const int t0 = mt * 16 + gr, t1 = t0 + 8;
 
         float acc[NT][4];
@@ -395,8 +420,11 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
-        if (DELTA || !holder) {                                     // k S or q S, 16 tokens
+        Scal next = {};
+        if (warp == 4 && c + 1 < n_chunks) next = fetch_scal(c + 1);
+        if (DELTA ? group < 2 : group == 1) {                       // k S or q S, 16 tokens
             const uint32_t a_at = (holder ? k : q) + ((mt * 16 + lr + l8 * 8) * lk + l16 * 8) * 2;
+#pragma unroll 2
             for (int ks = 0; ks < ksn; ++ks) {
                 uint32_t f[4];
                 skd::ldsm4(f, a_at + ks * 32);
@@ -414,7 +442,6 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 }
             }
         }
-        float p[8][4], row0 = 0.0f, row1 = 0.0f;
         if (holder) {
             const float e0 = DELTA ? s_e[b][t0] * s_rk[b][t0] : 0.0f, e1 = DELTA ? s_e[b][t1] * s_rk[b][t1] : 0.0f, b0 = s_step[b][t0], b1 = s_step[b][t1];
             const float f0 = s_f[b][t0] * s_rk[b][t0], f1 = s_f[b][t1] * s_rk[b][t1];
@@ -430,7 +457,7 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 else { put3(up_at + t0 * LV * 2 + at, Z::V_TERM, w0 * f0, w1 * f0); put3(up_at + t1 * LV * 2 + at, Z::V_TERM, w2 * f1, w3 * f1); }
             }
             if (DELTA) {
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                group_sync<1, SCAN_GROUP>();
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -459,59 +486,8 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                     put3(up_at + t0 * LV * 2 + at, Z::V_TERM, acc[n][0] * f0, acc[n][1] * f0); put3(up_at + t1 * LV * 2 + at, Z::V_TERM, acc[n][2] * f1, acc[n][3] * f1);
                 }
             }
-        } else {
-#pragma unroll
-            for (int n = 0; n < 8; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) p[n][i] = 0.0f;
-            const uint32_t a_at = q + ((mt * 16 + lr + l8 * 8) * lk + l16 * 8) * 2, b_at = k + ((lr + l16 * 8) * lk + l8 * 8) * 2;
-            for (int ks = 0; ks < ksn; ++ks) {
-                uint32_t f[4];
-                skd::ldsm4(f, a_at + ks * 32);
-#pragma unroll
-                for (int n = 0; n < 8; n += 2) {
-                    if (n > 2 * mt) break;
-                    uint32_t bb[4];
-                    skd::ldsm4(bb, b_at + (n * 8 * lk + ks * 16) * 2);
-                    skd::mma_bf16(p[n], f[0], f[1], f[2], f[3], bb[0], bb[1]);
-                    skd::mma_bf16(p[n + 1], f[0], f[1], f[2], f[3], bb[2], bb[3]);
-                }
-            }
-            const double G0 = sG[b][t0], G1 = sG[b][t1], end = sG[b][CH - 1];
-            float e0, e1;                                           // factors of S^T q now, and of the outputs at the end
-            row0 = s_rq[b][t0]; row1 = s_rq[b][t1];
-            if (end > -MILD_DECAY) {
-                // e^(G_t - G_s) = e^(G_t - G_end) e^(G_end - G_s): a factor per column here and one per row at the end, both in range
-#pragma unroll
-                for (int n = 0; n < 8; ++n) {
-                    if (n > 2 * mt + 1) break;
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int s = n * 8 + tq * 2 + i;
-                        const float f = s_col[b][s];
-                        p[n][i] *= s <= t0 ? f : 0.0f;
-                        p[n][i + 2] *= s <= t1 ? f : 0.0f;
-                    }
-                }
-                e0 = e1 = s_e[b][CH - 1];
-                row0 *= expf((float) (G0 - end)); row1 *= expf((float) (G1 - end));
-            } else {
-#pragma unroll
-                for (int n = 0; n < 8; ++n) {
-                    if (n > 2 * mt + 1) break;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int s = n * 8 + tq * 2 + (i & 1), t = i < 2 ? t0 : t1;
-                        p[n][i] *= s <= t ? expf((float) ((i < 2 ? G0 : G1) - sG[b][s])) * s_rk[b][s] * (DELTA ? 1.0f : s_step[b][s]) : 0.0f;
-                    }
-                }
-                e0 = s_e[b][t0]; e1 = s_e[b][t1];
-            }
-#pragma unroll
-            for (int n = 0; n < NT; ++n) { acc[n][0] *= e0; acc[n][1] *= e0; acc[n][2] *= e1; acc[n][3] *= e1; }
-        }
-        __syncthreads();
-        if (holder) {
+            if (DELTA) group_arrive<2, SCAN_THREADS>();
+            group_sync<1, SCAN_GROUP>();
             const float end = s_e[b][CH - 1];
 #pragma unroll
             for (int i = 0; i < KT; ++i) {
@@ -522,8 +498,7 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                     for (int e = 0; e < 4; ++e) S[i][n][e] *= end;
             }
 #pragma unroll
-            for (int ks = 0; ks < CH / 16; ++ks)
-{
+            for (int ks = 0; ks < CH / 16; ++ks) {
                 uint32_t f[KT][4];                                  // k transposed: rows are key coordinates
 #pragma unroll
                 for (int i = 0; i < KT; ++i) if (mt + 4 * i < ksn) skd::ldsm4_t(f[i], k + ((ks * 16 + lr + l16 * 8) * lk + 16 * (mt + 4 * i) + l8 * 8) * 2);
@@ -542,8 +517,84 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                         }
                 }
             }
+            group_sync<3, 2 * SCAN_GROUP>();
             put_state();
+        } else if (group == 1) {
+            group_arrive<3, 2 * SCAN_GROUP>();
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sq_at + (n * 4 + i) * SCAN_GROUP * 4), "f"(acc[n][i]) : "memory");
+            group_arrive<2, DELTA ? SCAN_THREADS : 2 * SCAN_GROUP>();
+            if (Z::STAGES == 2 && c + 1 < n_chunks) load_chunk(c + 1, b ^ 1);
+            if (warp == 4 && c + 1 < n_chunks) store_scal(next, b ^ 1);
         } else {
+            float p[8][4];
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) p[n][i] = 0.0f;
+            const uint32_t a_at = q + ((mt * 16 + lr + l8 * 8) * lk + l16 * 8) * 2, b_at = k + ((lr + l16 * 8) * lk + l8 * 8) * 2;
+            // all 64 keys, later ones than the tokens too: a branch per pair of tiles made each wait for its own load
+#pragma unroll 2
+            for (int ks = 0; ks < ksn; ++ks) {
+                uint32_t f[4], bb[4][4];
+                skd::ldsm4(f, a_at + ks * 32);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) skd::ldsm4(bb[n], b_at + (n * 16 * lk + ks * 16) * 2);
+#pragma unroll
+                for (int n = 0; n < 8; ++n) skd::mma_bf16(p[n], f[0], f[1], f[2], f[3], bb[n >> 1][2 * (n & 1)], bb[n >> 1][2 * (n & 1) + 1]);
+            }
+            const double G0 = sG[b][t0], G1 = sG[b][t1], end = sG[b][CH - 1];
+            float e0, e1;                                           // factors of S^T q now, and of the outputs at the end
+            float row0 = s_rq[b][t0], row1 = s_rq[b][t1];
+            if (end > -MILD_DECAY) {
+                // e^(G_t - G_s) = e^(G_t - G_end) e^(G_end - G_s): a factor per column here and one per row at the end, both in range
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    if (n > 2 * mt + 1) break;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int s = n * 8 + tq * 2 + i;
+                        const float f = s_col[b][s];
+                        p[n][i] *= s <= t0 ? f : 0.0f;
+                        p[n][i + 2] *= s <= t1 ? f : 0.0f;
+                    }
+                }
+                e0 = e1 = s_e[b][CH - 1];
+                row0 *= expf((float) (G0 - end)); row1 *= expf((float) (G1 - end));
+            } else {
+// the same around the last token before the warp's own 16, both factors at most one; its own 16 one by one
+                const double ref = sG[b][mt > 0 ? mt * 16 - 1 : 0];
+                const float r0 = expf((float) (G0 - ref)), r1 = expf((float) (G1 - ref));
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    if (n > 2 * mt + 1) break;
+                    if (n < 2 * mt) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const float f = s_ref[b][mt - 1][n * 8 + tq * 2 + i];
+                            p[n][i] *= r0 * f;
+                            p[n][i + 2] *= r1 * f;
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int s = n * 8 + tq * 2 + (i & 1), t = i < 2 ? t0 : t1;
+                        p[n][i] *= s <= t ? expf((float) ((i < 2 ? G0 : G1) - sG[b][s])) * s_rk[b][s] * (DELTA ? 1.0f : s_step[b][s]) : 0.0f;
+                    }
+                }
+                e0 = s_e[b][t0]; e1 = s_e[b][t1];
+            }
+            group_sync<2, DELTA ? SCAN_THREADS : 2 * SCAN_GROUP>();
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(acc[n][i]) : "r"(sq_at + (n * 4 + i) * SCAN_GROUP * 4));
+                    acc[n][i] *= i < 2 ? e0 : e1;
+                }
 #pragma unroll
             for (int ks = 0; ks < CH / 16; ++ks) {
                 if (ks > mt) break;
@@ -578,9 +629,8 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                     if (col + 1 < g.vdim) out[col + 1] = fmaf(acc[n][2 * e + 1], f, skip * skd::bf16_hi(x));
                 }
             }
-            if (warp == 7 && c + 1 < n_chunks) store_scal(next, b ^ 1);
         }
-        if (Z::STAGES == 1 && c + 1 < n_chunks) { __syncthreads(); load_chunk(c + 1, 0); }
+        if (Z::STAGES == 1 && c + 1 < n_chunks) { __syncthreads(); if (group == 1) load_chunk(c + 1, 0); }
     }
     if (holder)
 #pragma unroll
@@ -594,7 +644,7 @@ __global__ void __launch_bounds__(256, 1) recur_scan_kernel(const RecurArgs a, c
                 }
     // the convolution inputs the next pass needs; the kernel that reads the old ones is done
     const int keep = min(a.rows, g.taps), total = keep * g.conv_dim();
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    for (int i = blockIdx.x * SCAN_THREADS + threadIdx.x; i < total; i += gridDim.x * SCAN_THREADS) {
         const int row = a.rows - 1 - i / g.conv_dim(), ch = i % g.conv_dim();
         a.tail[(size_t) a.map.seq * g.tail_size() + (size_t) ((pos0 + row) % g.taps) * g.conv_dim() + ch] = a.proj[(size_t) row * a.proj_ld + a.conv_off + ch];
     }
@@ -604,7 +654,7 @@ template <bool DELTA, int VT, int KT>
 int32_t run_scan(const RecurArgs& a, const Work& w, cudaStream_t s) {
     const int bytes = ScanShape<DELTA, VT, KT>::smem(w.kp);
     SK_TRY(ensure_dynamic_smem((const void*) recur_scan_kernel<DELTA, VT, KT>, bytes));
-    SK_CUDA(launch_pdl(recur_scan_kernel<DELTA, VT, KT>, dim3(a.g.heads * (w.vp / VT)), dim3(256), bytes, s, a, w));
+    SK_CUDA(launch_pdl(recur_scan_kernel<DELTA, VT, KT>, dim3(a.g.heads * (w.vp / VT)), dim3(SCAN_THREADS), bytes, s, a, w));
     return SKAINET_CUDA_OK;
 }
 

@@ -1,0 +1,31 @@
+"""Prompts through the chunk scan (csrc/recurrence_chunk.cu) with decays whose sum over a chunk lies just beyond the bound up to which one
+pair of factors serves the whole chunk: each block of 16 tokens then refers to the last token before it, so that neighbours on both sides of
+a block's edge still see one another. Row counts around the edges of blocks and chunks, a second pass behind the first.
+
+Bar: that of the design's own tests for bfloat16; a reference one token off changes every key's weight by e."""
+import numpy as np
+import pytest
+
+import fomalix_models as M
+from oracle import fomalix as F
+from test_gpu_fomalix import TOL, make, portions  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+MIXERS = {"delta": M.delta(heads=6, kv_heads=3, dim=32, vdim=32), "delta_wide": M.delta(heads=40, kv_heads=20, dim=32, vdim=64),
+          "space": M.mamba(heads=6, groups=2, state=64, vdim=80, norm_groups=1), "space_wide": M.mamba(heads=80, groups=2, state=32, vdim=64, norm_groups=1)}
+
+
+@pytest.mark.parametrize("name", list(MIXERS))
+def test_strong_decay_across_block_edges(make, name):  # noqa: F811
+    cfg = M.config([(MIXERS[name], None)], width=64)
+    w = M.random_weights(cfg, 11)
+    heads = MIXERS[name][1]["heads"]
+    w["l0.mix.A_log"][:] = np.resize([0.6, 1.2, 1.6], heads)        # 0.6, 1.1 and 1.7 a token where the step's input is zero
+    w["l0.mix.dt_bias"][:] = -0.5
+    m = make(cfg, w, "bfloat16", prefill_rows=200, max_seq=256)
+    t = M.tokens(cfg, 200, 5)
+    ref = F.forward(cfg, w, t)
+    for cut in ([200], [17, 183], [64, 63, 73], [81, 119]):
+        m.reset()
+        assert M.error(portions(m, t, cut), ref) < TOL["bfloat16"], cut
