@@ -13,12 +13,11 @@
 // The sums are exact whatever the data, and (8 or 256) * high + low, an integer, is rounded once.
 // S2 is one f16 MMA of K = 16: mins (twice) times the sums of 32 codes, each in two parts that f16 holds.
 //
-// Persistent CTA of 128 weight rows (TMEM lanes) x N activation rows (TMEM columns; N = 16, 32, 64 or 128 by the batch). Warps:
+// Persistent CTA of 128 weight rows (TMEM lanes) x N activation rows (TMEM columns; N = 16, 32 or 64 by the batch). Warps:
 //   producers   sets of four warps, a thread a weight row; a set unpacks half a super-block (128 elements) into a slot of the A ring
 //               in TMEM (tcgen05.st), the sets taking halves in turn;
-//   epilogue    eight or sixteen warps fold finished super-blocks out of TMEM (tcgen05.ld), up to 32 fp32 accumulators a thread;
-//   one warp    issues the MMAs and commits; two accumulator sets, so the MMAs of one overlap the fold of the other: super-blocks in
-//               turn, or, at N = 128, the two halves of the columns, which share the A operand;
+//   epilogue    eight warps fold finished super-blocks out of TMEM (tcgen05.ld), up to 32 fp32 accumulators a thread;
+//   one warp    issues the MMAs and commits; two accumulator sets for super-blocks in turn, so the MMAs of one overlap the fold of the other;
 //   two warps   post the copies of weight tiles and activation tiles (tensor maps, 128-byte swizzle); one prepares S2's sums and the
 //               block scales of the columns.
 // Work: whole tiles in rounds of the grid; where the tiles left over are few, a cluster of CTAs shares each by parts of the contraction (Q4_K), whose
